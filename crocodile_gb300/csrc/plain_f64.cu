@@ -55,23 +55,58 @@ __global__ void k_grid_plain(PlainArgs A, int start, int count,
   atomicAdd(&grid[2 * cell + 1], val.y);
 }
 
+// Degridding: PLAIN_LANES threads per visibility, thread l summing taps
+// l, l + PLAIN_LANES, ... (separable kernels: footprint rows, so that the row
+// factor is applied once per row), then a shuffle reduction.  A group of some
+// thousand visibilities runs on few threads when each takes a whole footprint,
+// and its S * S dependent loads then set the time of every launch: 50,000
+// visibilities in 31 groups, S 9, took 1.51 ms with one thread per visibility
+// (49 us per launch); with eight the whole w_cache_imaging and w_cache_predict
+// pair of that size went from 1.65 to 1.00 ms.  Eight rather than 32 because GB300's
+// FP64 units take two FMAs per clock and SM: the reduction's additions would
+// cost as much as the taps.
+constexpr int PLAIN_LANES = 8;
+
+__device__ __forceinline__ void zfma(double2 &acc, double2 a, double2 b) {
+  acc.x = fma(-a.y, b.y, fma(a.x, b.x, acc.x));
+  acc.y = fma(a.y, b.x, fma(a.x, b.y, acc.y));
+}
+
 __global__ void k_degrid_plain(PlainArgs A, int start, int count,
                                const double2 *__restrict__ ktab,
                                const double2 *__restrict__ grid,
                                double2 *__restrict__ out) {
   if (any_failed(A.status)) return;
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= count) return;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int sub = threadIdx.x % PLAIN_LANES;
+  const bool live = t0 / PLAIN_LANES < count;
+  const int j = live ? (int)(t0 / PLAIN_LANES) : count - 1;  // the shuffles need whole warps
+  const int S = A.S;
   const VisRec r = A.recs[start + j];
+  const double2 *g = grid + (size_t)r.y0 * A.W + r.x0;
   double2 sum = make_double2(0.0, 0.0);
-  for (int dy = 0; dy < A.S; ++dy)
-    for (int dx = 0; dx < A.S; ++dx) {
-      const double2 g = grid[(size_t)(r.y0 + dy) * A.W + (r.x0 + dx)];
-      const double2 p = zmul(g, plain_kernel(A, ktab, r, dy, dx));
-      sum.x += p.x;
-      sum.y += p.y;
+  if (A.sep) {
+    const double2 *ky = ktab + (long long)r.k0 * S, *kx = ktab + (long long)r.k1 * S;
+    for (int dy = sub; dy < S; dy += PLAIN_LANES) {
+      double2 row = make_double2(0.0, 0.0);
+      for (int dx = 0; dx < S; ++dx) zfma(row, g[(size_t)dy * A.W + dx], kx[dx]);
+      zfma(sum, row, ky[dy]);
     }
-  out[A.perm[start + j]] = sum;
+  } else {
+    const int SS = S * S;
+    const double2 *k = ktab + ((long long)r.k0 * A.Q * A.Q + r.k1) * SS;
+    int dy = sub / S, dx = sub - dy * S;
+    for (int t = sub; t < SS; t += PLAIN_LANES) {
+      zfma(sum, g[(size_t)dy * A.W + dx], k[t]);
+      for (dx += PLAIN_LANES; dx >= S; dx -= S) ++dy;
+    }
+  }
+#pragma unroll
+  for (int o = PLAIN_LANES / 2; o > 0; o >>= 1) {
+    sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+    sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+  }
+  if (live && sub == 0) out[A.perm[start + j]] = sum;
 }
 
 // Boxcar cell: N//2 + floor(0.5 + N*p) with numpy's wrap of indices in [-N, 0).
@@ -189,7 +224,8 @@ int cg_degrid_fp64(const cg_plan *p, const void *ktab, const void *grid, void *o
     const int c = p->h_counts[g];
     if (!c) continue;
     const double2 *layer_grid = (const double2 *)grid + (size_t)(g / p->gper) * p->H * p->W;
-    k_degrid_plain<<<(unsigned)((c + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
+    const int64_t threads = (int64_t)c * PLAIN_LANES;
+    k_degrid_plain<<<(unsigned)((threads + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
         A, p->h_offsets[g], c, (const double2 *)ktab, layer_grid, (double2 *)out);
   }
   CG_LAUNCH("degrid_fp64");

@@ -1,0 +1,44 @@
+"""Kernel variants at the sizes where their splits can go wrong (tile edges, lane
+remainders, the smallest and largest supports), against the complex128 oracle."""
+
+import numpy
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    from crocodile_gb300 import _lib, engine, synthesis
+    from oracle import crocodile_oracle
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    return torch, _lib, engine, synthesis, crocodile_oracle
+
+
+def _case(seed, n, S, Q, sep, G=1, rmax=0.3):
+    rng = numpy.random.default_rng(seed)
+    uvw = numpy.column_stack([rng.uniform(-rmax, rmax, n), rng.uniform(-rmax, rmax, n),
+                              numpy.zeros(n)])
+    shape = (G, Q, S) if sep else (G, Q, Q, S, S)
+    gcf = rng.normal(size=shape) + 1j * rng.normal(size=shape)
+    src = rng.integers(0, G, n)[:, None]
+    return rng, uvw, gcf, src
+
+
+@pytest.mark.parametrize("sep", [True, False])
+@pytest.mark.parametrize("S,n", [(1, 1), (2, 33), (7, 5), (8, 100), (9, 257), (16, 31), (32, 3)])
+def test_plain_fp64_degrid(env, S, n, sep):
+    """Eight threads per visibility: supports below, at and above eight, a last block
+    with idle threads.  Tolerance: S^2 products of unit-variance terms, each with a few
+    roundings of 2^-53, against a sum that random signs leave S times smaller than its
+    terms' total."""
+    _, _, E, S_, O = env
+    rng, uvw, gcf, src = _case(S + n, n, S, 4, sep, G=3)
+    N = 96
+    a = rng.normal(size=(N, N)) + 1j * rng.normal(size=(N, N))
+    got = S_.convdegrid(gcf, a, uvw[:, :2], src, precision="fp64")
+    want = O.convdegrid(gcf, a, uvw[:, :2], src)
+    tol = 4 * (S * S + 8) * S * 2.0 ** -53
+    assert numpy.abs(got - want).max() <= tol * max(numpy.abs(want).max(), 1.0)
