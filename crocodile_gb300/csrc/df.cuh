@@ -100,6 +100,108 @@ __device__ __forceinline__ cdf cdf_scale(const cdf &a, df w) {
   return {df_mul(a.re, w), df_mul(a.im, w)};
 }
 
+// ---------------------------------------------------------------- packed pairs
+// Two independent double-float values in the halves of 64-bit registers, for
+// sm_100's packed FP32 instructions (add / mul / fma .rn.f32x2: one issue slot
+// for two FP32 operations, each rounded as its scalar form, so the results
+// are the scalar functions' bit for bit).  The transforms issue instructions
+// for most of their time, so pairs halve what bounds them.
+struct f32p {
+  unsigned long long v;
+};
+
+__device__ __forceinline__ f32p p_pack(float a, float b) {
+  f32p r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void p_unpack(f32p p, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ f32p p_add(f32p a, f32p b) {
+  f32p r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32p p_sub(f32p a, f32p b) {
+  f32p r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32p p_mul(f32p a, f32p b) {
+  f32p r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32p p_fma(f32p a, f32p b, f32p c) {
+  f32p r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+struct df2 {  // two double-floats
+  f32p hi, lo;
+};
+struct cdf2 {  // two complex double-floats
+  df2 re, im;
+};
+
+__device__ __forceinline__ df2 df2_renorm(f32p s, f32p c) {  // fast_two_sum
+  const f32p r = p_add(s, c);
+  return {r, p_sub(c, p_sub(r, s))};
+}
+// df_add_fast on both halves, and its difference form (the same rounded
+// operations as adding the negation)
+__device__ __forceinline__ df2 df2_add_fast(const df2 &x, const df2 &y) {
+  const f32p s = p_add(x.hi, y.hi), bb = p_sub(s, x.hi);
+  const f32p e = p_add(p_sub(x.hi, p_sub(s, bb)), p_sub(y.hi, bb));
+  return df2_renorm(s, p_add(e, p_add(x.lo, y.lo)));
+}
+__device__ __forceinline__ df2 df2_sub_fast(const df2 &x, const df2 &y) {
+  const f32p s = p_sub(x.hi, y.hi), bb = p_sub(s, x.hi);
+  const f32p e = p_sub(p_sub(x.hi, p_sub(s, bb)), p_add(y.hi, bb));
+  return df2_renorm(s, p_add(e, p_sub(x.lo, y.lo)));
+}
+__device__ __forceinline__ cdf2 cdf2_add_f(const cdf2 &a, const cdf2 &b) {
+  return {df2_add_fast(a.re, b.re), df2_add_fast(a.im, b.im)};
+}
+__device__ __forceinline__ cdf2 cdf2_sub_f(const cdf2 &a, const cdf2 &b) {
+  return {df2_sub_fast(a.re, b.re), df2_sub_fast(a.im, b.im)};
+}
+// df_dot2 on both halves, for x y + z t with the negations -y.hi, -t.hi at
+// hand (the products' errors come out negated and are subtracted)
+__device__ __forceinline__ df2 df2_dot2(const df2 &x, const df2 &y, f32p nyh, const df2 &z,
+                                        const df2 &t, f32p nth) {
+  const f32p p1 = p_mul(x.hi, y.hi), p2 = p_mul(z.hi, t.hi);
+  const f32p e1 = p_fma(x.hi, nyh, p1), e2 = p_fma(z.hi, nth, p2);
+  const f32p s = p_add(p1, p2), bb = p_sub(s, p1);
+  const f32p e = p_add(p_sub(p1, p_sub(s, bb)), p_sub(p2, bb));
+  f32p c = p_sub(e, p_add(e1, e2));
+  c = p_fma(x.hi, y.lo, c);
+  c = p_fma(x.lo, y.hi, c);
+  c = p_fma(z.hi, t.lo, c);
+  c = p_fma(z.lo, t.hi, c);
+  return df2_renorm(s, c);
+}
+// cdf_mul_f of both halves with one scalar factor w (float4 as cdf_load)
+__device__ __forceinline__ cdf2 cdf2_mul_f(const cdf2 &a, const float4 &w) {
+  const df2 wr = {p_pack(w.x, w.x), p_pack(w.y, w.y)};
+  const df2 wi = {p_pack(w.z, w.z), p_pack(w.w, w.w)};
+  const df2 nwi = {p_pack(-w.z, -w.z), p_pack(-w.w, -w.w)};
+  const f32p nwrh = p_pack(-w.x, -w.x);
+  return {df2_dot2(a.re, wr, nwrh, a.im, nwi, wi.hi), df2_dot2(a.re, wi, nwi.hi, a.im, wr, nwrh)};
+}
+__device__ __forceinline__ cdf2 cdf2_pack(const cdf &a, const cdf &b) {
+  return {{p_pack(a.re.hi, b.re.hi), p_pack(a.re.lo, b.re.lo)},
+          {p_pack(a.im.hi, b.im.hi), p_pack(a.im.lo, b.im.lo)}};
+}
+__device__ __forceinline__ void cdf2_unpack(const cdf2 &v, cdf &a, cdf &b) {
+  p_unpack(v.re.hi, a.re.hi, b.re.hi);
+  p_unpack(v.re.lo, a.re.lo, b.re.lo);
+  p_unpack(v.im.hi, a.im.hi, b.im.hi);
+  p_unpack(v.im.lo, a.im.lo, b.im.lo);
+}
+
 // FP64 <-> double-float at the edges of a pipeline, by integer operations on
 // the bit patterns (df_convert.h): the same results as the FP64 forms
 // (float)v, (float)(v - hi) and (double)hi + (double)lo without the FP64 pipe

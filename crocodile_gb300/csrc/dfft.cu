@@ -36,10 +36,6 @@ namespace cg {
 
 namespace {
 
-using dfk::AtCol;
-using dfk::radix2_first;
-using dfk::radix4;
-
 // ---------------------------------------------------------------- I/O policies
 // ld(row, i) / st(row, i, v): element i of transform row `row`
 
@@ -76,59 +72,56 @@ struct IoRowsCentred {
 
 // ---------------------------------------------------------------- column transforms
 // Planes [nplanes][N][W] of double-float, transformed along N (the columns);
-// each CTA takes C adjacent columns of one plane (C * 16 bytes per row read),
-// T threads; then the centred post-modulation (-1)^(l + k + phase) * scale and
-// complex128 out in place.
-template <int LOGN, int C, int T>
-__global__ void __launch_bounds__(T)
+// each CTA takes P pairs of adjacent columns of one plane (P * 32 bytes per
+// row read), N/4 threads per pair, neighbouring threads on neighbouring pairs
+// so that their 32-byte accesses join; then the centred post-modulation
+// (-1)^(l + k + phase) * scale and complex128 out in place.  The planes'
+// stride in shared memory puts the P pairs of one index on different banks.
+constexpr int col_plane(int n, int P) {
+  const int want = P >= 8 ? 1 : 8 / P % 8;  // stride mod 8 (16-byte units)
+  int s = dfk::pair_plane(n);
+  while (s % 8 != want) ++s;
+  return s;
+}
+
+template <int LOGN, int P>
+__global__ void __launch_bounds__((1 << LOGN) / 4 * P, dfk::DFFT_SM_THREADS / ((1 << LOGN) / 4 * P))
     k_dfft_cols_centred(double2 *d, int64_t nplanes, int W, int phase, float scale,
                         const float4 *__restrict__ tw, int inverse) {
   constexpr int N = 1 << LOGN;
   constexpr int Q = N / 4;
-  extern __shared__ float dsm[];
-  cdf *buf0 = (cdf *)dsm;    // [N][C]
-  cdf *buf1 = buf0 + N * C;  // [N][C]
-  cdf *stw = buf1 + N * C;   // [3N/4]
-  for (int k = threadIdx.x; k < 3 * Q; k += T) stw[k] = cdf_load(tw[k]);
+  constexpr int PL = col_plane(N, P);
+  extern __shared__ __align__(16) unsigned char dsm_raw[];
+  float4 *planes = (float4 *)dsm_raw;  // [re, im][P][PL]
+  float4 *stw = planes + 2 * P * PL;   // [3N/4]
+  const int p = threadIdx.x % P, t = threadIdx.x / P;
+  float4 *re = planes + p * PL, *im = planes + (P + p) * PL;
+  for (int k = threadIdx.x; k < 3 * Q; k += blockDim.x) stw[k] = tw[k];
   const bool inv = inverse != 0;
-  const int groups = W / C;
+  const int groups = W / (2 * P);
   const int64_t jobs = nplanes * groups;
+  __syncthreads();
   for (int64_t job = blockIdx.x; job < jobs; job += gridDim.x) {
     const int64_t plane = job / groups;
-    const int c0 = (int)(job - plane * groups) * C;
-    const float4 *src = (const float4 *)(d + plane * N * W) + c0;
-    for (int e = threadIdx.x; e < N * C; e += T) {
-      const int i = e / C, c = e - (e / C) * C;
-      buf0[e] = cdf_load(src[(int64_t)i * W + c]);
-    }
-    __syncthreads();
-    cdf *x = buf0, *y = buf1;
-    if (LOGN & 1) {
-      for (int b = threadIdx.x; b < N / 2 * C; b += T)
-        radix2_first<N>(x, y, stw, b / C, AtCol<C>{b % C});
-      __syncthreads();
-      cdf *tmp = x;
-      x = y;
-      y = tmp;
-    }
+    const int c = ((int)(job - plane * groups) * P + p) * 2;
+    double2 *col = d + plane * N * W + c;
+    cdf2 e[4];
 #pragma unroll
-    for (int ls = (LOGN & 1); ls < LOGN; ls += 2) {
-      for (int b = threadIdx.x; b < Q * C; b += T)
-        radix4<N>(x, y, stw, b / C, 1 << ls, inv, AtCol<C>{b % C});
-      __syncthreads();
-      cdf *tmp = x;
-      x = y;
-      y = tmp;
+    for (int k = 0; k < 4; ++k) {
+      const float4 *src = (const float4 *)(col + (int64_t)(t + k * Q) * W);
+      e[k] = cdf2_pack(cdf_load(src[0]), cdf_load(src[1]));
     }
-    double2 *dst = d + plane * N * W + c0;
-    for (int e = threadIdx.x; e < N * C; e += T) {
-      const int l = e / C, c = e - (e / C) * C;
-      const float sg = ((l + c0 + c + phase) & 1) ? -scale : scale;  // a power of two
-      const cdf v = x[e];
-      const cdf w = {{v.re.hi * sg, v.re.lo * sg}, {v.im.hi * sg, v.im.lo * sg}};
-      dst[(int64_t)l * W + c] = cdf_to(w);
+    dfk::pair_fft<LOGN>(e, re, im, stw, t, inv);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int l = t + ((k & 1) && !inv ? 4 - k : k) * Q;
+      const float sg = ((l + c + phase) & 1) ? -scale : scale;  // a power of two
+      cdf a, b;
+      cdf2_unpack(e[k], a, b);
+      double2 *dst = col + (int64_t)l * W;
+      dst[0] = cdf_to({{a.re.hi * sg, a.re.lo * sg}, {a.im.hi * sg, a.im.lo * sg}});
+      dst[1] = cdf_to({{b.re.hi * -sg, b.re.lo * -sg}, {b.im.hi * -sg, b.im.lo * -sg}});
     }
-    __syncthreads();
   }
 }
 
@@ -233,19 +226,18 @@ int dfft_twiddles(int n, int sign, const float4 **out) {
 
 namespace {
 
-template <int LOGN, int C>
+template <int LOGN, int P>
 int launch_cols(double2 *d, int64_t nplanes, int W, int phase, float scale, const float4 *tw,
                 int inverse, cudaStream_t st) {
   constexpr int N = 1 << LOGN;
-  constexpr int T = 256;
-  const size_t smem = (size_t)(2 * N * C + 3 * N / 4) * sizeof(cdf);
+  const size_t smem = (size_t)(2 * P * col_plane(N, P) + 3 * N / 4) * sizeof(float4);
   if (smem > 48 * 1024)
-    CG_CUDA(cudaFuncSetAttribute(k_dfft_cols_centred<LOGN, C, T>,
+    CG_CUDA(cudaFuncSetAttribute(k_dfft_cols_centred<LOGN, P>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t jobs = nplanes * (W / C);
+  const int64_t jobs = nplanes * (W / (2 * P));
   const unsigned grid = (unsigned)std::min<int64_t>(jobs, (int64_t)num_sms() * 8);
-  k_dfft_cols_centred<LOGN, C, T><<<grid, T, smem, st>>>(d, nplanes, W, phase, scale, tw,
-                                                         inverse);
+  k_dfft_cols_centred<LOGN, P><<<grid, N / 4 * P, smem, st>>>(d, nplanes, W, phase, scale, tw,
+                                                              inverse);
   CG_LAUNCH("double-float column FFT");
   return CG_OK;
 }
@@ -308,13 +300,13 @@ int dfft2_centred(double2 *data, int64_t batch, int H, int W, int inverse, cudaS
   if ((rc = dfft_twiddles(H, inverse ? 1 : -1, &tw))) return rc;
   const int phase = (H / 2 + W / 2) & 1;
   const float scale = inverse ? 1.0f / ((float)H * (float)W) : 1.0f;  // a power of two
-  switch (H) {  // columns per CTA: measured best for 512 at 2 (38 KB, 5 CTAs per SM)
-    case 64: return launch_cols<6, 16>(data, batch, W, phase, scale, tw, inverse, st);
-    case 128: return launch_cols<7, 16>(data, batch, W, phase, scale, tw, inverse, st);
-    case 256: return launch_cols<8, 8>(data, batch, W, phase, scale, tw, inverse, st);
-    case 512: return launch_cols<9, 2>(data, batch, W, phase, scale, tw, inverse, st);
-    case 1024: return launch_cols<10, 4>(data, batch, W, phase, scale, tw, inverse, st);
-    case 2048: return launch_cols<11, 2>(data, batch, W, phase, scale, tw, inverse, st);
+  switch (H) {  // pairs of columns per CTA: 256 threads up to 1024
+    case 64: return launch_cols<6, dfk::pairs_for(6)>(data, batch, W, phase, scale, tw, inverse, st);
+    case 128: return launch_cols<7, dfk::pairs_for(7)>(data, batch, W, phase, scale, tw, inverse, st);
+    case 256: return launch_cols<8, dfk::pairs_for(8)>(data, batch, W, phase, scale, tw, inverse, st);
+    case 512: return launch_cols<9, dfk::pairs_for(9)>(data, batch, W, phase, scale, tw, inverse, st);
+    case 1024: return launch_cols<10, dfk::pairs_for(10)>(data, batch, W, phase, scale, tw, inverse, st);
+    case 2048: return launch_cols<11, dfk::pairs_for(11)>(data, batch, W, phase, scale, tw, inverse, st);
   }
   return set_error(CG_ERR_ARG, "unsupported double-float FFT length %d", H);
 }
