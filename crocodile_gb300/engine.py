@@ -31,6 +31,10 @@ def require_cuda():
     L.lib()
 
 
+def is_device(x):
+    return isinstance(x, torch.Tensor) and x.is_cuda
+
+
 def cuda_tensor(x, dtype):
     """x (numpy array or tensor) as a contiguous CUDA tensor of dtype."""
     if isinstance(x, torch.Tensor):
@@ -423,6 +427,20 @@ def fft_df_(t, inverse):
                          "sides 64..2048")
     L.call("cg_fft2_centred_df", _p(t), t.numel() // (H * W), H, W, int(inverse), stream())
     return t
+
+
+def fft_df_window(out, inverse, src=None, out_size=None):
+    """Centred (i)fft of complex128 planes into ``out`` [..., H, W] (contiguous) in
+    double-float arithmetic (cg_fft2_window_df): of the planes src [planes, h, w]
+    (last stride 1) in the middle of zeros, or of ``out`` itself; out_size (oh, ow):
+    only the middle oh x ow of the result is written."""
+    H, W = out.shape[-2], out.shape[-1]
+    oh, ow = (H, W) if out_size is None else out_size
+    h, w = (H, W) if src is None else (src.shape[-2], src.shape[-1])
+    L.call("cg_fft2_window_df", _p(out), _p(src), 0 if src is None else src.stride(0),
+           0 if src is None else src.stride(1), out.numel() // (H * W), H, W, h, w, oh, ow,
+           int(inverse), stream())
+    return out
 
 
 def fft_timeouts(reset=True):

@@ -160,10 +160,16 @@ class Recombine:
     def _fft2_(self, t, inverse):
         # the double-float 2-D transform where its sizes allow ("auto"), else
         # FP64 cuFFT
-        if self.fft == "auto" and E.dfft2_supported(self.xM_size, self.xM_size) \
-                and t.is_contiguous():
+        if self._df2() and t.is_contiguous():
             return E.fft_df_(t, inverse)
         return E.fft_(t, inverse)
+
+    def _df2(self):
+        return self.fft == "auto" and E.dfft2_supported(self.xM_size, self.xM_size)
+
+    def _crop(self, approx):
+        c = self.xM_size // 2 - self.xA_size // 2
+        return approx[..., c:c + self.xA_size, c:c + self.xA_size]
 
     def facet_add(self, approx, facet, offs0, offs1, facet_off0, facet_off1, check=True):
         """approx [n0, n1, xM, xM] (centred) += the contributions of one centred
@@ -197,10 +203,7 @@ class Recombine:
         """The subgrids from their summed contributions: centred ifft (in place)
         and, with crop, the middle xA_size (a view)."""
         self._fft2_(approx, inverse=True)
-        if not crop:
-            return approx
-        c = self.xM_size // 2 - self.xA_size // 2
-        return approx[..., c:c + self.xA_size, c:c + self.xA_size]
+        return self._crop(approx) if crop else approx
 
     def recombine(self, facets, facet_offs0, facet_offs1, offs0, offs1, crop=True):
         """All subgrids [n0, n1, xA, xA] (or [.., xM, xM] without crop) of the
@@ -215,6 +218,9 @@ class Recombine:
             for j1, fo1 in enumerate(facet_offs1):
                 self.facet_add(approx, facets[j0][j1], o0, o1, fo0, fo1, check=False)
         self.status.check()
+        if crop and self._df2() and approx.numel():  # approx is ours: only the kept block
+            E.fft_df_window(approx, True, out_size=(self.xA_size, self.xA_size))
+            return self._crop(approx)
         return self.finish_subgrids(approx, crop=crop)
 
     # ------------------------------------------------------ subgrid -> facet
@@ -222,6 +228,11 @@ class Recombine:
     def subgrid_spectra(self, subgrids):
         """FS [..., xM, xM]: centred FFT of each centred subgrid [..., xA, xA]
         (or already [..., xM, xM]) zero-padded to xM_size."""
+        planes = self._planes(subgrids)
+        if planes is not None:
+            fs = torch.empty(tuple(subgrids.shape[:-2]) + (self.xM_size, self.xM_size),
+                             dtype=self.dtype, device="cuda")
+            return E.fft_df_window(fs, False, planes)
         s = E.cuda_tensor(subgrids, self.dtype)
         xA = s.shape[-1]
         if xA != self.xM_size:
@@ -232,6 +243,19 @@ class Recombine:
         else:
             fs = s.clone()
         return self._fft2_(fs, inverse=False)
+
+    def _planes(self, t):
+        """Device subgrids as [planes, xA, xA] that the double-float transform can
+        read where they lie (a view of recombine's result too), or None."""
+        if not (self._df2() and E.is_device(t) and t.dtype == self.dtype and t.dim() >= 2
+                and t.device.index == torch.cuda.current_device()
+                and t.numel() and t.shape[-2] == t.shape[-1] <= self.xM_size
+                and t.stride(-1) == 1) or t.is_conj() or t.is_neg():
+            return None
+        try:
+            return t.view((-1,) + tuple(t.shape[-2:]))
+        except RuntimeError:
+            return None
 
     def subgrids_to_facet(self, fs, offs0, offs1, facet_off0, facet_off1, out=None,
                           accumulate=False, check=True):

@@ -352,6 +352,16 @@ int cg_fft_rows_df(void *data_c128, int64_t batch, int n, int inverse, cg_stream
  * and the 1/(H W) of the inverse. */
 int cg_fft2_centred_df(void *data_c128, int64_t batch, int H, int W, int inverse,
                        cg_stream_t stream);
+/* The same transform of blocks: the in_h x in_w planes at src (element strides
+ * src_plane between planes and src_pitch between rows) in the middle (from
+ * H/2 - in_h/2, W/2 - in_w/2) of zero planes, into the planes H x W at data,
+ * of which the middle out_h x out_w is written and the rest left unspecified.
+ * src NULL: data itself (in_h = H, in_w = W).  src and data must not overlap
+ * otherwise.  Replaces the notebook's fft(pad_mid(..)) and extract_mid(ifft(..))
+ * (facet-subgrid-impl.ipynb cells 18, 30). */
+int cg_fft2_window_df(void *data_c128, const void *src, int64_t src_plane, int64_t src_pitch,
+                      int64_t batch, int H, int W, int in_h, int in_w, int out_h, int out_w,
+                      int inverse, cg_stream_t stream);
 
 /* Dirty image / PSF of a grid (synthesis.py:904-907): image = Re(ifft(
  * make_grid_hermitian(grid))), written as float32 H x W; the grid is

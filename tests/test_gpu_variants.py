@@ -42,3 +42,27 @@ def test_plain_fp64_degrid(env, S, n, sep):
     want = O.convdegrid(gcf, a, uvw[:, :2], src)
     tol = 4 * (S * S + 8) * S * 2.0 ** -53
     assert numpy.abs(got - want).max() <= tol * max(numpy.abs(want).max(), 1.0)
+
+
+@pytest.mark.parametrize("H,W,h,w,oh,ow", [(64, 64, 64, 64, 1, 1), (64, 128, 5, 37, 7, 9),
+                                           (512, 64, 384, 33, 384, 64), (128, 512, 1, 512, 128, 31),
+                                           (2048, 64, 2047, 2, 3, 64), (256, 256, 256, 256, 256, 255)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_fft_df_window(env, H, W, h, w, oh, ow, inverse):
+    """Blocks of odd sizes and places in padded planes, three planes (an odd number of
+    rows in pairs), read through strides; tolerance as for whole planes: 5e-14 of the
+    peak (about 2^-44 per stage of double-float rounding)."""
+    torch, _, E, S, O = env
+    rng = numpy.random.default_rng(H + w)
+    big = rng.normal(size=(3, h + 2, w + 3)) + 1j * rng.normal(size=(3, h + 2, w + 3))
+    src = torch.from_numpy(big).cuda()[:, 1:h + 1, 2:w + 2]
+    out = torch.full((3, H, W), 7.0, dtype=torch.complex128, device="cuda")
+    E.fft_df_window(out, inverse, src, (oh, ow))
+    r, c = H // 2 - h // 2, W // 2 - w // 2
+    R, C = H // 2 - oh // 2, W // 2 - ow // 2
+    for p in range(3):
+        full = numpy.zeros((H, W), dtype=complex)
+        full[r:r + h, c:c + w] = big[p, 1:h + 1, 2:w + 2]
+        want = (O.ifft if inverse else O.fft)(full)
+        got = out[p].cpu().numpy()[R:R + oh, C:C + ow]
+        assert numpy.abs(got - want[R:R + oh, C:C + ow]).max() <= 5e-14 * numpy.abs(want).max()
