@@ -849,7 +849,9 @@ def run_ours(args):
         kname = {L.CG_LAYOUT_LANE: "k_lane", L.CG_LAYOUT_OWNER: "k_grid_tiled"}.get(lay,
                                                                                    "k_grid_warp")
     else:
-        kname = "k_degrid_ring" if tuned.get("dvis") == 3 else "k_degrid_tiled"
+        # automatic (dvis 0): the ring beyond 4 GiB of table, else the direct degridder
+        ring = tuned.get("dvis") == 3 or G.kt.table.numel() * 8 > 4 << 30
+        kname = "k_degrid_ring" if ring else "k_degrid_direct"
     peaks = {}
     pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pk):

@@ -580,6 +580,215 @@ static void *grid_warp_kernel_for(int maxt) {
   }
 }
 
+// ---------------------------------------------------------------- direct kernels
+// Degridding and gridding straight on the grid, for supports up to 16, with no
+// window in shared memory: LV lanes share a visibility, so a warp works on
+// 32 / LV of them at once, and neighbouring visibilities (the plan's order)
+// find their cells in L1, or meet in L2.  What bounds the windowed kernels on
+// small supports is instructions and waiting, not memory: one warp per
+// visibility leaves two taps of S 8 to a lane beside ten shuffles of the
+// reduction (102 warp instructions per visibility), and each work item stages
+// (T + S - 1)^2 cells between block barriers (262 on the sub-grids of w-towers,
+// 13 visibilities to a tile).
+//
+// Lane l of a group takes taps l, l + LV, ..., every load of a visibility
+// issued together.  The degridder keeps the windowed kernels' order of
+// summation, bit for bit: theirs adds taps v, v + 32, ... in lane v and then
+// halves 32 lanes; here the partial sums of lanes l, l + LV, ... live in one
+// lane and the first halvings are additions of its own.
+//
+// Degridding, 1M visibilities, 2048^2, S 8 separable: 79 against 142 us; S 8
+// of 500k visibilities, 4-D table: 54 against 94; w-projection S 16, 2M: 397
+// against 479; 4M visibilities on 32 stacked 4096^2 grids: 0.60 against 2.06 ms.
+struct DirectArgs {
+  TiledArgs A;
+  int64_t n;
+  int layered;  // grids of a stack: by work item, which knows its layer
+};
+
+// Calls f(start, nb, grid offset) for batches of at most 32 sorted
+// visibilities of one grid, warp by warp.
+template <class F>
+__device__ __forceinline__ void direct_batches(const DirectArgs &D, F f) {
+  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  if (!D.layered) {
+    for (int64_t b = gw * 32; b < D.n; b += nw * 32)
+      f((int)b, (int)min((int64_t)32, D.n - b), (size_t)0);
+    return;
+  }
+  const int nitems = *D.A.nitems;
+  for (int64_t it = gw; it < nitems; it += nw) {
+    const WorkItem w = D.A.items[it];
+    const size_t off = (size_t)(w.tile / D.A.tpl) * D.A.H * D.A.W;
+    for (int b = 0; b < w.count; b += 32) f(w.start + b, min(32, w.count - b), off);
+  }
+}
+
+constexpr int direct_lanes(int S) { return S <= 8 ? 8 : S <= 11 ? 16 : 32; }
+
+template <bool SEP, int S>
+__global__ void __launch_bounds__(256, SEP && S >= 10 && S < 16 ? 3 : 4) k_degrid_direct(DirectArgs D,
+                                                          const float2 *__restrict__ ktab,
+                                                          const float2 *__restrict__ grid,
+                                                          float2 *__restrict__ out) {
+  const TiledArgs &A = D.A;
+  if (status_failed(A.status)) return;
+  constexpr int SS = S * S, LV = direct_lanes(S), NV = 32 / LV, NA = 32 / LV;
+  constexpr int MT = (SS + LV - 1) / LV;
+  const int QQ = A.Q * A.Q;
+  const int lane = threadIdx.x & 31, l = lane % LV, grp = lane / LV;
+  direct_batches(D, [&](int start, int nb, size_t goff) {
+    VisRec r = {0, 0, 0, 0};
+    int dst = 0;
+    if (lane < nb) {
+      r = A.recs[start + lane];
+      dst = A.perm[start + lane];
+    }
+    const unsigned cell = (unsigned)r.y0 * A.W + r.x0;
+    for (int q = 0; q < nb; q += NV) {
+      const int v = min(q + grp, nb - 1);
+      const float2 *g = grid + goff + __shfl_sync(0xffffffffu, cell, v);
+      const int k0 = __shfl_sync(0xffffffffu, r.k0, v), k1 = __shfl_sync(0xffffffffu, r.k1, v);
+      const int to = __shfl_sync(0xffffffffu, dst, v);
+      const float2 *ky = ktab + (int64_t)k0 * S, *kx = ktab + (int64_t)k1 * S;
+      const float2 *kk = ktab + ((int64_t)k0 * QQ + k1) * SS + l;
+      float2 acc[NA], c[MT], k[MT];
+#pragma unroll
+      for (int j = 0; j < NA; ++j) acc[j] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const int t = l + LV * m;
+        if (t < SS) {
+          const int dy = t / S, dx = t - dy * S;
+          c[m] = __ldg(&g[(unsigned)dy * A.W + dx]);
+          k[m] = SEP ? cmul(__ldg(&ky[dy]), __ldg(&kx[dx])) : __ldg(&kk[LV * m]);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+        if (l + LV * m < SS) cfma(acc[m % NA], c[m], k[m]);
+#pragma unroll
+      for (int o = NA / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < o; ++j) {
+          acc[j].x += acc[j + o].x;
+          acc[j].y += acc[j + o].y;
+        }
+      float2 sum = acc[0];
+#pragma unroll
+      for (int o = LV / 2; o > 0; o >>= 1) {
+        sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+        sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+      }
+      if (l == 0 && q + grp < nb) out[to] = sum;
+    }
+  });
+}
+
+// Taps as float2 atomics into the grid.  Separable tables: lane l of LV >= S
+// takes column l, its factor times the value once, and runs down the rows.
+template <bool SEP, int S>
+__global__ void __launch_bounds__(256, 4) k_grid_direct(DirectArgs D, int mode,
+                                                        const float2 *__restrict__ ktab,
+                                                        const float2 *__restrict__ vis,
+                                                        const float *__restrict__ weight,
+                                                        float2 *__restrict__ grid) {
+  const TiledArgs &A = D.A;
+  if (status_failed(A.status)) return;
+  constexpr int SS = S * S, LV = !SEP ? direct_lanes(S) : S <= 4 ? 4 : S <= 8 ? 8 : 16;
+  constexpr int NV = 32 / LV, MT = SEP ? S : (SS + LV - 1) / LV;
+  const int QQ = A.Q * A.Q;
+  const int lane = threadIdx.x & 31, l = lane % LV, grp = lane / LV;
+  direct_batches(D, [&](int start, int nb, size_t goff) {
+    VisRec r = {0, 0, 0, 0};
+    float2 val = make_float2(0.f, 0.f);
+    if (lane < nb) {
+      r = A.recs[start + lane];
+      const int src = A.perm[start + lane];
+      if (mode == 2) {
+        val.x = weight[src];
+      } else {
+        val = vis[src];
+        if (mode == 1) {
+          const float wt = weight[src];
+          val.x *= wt;
+          val.y *= wt;
+        }
+      }
+    }
+    const unsigned cell = (unsigned)r.y0 * A.W + r.x0;
+    for (int q = 0; q < nb; q += NV) {
+      const int v = min(q + grp, nb - 1);
+      float2 *g = grid + goff + __shfl_sync(0xffffffffu, cell, v);
+      const int k0 = __shfl_sync(0xffffffffu, r.k0, v), k1 = __shfl_sync(0xffffffffu, r.k1, v);
+      const float2 u = make_float2(__shfl_sync(0xffffffffu, val.x, v),
+                                   __shfl_sync(0xffffffffu, val.y, v));
+      if (q + grp >= nb) continue;  // (nothing below waits for the other lanes)
+      float2 k[MT];
+      if (SEP) {
+        if (l < S) {
+          const float2 *ky = ktab + (int64_t)k0 * S, *kx = ktab + (int64_t)k1 * S;
+          const float2 col = cmul(__ldg(&kx[l]), u);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) k[m] = __ldg(&ky[m]);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) atomicAdd(&g[(unsigned)m * A.W + l], cmul(k[m], col));
+        }
+      } else {
+        const float2 *kk = ktab + ((int64_t)k0 * QQ + k1) * SS + l;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+          if (l + LV * m < SS) k[m] = __ldg(&kk[LV * m]);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          const int t = l + LV * m, dy = t / S, dx = t - dy * S;
+          if (t < SS) atomicAdd(&g[(unsigned)dy * A.W + dx], cmul(k[m], u));
+        }
+      }
+    }
+  });
+}
+
+template <bool SEP, int S = 16>
+static void *degrid_direct_for(int support) {
+  if (support == S) return (void *)k_degrid_direct<SEP, S>;
+  if constexpr (S > 1) return degrid_direct_for<SEP, S - 1>(support);
+  return nullptr;
+}
+template <bool SEP, int S = 16>
+static void *grid_direct_for(int support) {
+  if (support == S) return (void *)k_grid_direct<SEP, S>;
+  if constexpr (S > 1) return grid_direct_for<SEP, S - 1>(support);
+  return nullptr;
+}
+
+static int direct_launch(const cg_plan *p, void *fn, void **args, cudaStream_t s) {
+  int per_sm = 0;
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
+  const int64_t warps = p->layers > 1 ? p->max_items : (p->n + 31) / 32;
+  const int64_t blocks = std::max<int64_t>(
+      1, std::min<int64_t>((int64_t)std::max(per_sm, 1) * num_sms(), (warps + 7) / 8));
+  CG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(256), args, 0, s));
+  return CG_OK;
+}
+
+static DirectArgs direct_args(const cg_plan *p) {
+  DirectArgs D;
+  D.A = tiled_args(p);
+  D.n = p->n;
+  D.layered = p->layers > 1;
+  return D;
+}
+
+static int direct_grid_launch(const cg_plan *p, const float2 *ktab, const float2 *vis,
+                              const float *weight, int mode, float2 *grid, cudaStream_t s) {
+  void *fn = p->kd.sep ? grid_direct_for<true>(p->kd.S) : grid_direct_for<false>(p->kd.S);
+  DirectArgs D = direct_args(p);
+  void *args[] = {&D, &mode, &ktab, &vis, &weight, &grid};
+  return direct_launch(p, fn, args, s);
+}
+
 static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
                        const float *weight, int mode, void *grid, cudaStream_t s) {
   CG_REQUIRE(p && p->mode == CG_PLAN_TILED, "cg_grid needs a CG_PLAN_TILED plan");
@@ -673,6 +882,9 @@ int cg_grid_sparse(const cg_plan *p, const void *ktab, const void *vis, void *gr
   CG_REQUIRE(p && p->mode == CG_PLAN_TILED, "cg_grid_sparse needs a CG_PLAN_TILED plan");
   if (p->n == 0) return CG_OK;
   CG_REQUIRE(ktab && vis && grid, "NULL argument");
+  if (p->kd.S <= 16)
+    return direct_grid_launch(p, (const float2 *)ktab, (const float2 *)vis, nullptr, 0,
+                              (float2 *)grid, (cudaStream_t)stream);
   const int SS = p->kd.S * p->kd.S;
   const int need = (SS + 31) / 32;
   void (*fn)(TiledArgs, const float2 *, const float2 *, float2 *) = nullptr;
@@ -698,17 +910,36 @@ int cg_degrid(const cg_plan *p, const void *ktab, const void *grid, void *out,
   CG_REQUIRE(ktab && grid && out, "NULL argument");
   cudaStream_t s = (cudaStream_t)stream;
   const int dvis = tuning().dvis;
+  const bool lane = layout_for(p->kd) == CG_LAYOUT_LANE;
   // dvis 1: lane-layout plans through the lane kernel's degridding traversal
-  // (slices by bulk copies, no output grid); everything else through the
-  // tiled degridder, which is the faster of the two at S 16
-  if (dvis == 1 && layout_for(p->kd) == CG_LAYOUT_LANE)
+  // (slices by bulk copies, no output grid)
+  if (dvis == 1 && lane)
     return lane_launch(p, (const float2 *)ktab, nullptr, nullptr, 0, nullptr,
                        (const float2 *)grid, (float2 *)out, 0, true, s);
-  // dvis 3: the shared window with per-warp slice rings, where the table streams
-  if (dvis == 3) {
+  // Automatic: the direct degridder, except where it measured slower.
+  //  - Tables far beyond L2 under dense visibilities: the slices come from HBM,
+  //    and the ring keeps four times as many bytes of them in flight (AW,
+  //    16.1M visibilities, 12.4 GB table: 3.67 ms, tiled 3.91, direct 4.56;
+  //    1.35M, 4.1 GB: 0.387 both; 1.75M on 8192^2, 1.8 GB: direct 0.43, ring
+  //    0.73; below that direct leads).
+  //  - S 13 to 15, 4-D, some hundred visibilities to a tile: rows that do not
+  //    fill the lanes (S 15, 3M visibilities on 4096^2: tiled 592, direct 647
+  //    us; 300k on 2048^2: 95 against 85).
+  const int64_t slices = (int64_t)p->kd.G * p->kd.Q * (p->kd.sep ? 1 : p->kd.Q);
+  const int64_t table = slices * p->kd.S * (p->kd.sep ? 1 : p->kd.S) * (int64_t)sizeof(float2);
+  const int64_t per_tile = p->n / std::max(p->ntx * p->nty * p->layers, 1);
+  const bool streams = lane && table > ((int64_t)4 << 30) && per_tile >= 16;
+  const bool ragged = !p->kd.sep && p->kd.S >= 13 && p->kd.S <= 15 && per_tile >= 400;
+  if (dvis == 3 || (dvis == 0 && streams)) {
     const int rc = ring_degrid_launch(p, (const float2 *)ktab, (const float2 *)grid,
                                       (float2 *)out, s);
     if (rc != CG_ERR_ARG) return rc;
+  }
+  if ((dvis == 0 || dvis == 1 || dvis == 3) && p->kd.S <= 16 && !ragged) {
+    void *fn = p->kd.sep ? degrid_direct_for<true>(p->kd.S) : degrid_direct_for<false>(p->kd.S);
+    DirectArgs D = direct_args(p);
+    void *args[] = {&D, &ktab, &grid, &out};
+    return direct_launch(p, fn, args, s);
   }
   TiledArgs A = tiled_args(p);
   const int SS = p->kd.S * p->kd.S;

@@ -105,12 +105,16 @@ typedef struct {
  * residues per owner-layout thread (1..8), or bulk-copy stages per
  * lane-layout warp (2..4; other values: 3); groups: owner-layout thread
  * groups, or warp-layout warps, per CTA (1..8), or lane-layout warps per
- * CTA (1..16); dvis: the degridder: 0 (automatic) or 2 runs the tiled
- * degridder with 2 visibilities per warp step, 4 with 4; 1 runs lane-layout
- * plans through the lane kernel's degridding traversal (others as 0); 3 runs
- * plans whose table streams by bulk copies (non-separable, S <= 16, 16-byte
- * slices) through the ring degridder: the item's window in shared memory,
- * each warp's slices by bulk copies through a 2-stage ring (others as 0).  layout 0 picks CG_LAYOUT_LANE (with 16-cell tiles) for
+ * CTA (1..16); dvis: the degridder: 0 (automatic) runs the direct degridder
+ * (S <= 16: lanes gather the footprint from the grid, no shared memory), the
+ * ring degridder where the table is far larger than L2, and the tiled one for
+ * wider supports; 2 and 4 the tiled degridder with that many visibilities per
+ * warp step; 1 lane-layout plans through the lane kernel's degridding traversal
+ * (others as 0); 3 plans whose table streams by bulk copies (non-separable,
+ * S <= 16, 16-byte slices) through the ring degridder: the item's window in
+ * shared memory, each warp's slices by bulk copies through a 2-stage ring
+ * (others as 0).  All of them but 1 sum a visibility's taps in the same order.
+ * layout 0 picks CG_LAYOUT_LANE (with 16-cell tiles) for
  * non-separable tables with even S <= 16, whose slices stream by bulk
  * copies as they are, and CG_LAYOUT_WARP otherwise.  Process-wide. */
 #define CG_LAYOUT_WARP 1

@@ -66,3 +66,62 @@ def test_fft_df_window(env, H, W, h, w, oh, ow, inverse):
         want = (O.ifft if inverse else O.fft)(full)
         got = out[p].cpu().numpy()[R:R + oh, C:C + ow]
         assert numpy.abs(got - want[R:R + oh, C:C + ow]).max() <= 5e-14 * numpy.abs(want).max()
+
+
+def _grids(torch, rng, N, layers=1):
+    g = rng.normal(size=(layers, N, N)) + 1j * rng.normal(size=(layers, N, N))
+    return g.astype(numpy.complex64)
+
+
+@pytest.mark.parametrize("sep", [True, False])
+@pytest.mark.parametrize("S", list(range(1, 18)))
+def test_degrid_direct_bits(env, S, sep):
+    """The direct degridder adds in the tiled degridder's order: equal bits for every
+    support (17: both tiled), visibility counts that leave lanes and batches partly
+    filled, and stacked grids."""
+    torch, L, E, _, _ = env
+    from crocodile_gb300 import autotune
+    for n, layers in ((1, 1), (37, 1), (1000, 3)):
+        rng, uvw, gcf, src = _case(S, n, S, 4, sep, G=3)
+        N = 80
+        kt = E.KernelTable.from_gcf(gcf, 1, E.CF)
+        lay = rng.integers(0, layers, n).astype(numpy.int32)
+        plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32),
+                      layers=None if layers == 1 else (layers, lay))
+        g = torch.from_numpy(_grids(torch, rng, N, layers)).cuda()
+        got = {}
+        for dvis in (0, 2, 4):
+            autotune.set_tuning(dvis=dvis)
+            try:
+                got[dvis] = plan.degrid(kt, g)
+            finally:
+                autotune.set_tuning()
+        plan.check()
+        assert torch.equal(torch.view_as_real(got[0]), torch.view_as_real(got[2]))
+        assert torch.equal(torch.view_as_real(got[4]), torch.view_as_real(got[2]))
+
+
+@pytest.mark.parametrize("sep", [True, False])
+@pytest.mark.parametrize("S", [1, 2, 4, 5, 8, 9, 11, 12, 16, 17])
+def test_grid_direct(env, S, sep):
+    """The direct gridder (cg_grid_sparse) over stacked grids and one grid against the
+    oracle.  Tolerance 2e-6: complex64 products (2^-24 each) summed over at most a few
+    hundred visibilities per cell."""
+    torch, L, E, _, O = env
+    for n, layers in ((3, 1), (500, 1), (700, 3)):
+        rng, uvw, gcf, src = _case(S + n, n, S, 4, sep, G=3)
+        N = 80
+        kt = E.KernelTable.from_gcf(gcf, 1, E.CF)
+        vis = rng.normal(size=n) + 1j * rng.normal(size=n)
+        lay = rng.integers(0, layers, n).astype(numpy.int32)
+        plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32),
+                      layers=None if layers == 1 else (layers, lay))
+        g = torch.zeros((layers, N, N), dtype=E.CF, device="cuda")
+        plan.grid_sparse(kt, E.cuda_tensor(vis, E.CF), g)
+        plan.check()
+        want = numpy.zeros((layers, N, N), dtype=complex)
+        for p in range(layers):
+            s = lay == p
+            if s.any():
+                O.convgrid(gcf, want[p], uvw[s, :2], src[s], vis[s])
+        assert numpy.linalg.norm(g.cpu().numpy() - want) <= 2e-6 * numpy.linalg.norm(want)
