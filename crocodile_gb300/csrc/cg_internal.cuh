@@ -263,6 +263,8 @@ struct cg_plan {
   int subshift; // sub-tile edge = 1 << subshift cells (4, or more for huge grid stacks)
   int64_t max_items;
   int chunk;    // visibilities per work item
+  int outer;    // window edge of the separable gridder (grid_outer.cu), 0: another gridder
+  int lean;     // plan_geometry: the choices that need the least workspace
   int slice_stride;  // lane layout: elements between S x S slices of the table it reads
   int64_t kpad_slices;  // lane layout, slices padded to a 16-byte multiple: slices to copy
   // device arrays inside the caller's workspace

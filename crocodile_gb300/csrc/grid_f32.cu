@@ -809,7 +809,18 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   void *args[12];
   int gsize = 0, ngroups = 0;
   bool shared = false;
+  if (p->outer) return outer_launch(p, kt, vv, nullptr, weight, mode, gg, s);
   const int layout = layout_for(p->kd);
+  // Automatic, another gridder than the plan's layout names: taps straight into
+  // the grid while few visibilities meet in a cell (L2 takes atomics on one
+  // address in turn) and, for supports that fill the lane gridder's lanes, few
+  // visibilities in all (direct / lane or warp gridder, us: S 9, 2M on 2048^2: 383 /
+  // 437, on 300^2: 685 / 432; S 8, 2M on 2048^2: 299 / 362; S 6, 500k: 63 / 100; S 12,
+  // 2M: 607 / 579; S 16, 500k: 241 / 172, 50k on 1024^2: 44 / 55; S 15, 1M: 441 / 458).
+  const double rho = (double)p->n / ((double)p->H * (double)p->W * (double)p->layers);
+  if (t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0 && S <= 16 && rho < 1.5 &&
+      (S <= 11 || layout != CG_LAYOUT_LANE || p->n < 100000))
+    return direct_grid_launch(p, kt, vv, weight, mode, gg, s);
   if (layout == CG_LAYOUT_LANE)
     return lane_launch(p, kt, vv, weight, mode, gg, nullptr, nullptr, 0, false, s);
   if (layout != CG_LAYOUT_OWNER) {
@@ -977,6 +988,21 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
   cudaStream_t s = (cudaStream_t)stream;
   const int S = p->kd.S;
   const cg_tuning t = tuning();
+  // Separable tables, small tiles: a block per tile has too little to do in one
+  // traversal, and the table is small, so reading it twice costs nothing.  Not
+  // in place: the second pass reads what the first would have overwritten.
+  const char *vi0 = (const char *)vis_in, *vo0 = (const char *)vis_out;
+  const size_t vbytes = (size_t)p->n * sizeof(float2);
+  const bool apart = !vis_in || !vis_out || vi0 + vbytes <= vo0 || vo0 + vbytes <= vi0;
+  if (p->outer && apart && (vis_out || !residual)) {
+    if (vis_out) {
+      const int rc = cg_degrid(p, ktab, grid_in, vis_out, stream);
+      if (rc) return rc;
+    }
+    if (!vis_in) return CG_OK;
+    return outer_launch(p, (const float2 *)ktab, (const float2 *)vis_in, (const float2 *)vis_out,
+                        nullptr, residual ? 3 : 0, (float2 *)grid_out, s);
+  }
   if (layout_for(p->kd) == CG_LAYOUT_LANE)
     return lane_launch(p, (const float2 *)ktab, (const float2 *)vis_in, nullptr, 0,
                        (float2 *)grid_out, (const float2 *)grid_in, (float2 *)vis_out, residual,

@@ -30,6 +30,7 @@ int plan_build_tiled_into(cg_plan *p, const cg_kernel_desc *kd, int H, int W,
                           const double *uvw, int64_t stride, double lam,
                           const int32_t *kidx, int64_t n, void *workspace,
                           size_t workspace_bytes, int32_t *d_status, cudaStream_t s);
+size_t plan_workspace_least(const cg_kernel_desc *kd, int H, int W, int64_t n);
 }
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[CG_NOALLOC_SCRATCH_BYTES];
@@ -59,7 +60,7 @@ extern "C" int cg_grid_noalloc(const cg_kernel_desc *kd, int H, int W, const dou
                                int64_t stride, double lam, const int32_t *kidx, int64_t n,
                                const void *ktab_c64, const void *vis_c64, void *grid_c64,
                                int32_t *d_status, cg_stream_t stream) {
-  const size_t need = cg_plan_workspace_bytes(CG_PLAN_TILED, n, H, W, kd);
+  const size_t need = cg::plan_workspace_least(kd, H, W, n);
   if (need == 0) return CG_ERR_ARG;  // message set by the size query
   if (need > (size_t)CG_NOALLOC_SCRATCH_BYTES)
     return cg::set_error(CG_ERR_WORKSPACE,

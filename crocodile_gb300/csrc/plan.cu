@@ -507,9 +507,35 @@ static int tile_edge(const cg_kernel_desc &kd, int req) {
   return 64;
 }
 
+// Window edge of the register-window gridder for separable tables
+// (grid_outer.cu) and its tile edge T (window >= T + S - 1), or 0 where another
+// gridder runs: its cost per visibility hardly depends on S, and its flush per
+// tile is spread over the tile's visibilities, so it takes wide supports, and
+// narrow ones where visibilities are dense (direct gridder / this one, us: S 8,
+// 0.24 visibilities per cell, 1M: 159 / 124, 0.06: 136 / 176; S 13, 0.06: 297 /
+// 243; S 16, 0.05, 200k: 101 / 81; S 6, 0.24: 97 / 125, 1.0: 120 / 111).  Stacks of
+// grids, requested or tuned tiles and tuned layouts keep the other gridders.
+static int outer_edge(const cg_plan &p, int &T) {
+  const cg_tuning t = tuning();
+  const int S = p.kd.S;
+  if (p.lean || !p.kd.sep || S > 16 || p.layers != 1 || p.tile_req > 0 || t.tile > 0 ||
+      t.layout > 0 || (int64_t)p.kd.G * p.kd.Q * S >= INT32_MAX)
+    return 0;
+  const double rho = (double)p.n / ((double)p.H * (double)p.W);
+  if (rho < (S >= 10 ? 0.03 : S >= 7 ? 0.1 : 1.5)) return 0;
+  if (S <= 9) {
+    T = S <= 5 ? 12 : 8;
+    return 16;
+  }
+  T = S <= 13 ? 12 : 8;
+  return 24;
+}
+
 static void plan_geometry(cg_plan &p) {
   if (p.mode == CG_PLAN_TILED) {
-    p.T = tile_edge(p.kd, p.tile_req);
+    int outer_T = 0;
+    p.outer = outer_edge(p, outer_T);
+    p.T = p.outer ? outer_T : tile_edge(p.kd, p.tile_req);
     p.ntx = (p.W + p.T - 1) / p.T;
     p.nty = (p.H + p.T - 1) / p.T;
     // Morton blocks of up to 32 x 32 tiles (no larger than the grid needs)
@@ -520,12 +546,12 @@ static void plan_geometry(cg_plan &p) {
     p.ntiles = p.tpl * p.layers;
     const cg_tuning t = tuning();
     // 4x4-cell sub-tiles, 2^sublog per tile edge (4 << full >= T), except for the
-    // lane layout, whose private windows need no order inside a tile (tile
-    // buckets only).  The sub-tile edge is 1 << subshift cells, so that an
+    // lane layout and the separable gridder, whose private windows need no order
+    // inside a tile (tile buckets only).  The sub-tile edge is 1 << subshift cells, so that an
     // in-tile coordinate shifted by subshift is always below 2^sublog.
     int full = 0;
     while ((4 << full) < p.T) ++full;
-    p.sublog = layout_for(p.kd) == CG_LAYOUT_LANE ? 0 : full;
+    p.sublog = p.outer || layout_for(p.kd) == CG_LAYOUT_LANE ? 0 : full;
     p.subshift = 2 + full - p.sublog;
     // keep the histogram (4 B per bucket) within 2^24 buckets: coarser sub-tiles
     // for very large grid stacks
@@ -539,12 +565,23 @@ static void plan_geometry(cg_plan &p) {
     // consecutive 8-byte bank pairs of the window (no bank conflicts)
     p.pitch = p.win;
     while ((p.pitch - p.kd.S) % 16 != 0) ++p.pitch;
-    int64_t want = p.n / (int64_t)(num_sms() * 16) + 1;
-    // lane layout: one warp per item, ~12 warps per SM, so shorter items
-    p.chunk = t.chunk > 0                              ? t.chunk
-              : layout_for(p.kd) == CG_LAYOUT_LANE ? 512
-                                                   : (int)std::min<int64_t>(
-                                                         2048, std::max<int64_t>(256, want));
+    // Visibilities per work item.  The tiled kernels take an item per CTA.  The
+    // lane gridder and the separable gridder take one per warp, so that an item
+    // is a chain of its visibilities' updates: short enough for a few items per
+    // warp (14 lane, 24 separable warps per SM), long enough to be worth a
+    // window's flush (S 16 lane gridder, 500k visibilities, 2048^2: 276 us with
+    // 512, 172 with 128, 179 with 64; 50k on 1024^2: 185 against 55 with 64; 2M
+    // on 4096^2: 606 with 512, 614 with 128).
+    const int64_t per_warp = p.n / (int64_t)(num_sms() * (p.outer ? 64 : 28));
+    auto clamp = [](int64_t v, int64_t lo, int64_t hi) {
+      return (int)(std::min(hi, std::max(lo, v)) & ~(int64_t)31);
+    };
+    p.chunk = t.chunk > 0 ? t.chunk
+              : p.outer   ? clamp(per_warp, 32, 256)
+              : layout_for(p.kd) == CG_LAYOUT_LANE
+                  ? (p.lean ? 512 : clamp(per_warp, 64, 512))
+                  : (int)std::min<int64_t>(
+                        2048, std::max<int64_t>(256, p.n / (int64_t)(num_sms() * 16) + 1));
     p.max_items = (p.n + p.chunk - 1) / p.chunk + p.ntiles;
     // The lane gridder streams each visibility's S x S slice with one bulk copy,
     // which needs a multiple of 16 bytes: for odd S * S it reads a copy of the
@@ -636,7 +673,12 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   p->tile_req = tile_req;
   plan_geometry(*p);
   CG_REQUIRE((int64_t)p->nbuckets < (int64_t)INT32_MAX / 2, "too many tiles");
-  const Layout L = layout_of(*p);
+  Layout L = layout_of(*p);
+  if (p->mode == CG_PLAN_TILED && workspace_bytes < L.total) {  // short items and small tiles take more
+    p->lean = 1;
+    plan_geometry(*p);
+    L = layout_of(*p);
+  }
   if (!workspace || workspace_bytes < L.total)
     return set_error(CG_ERR_WORKSPACE, "plan needs %zu workspace bytes, got %zu", L.total,
                      workspace_bytes);
@@ -722,6 +764,26 @@ int plan_build_tiled_into(cg_plan *p, const cg_kernel_desc *kd, int H, int W,
                           size_t workspace_bytes, int32_t *d_status, cudaStream_t s) {
   return plan_build_into(p, CG_PLAN_TILED, kd, H, W, uvw, stride, lam, kidx, 0.0, 0, 1, nullptr,
                          nullptr, 0, n, workspace, workspace_bytes, d_status, s);
+}
+
+// The least workspace a tiled plan can be built in (cg_plan_workspace_bytes is
+// what it would take of a larger one).
+size_t plan_workspace_least(const cg_kernel_desc *kd, int H, int W, int64_t n) {
+  if (check_desc(kd, H, W) != CG_OK) return 0;
+  cg_plan p;
+  memset(&p, 0, sizeof(p));
+  p.mode = CG_PLAN_TILED;
+  p.kd = *kd;
+  p.H = H;
+  p.W = W;
+  p.n = n;
+  p.layers = 1;
+  p.gper = kd->G;
+  plan_geometry(p);
+  const size_t need = layout_of(p).total;
+  p.lean = 1;
+  plan_geometry(p);
+  return std::min(need, layout_of(p).total);
 }
 
 // Heap plan; the groups form also copies the group ranges to the host.

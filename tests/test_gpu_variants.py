@@ -125,3 +125,46 @@ def test_grid_direct(env, S, sep):
             if s.any():
                 O.convgrid(gcf, want[p], uvw[s, :2], src[s], vis[s])
         assert numpy.linalg.norm(g.cpu().numpy() - want) <= 2e-6 * numpy.linalg.norm(want)
+
+
+@pytest.mark.parametrize("S", [1, 4, 5, 6, 7, 8, 9, 10, 13, 14, 16])
+@pytest.mark.parametrize("N", [64, 81, 100])
+def test_grid_separable_dense(env, N, S):
+    """Separable tables on dense visibilities (the register-window gridder): every
+    window and tile edge, grids that end inside a tile, footprints that touch the
+    grid's edges, items cut in short batches, weights, and the fused pass, against the
+    oracle.  Tolerance 3e-6: a few hundred complex64 products summed per cell."""
+    torch, L, E, _, O = env
+    n = 5 * N * N // 2
+    rng, uvw, gcf, src = _case(S + N, n, S, 4, True, G=2, rmax=0.5 - (S // 2 + 1) / N)
+    x = O.frac_coords((N, N), 4, uvw[:, :2])
+    ok = ((x[0] - S // 2 >= 0) & (x[0] - S // 2 + S <= N) & (x[2] - S // 2 >= 0) &
+          (x[2] - S // 2 + S <= N))
+    uvw, src = uvw[ok], src[ok]
+    n = len(uvw)
+    vis = (rng.normal(size=n) + 1j * rng.normal(size=n)).astype(numpy.complex64)
+    wt = rng.uniform(0.5, 2, n).astype(numpy.float32)
+    kt = E.KernelTable.from_gcf(gcf, 1, E.CF)
+    plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32))
+    assert plan.info()["tile"] == (12 if S <= 5 or 10 <= S <= 13 else 8)
+    v, w = E.cuda_tensor(vis, E.CF), E.cuda_tensor(wt, torch.float32)
+    for got, val in ((plan.grid(kt, v, torch.zeros((N, N), dtype=E.CF, device="cuda")), vis),
+                     (plan.grid_weighted(kt, v, w, torch.zeros((N, N), dtype=E.CF,
+                                                               device="cuda")), vis * wt),
+                     (plan.grid_weighted(kt, None, w, torch.zeros((N, N), dtype=E.CF,
+                                                                  device="cuda")), wt)):
+        want = numpy.zeros((N, N), dtype=complex)
+        O.convgrid(gcf, want, uvw[:, :2], src, val)
+        assert numpy.linalg.norm(got.cpu().numpy() - want) <= 3e-6 * numpy.linalg.norm(want)
+    model = E.cuda_tensor(_grids(torch, rng, N)[0], E.CF)
+    out = torch.zeros((N, N), dtype=E.CF, device="cuda")
+    d = plan.degrid_grid(kt, model, v, out, residual=True)
+    place = v.clone()  # in place: one traversal
+    out2 = torch.zeros((N, N), dtype=E.CF, device="cuda")
+    plan.degrid_grid(kt, model, place, out2, residual=True, vis_out=place)
+    plan.check()
+    dw = O.convdegrid(gcf, model.cpu().numpy().astype(complex), uvw[:, :2], src)
+    want = numpy.zeros((N, N), dtype=complex)
+    O.convgrid(gcf, want, uvw[:, :2], src, vis - dw)
+    for got, ref in ((d, dw), (place, dw), (out, want), (out2, want)):
+        assert numpy.linalg.norm(got.cpu().numpy() - ref) <= 3e-6 * numpy.linalg.norm(ref)
