@@ -22,12 +22,20 @@ def _p(t):
 
 
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the raw handle: torch.cuda.current_stream() builds a Stream object, 5 us a call
+    # against 0.4 here, and an imaging call asks about ten times
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+_cuda_seen = False
 
 
 def require_cuda():
-    if not torch.cuda.is_available():
-        raise RuntimeError("crocodile_gb300 needs a CUDA GPU (sm_103a); none is visible")
+    global _cuda_seen
+    if not _cuda_seen:
+        if not torch.cuda.is_available():
+            raise RuntimeError("crocodile_gb300 needs a CUDA GPU (sm_103a); none is visible")
+        _cuda_seen = True
     L.lib()
 
 
@@ -38,6 +46,9 @@ def is_device(x):
 def cuda_tensor(x, dtype):
     """x (numpy array or tensor) as a contiguous CUDA tensor of dtype."""
     if isinstance(x, torch.Tensor):
+        if x.dtype == dtype and x.is_cuda and x.is_contiguous() \
+                and x.get_device() == torch.cuda.current_device():
+            return x  # what the conversions below would return, without their cost
         t = x.to(device="cuda", dtype=dtype)
     else:
         a = numpy.asarray(x)
@@ -51,7 +62,8 @@ class Status:
     """The CG_STATUS_WORDS device counters shared by a sequence of calls."""
 
     def __init__(self):
-        self.t = torch.zeros(L.CG_STATUS_WORDS, dtype=torch.int32, device="cuda")
+        self.t = torch.empty(L.CG_STATUS_WORDS, dtype=torch.int32, device="cuda")
+        self.reset()
 
     def reset(self):
         L.call("cg_status_reset", _p(self.t), stream())
@@ -195,8 +207,6 @@ class Plan:
             L.raise_for(L.CG_ERR_ARG, "cg_plan_workspace_bytes_ex")
         self.ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
         self.status = status or Status()
-        if status is None:
-            self.status.reset()
         h = ctypes.c_void_p()
         L.call("cg_plan_create_ex", ctypes.byref(h), mode, ctypes.byref(kd), self.shape[0],
                self.shape[1], _p(self.uvw), self.uvw.stride(0), float(lam), _p(self.kidx),
@@ -506,8 +516,6 @@ def w_kernels(theta, ws_list, NpixFF, NpixKern, Qpx, invert=True, dl=0.0, dm=0.0
     w = numpy.ascontiguousarray(numpy.asarray(ws_list, dtype=numpy.float64).ravel())
     nw = len(w)
     st = status or Status()
-    if status is None:
-        st.reset()
     per = L.lib().cg_w_kernels_workspace_bytes(1, int(NpixFF), int(Qpx))
     full = L.lib().cg_w_kernels_workspace_bytes(nw, int(NpixFF), int(Qpx))
     nbytes = int(min(full, max(per + 256 + 8 * nw, max_workspace)))
@@ -534,8 +542,6 @@ def aw_kernels(A, Wk, a1, a2, wi, dtype=CF, status=None):
     nW, Q, S = Wk.shape[0], Wk.shape[1], Wk.shape[-1]
     nk = a1.shape[0]
     st = status or Status()
-    if status is None:
-        st.reset()
     nbytes = L.lib().cg_aw_kernels_workspace_bytes(nk, SA, nW, Q, S)
     ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
     out = torch.empty((nk, Q, Q, SA, SA), dtype=dtype, device="cuda")
