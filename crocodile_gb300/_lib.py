@@ -148,6 +148,8 @@ SIGNATURES = {
     "cg_aw_kernels": (c_int, [P, c_int, c_int, P, c_int, c_int, c_int, P, P, P, c_int, P, c_int,
                               P, c_size_t, P, P]),
     "cg_w_bins": (c_int, [P, c_int64, c_int64, c_double, P, P, P, P, P]),
+    "cg_uvw_ranges": (c_int, [P, c_int64, c_int64, c_double, P, P, P, P, P]),
+    "cg_pad_even": (c_int, [P, c_int64, c_int, P, P]),
     "cg_w_bins_fixed": (c_int, [P, c_int64, c_int64, c_double, c_int, c_int, P, P, P]),
 }
 

@@ -102,7 +102,7 @@ class KernelTable:
         return self if dtype == self.dtype else KernelTable(self.table.to(dtype), self.sep,
                                                             self.Q, self.S)
 
-    def padded_even(self, uvw, lam, shape):
+    def padded_even(self, uvw, lam, shape, bounds=None):
         """For a complex64 non-separable table of odd support S = 13 or 15, the same
         kernels zero-padded to S + 1 (a zero first row and column, so that tap j + 1
         of the padded kernel sits where tap j of the original did: footprints start
@@ -117,15 +117,15 @@ class KernelTable:
         if self.sep or self.dtype != CF or self.S not in (13, 15) or uvw.shape[0] == 0:
             return self
         N = min(int(shape[-2]), int(shape[-1]))
-        lo, hi = torch.aminmax(uvw[:, :2])
-        lo, hi = float(lo) / lam * N + N // 2, float(hi) / lam * N + N // 2
+        lo, hi = bounds if bounds is not None else uvw_ranges(uvw, 0.0, Status())[2]
+        lo, hi = lo / lam * N + N // 2, hi / lam * N + N // 2
         margin = self.S // 2 + 2
         if not (lo >= margin and hi <= N - 1 - margin):
             return self
         S, Q = self.S, self.Q
-        t = torch.zeros((self.G, Q, Q, S + 1, S + 1), dtype=CF, device=self.table.device)
-        t[..., 1:, 1:] = self.table.view(self.G, Q, Q, S, S)
-        return KernelTable(t.reshape(-1), False, Q, S + 1)
+        t = torch.empty(self.G * Q * Q * (S + 1) ** 2, dtype=CF, device=self.table.device)
+        L.call("cg_pad_even", _p(self.table), self.G * Q * Q, S, _p(t), stream())
+        return KernelTable(t, False, Q, S + 1)
 
     @classmethod
     def from_gcf(cls, gcf, nsrc, dtype=CF):
@@ -181,8 +181,11 @@ class Plan:
         (round(w / wstep) - kmin) inside the plan's coordinate pass.
         layers=(L, layer): grid visibility i into grid layer[i] of a stack of L grids.
         groups=(G, group): plain form only, one launch per group[i] in [0, G).
-        tile: this plan's grid tile edge (0: the tuning / automatic choice)."""
+        tile: this plan's grid tile edge (0: the tuning / automatic choice).
+        kidx may be a WBins, which stands for wbins."""
         require_cuda()
+        if isinstance(kidx, WBins):
+            kidx, wbins = None, (kidx.wstep, kidx.kmin)
         self.uvw = cuda_tensor(uvw, torch.float64)
         if self.uvw.dim() != 2 or self.uvw.shape[1] < 2:
             raise ValueError("uvw must be [n, >=2]")
@@ -310,6 +313,33 @@ def frac_coords(uvw, lam, shape, Q, status):
     L.call("cg_frac_coords", _p(uvw), uvw.stride(0), float(lam), n, int(shape[0]),
            int(shape[1]), int(Q), *[_p(o) for o in outs], _p(status.t), stream())
     return outs
+
+
+class WBins:
+    """In place of kernel indices: each visibility's kernel is its w bin, round(w /
+    wstep) - kmin, found in the plan's coordinate pass.  uv_bounds: the least and
+    greatest of all u and v."""
+
+    def __init__(self, wstep, kmin, uv_bounds):
+        self.wstep, self.kmin, self.uv_bounds = float(wstep), int(kmin), uv_bounds
+
+
+def uvw_ranges(uvw, wstep, status):
+    """(min w bin, max w bin, (min, max) of all u and v) (cg_uvw_ranges); wstep 0: no
+    bins."""
+    uvw = cuda_tensor(uvw, torch.float64)
+    work = torch.empty(24, dtype=torch.uint8, device="cuda")
+    uv, w = (ctypes.c_double * 2)(), (ctypes.c_int32 * 2)()
+    L.call("cg_uvw_ranges", _p(uvw), uvw.stride(0), uvw.shape[0], float(wstep), _p(work), uv, w,
+           _p(status.t), stream())
+    return int(w[0]), int(w[1]), (uv[0], uv[1])
+
+
+def w_range(uvw, wstep, status):
+    """uvw_ranges with w bins of a width that is not 0."""
+    if wstep == 0:
+        raise ValueError("wstep must be non-zero")
+    return uvw_ranges(uvw, wstep, status)
 
 
 def w_bins(uvw, wstep, status):

@@ -387,7 +387,7 @@ def _grid_into(ktab, kidx, uvw, lam, shape, vis, prec, weight=None, out=None, st
     src = ktab
     if prec == "fp32":
         uvw = E.cuda_tensor(uvw, torch.float64)
-        ktab = ktab.padded_even(uvw, lam, shape)  # same results, lane gridder
+        ktab = ktab.padded_even(uvw, lam, shape, getattr(kidx, "uv_bounds", None))  # lane gridder
     plan = E.Plan(uvw, lam, shape, ktab, kidx, mode, status)
     if ktab is not src:
         plan.accept(src, ktab)
@@ -414,7 +414,7 @@ def _degrid_from(ktab, kidx, uvw, lam, guv, prec):
     g = E.cuda_tensor(guv, dt)
     if prec == "fp32":
         uvw = E.cuda_tensor(uvw, torch.float64)
-        ktab = ktab.padded_even(uvw, lam, tuple(g.shape))  # same results, lane gridder
+        ktab = ktab.padded_even(uvw, lam, tuple(g.shape), getattr(kidx, "uv_bounds", None))
     plan = E.Plan(uvw, lam, tuple(g.shape), ktab, kidx, mode)
     out = plan.degrid(ktab, g) if prec == "fp32" else plan.degrid_fp64(ktab, g)
     plan.check()
@@ -558,12 +558,12 @@ def _spec_w_cache(theta, uvw_t, uvw_host, src, wstep, kernel_cache, kernel_fn, k
     nsrc = _src_cols(src, n)
     if kernel_cache is None and _is_w_kernel(kernel_fn) and nsrc == 0:
         st = E.Status()
-        kidx, kmin, kmax = E.w_bins(uvw_t, wstep, st)
+        kmin, kmax, uv = E.w_range(uvw_t, wstep, st)
         st.check()
         NpixFF, NpixKern, Qpx, invert, dl, dm, T = _wkw(kwargs)
         t = W_KERNEL_TABLES.get(theta, wstep, kmin, kmax, NpixFF, NpixKern, Qpx, invert, dl,
                                 dm, T, dtype)
-        return E.KernelTable(t.reshape(-1), False, Qpx, NpixKern), kidx
+        return E.KernelTable(t.reshape(-1), False, Qpx, NpixKern), E.WBins(wstep, kmin, uv)
     fn = kernel_cache if kernel_cache is not None else kernel_fn
     dev = _device_keys(theta, uvw_t, src, nsrc, wstep, fn, kwargs, dtype)
     if dev is not None:
@@ -632,7 +632,7 @@ def _device_keys(theta, uvw_t, src, nsrc, wstep, fn, kwargs, dtype):
         return None
     si, lo, rng = cols
     st = E.Status()
-    _, kmin, kmax = E.w_bins(uvw_t, wstep, st)
+    kmin, kmax, _ = E.w_range(uvw_t, wstep, st)
     st.check()
     nb = kmax - kmin + 1
     space = int(nb) * int(numpy.prod(rng))

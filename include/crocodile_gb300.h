@@ -71,6 +71,15 @@ int cg_frac_coords(const double *uvw, int64_t stride, double lam, int64_t n,
 int cg_w_bins(const double *uvw, int64_t stride, int64_t n, double wstep,
               int32_t *kidx, int32_t *d_minmax, int32_t *h_minmax,
               int32_t *d_status, cg_stream_t stream);
+/* The extremes of uvw in one pass: h_uv = (min, max) over all u and v (the
+ * minimum is -inf when one is NaN) and, for wstep != 0, h_w = (min, max) of the
+ * w bins round(w / wstep) (bins beyond +-1e9 are range errors and left out).
+ * d_work: 24 bytes of device scratch.  Synchronises the stream. */
+int cg_uvw_ranges(const double *uvw, int64_t stride, int64_t n, double wstep, void *d_work,
+                  double *h_uv, int32_t *h_w, int32_t *d_status, cg_stream_t stream);
+/* nslices complex64 kernels of S x S as (S + 1) x (S + 1) with a zero first row
+ * and column. */
+int cg_pad_even(const void *table, int64_t nslices, int S, void *out, cg_stream_t stream);
 /* Same bins against a kernel table that already covers k in [kmin, kmin+nk):
  * kidx[i] = k_i - kmin, bins outside the table are index errors.  Fully
  * stream-ordered (no synchronisation), for steady-state imaging loops. */

@@ -168,3 +168,39 @@ def test_grid_separable_dense(env, N, S):
     O.convgrid(gcf, want, uvw[:, :2], src, vis - dw)
     for got, ref in ((d, dw), (place, dw), (out, want), (out2, want)):
         assert numpy.linalg.norm(got.cpu().numpy() - ref) <= 3e-6 * numpy.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [1, 31, 257, 100000])
+def test_uvw_ranges(env, n):
+    """Extremes and w bins in one pass: equal to numpy's, bins half to even, negative
+    and NaN coordinates."""
+    torch, L, E, S, _ = env
+    rng = numpy.random.default_rng(n)
+    uvw = rng.normal(size=(n, 3)) * 10.0 ** rng.integers(-3, 5, (n, 1))
+    uvw[: n // 2, 2] = 2.5 * rng.integers(-9, 9, n // 2) + 1.25  # halves of the bin width
+    st = E.Status()
+    k = numpy.round(uvw[:, 2] / 2.5)
+    assert E.uvw_ranges(uvw, 2.5, st) == (k.min(), k.max(), (uvw[:, :2].min(), uvw[:, :2].max()))
+    st.check()
+    assert E.uvw_ranges(-numpy.abs(uvw), 0.0, st)[2] == (-numpy.abs(uvw[:, :2]).max(),
+                                                         -numpy.abs(uvw[:, :2]).min())
+    uvw[n - 1, 1] = numpy.nan
+    assert E.uvw_ranges(uvw, 0.0, st)[2][0] == -numpy.inf
+    uvw[n - 1, 2] = 1e12
+    E.uvw_ranges(uvw, 2.5, st)
+    with pytest.raises(AssertionError):
+        st.check()
+    with pytest.raises(ValueError):
+        S.w_cache_imaging(0.1, 1000.0, uvw, None, numpy.zeros(n), wstep=0, NpixFF=32, NpixKern=7,
+                          Qpx=4)
+
+
+@pytest.mark.parametrize("S,G", [(13, 1), (15, 5)])
+def test_pad_even(env, S, G):
+    torch, L, E, _, _ = env
+    t = torch.randn((G, 4, 4, S, S), dtype=E.CF, device="cuda")
+    uvw = torch.zeros((1, 3), dtype=torch.float64, device="cuda")
+    p = E.KernelTable(t.reshape(-1), False, 4, S).padded_even(uvw, 1.0, (128, 128))
+    want = torch.nn.functional.pad(torch.view_as_real(t), (0, 0, 1, 0, 1, 0))
+    assert p.S == S + 1
+    assert torch.equal(torch.view_as_real(p.table).reshape(want.shape), want)
