@@ -2,16 +2,16 @@
 // crocodile/synthesis.py:701-734, for 16 x 16 AW kernels and w sub-kernels of
 // support S <= 16).
 //
+// In FP64 (the complex64 form, k_aw_fftconv_f below, has shorter transforms):
 // out[k, f] = convolve2d(akern_k, W[w_k, f], 'same') is the middle 16 x 16
 // (offset o = (S - 1) / 2) of the full 31 x 31 linear convolution, which a
 // 32 x 32 circular convolution of the zero-padded inputs reproduces exactly.
 // So with FA_k = FFT32(akern_k) / 1024 and FW_wf = FFT32(W[w, f]) (batched
-// cuFFT, complex64), out[k, f] = crop(IFFT32(FA_k * FW_wf)).  The direct form
+// cuFFT), out[k, f] = crop(IFFT32(FA_k * FW_wf)).  The direct form
 // costs 256 x (taps <= 256) complex MACs per output sub-kernel; this one a
 // 1024-point product and a pruned 32 x 32 inverse transform.
 //
-// k_aw_fftconv (complex128 tables; complex64 ones run k_aw_fftconv_f below):
-// one CTA per AW key, FA_k in shared memory, each warp takes sub-kernels f
+// k_aw_fftconv (complex128 tables): one CTA per AW key, FA_k in shared memory, each warp takes sub-kernels f
 // in turn.  Lane = column k2: the warp loads FW_wf row by row
 // (coalesced), multiplies by FA_k, runs a 32-point decimation-in-frequency
 // inverse FFT over k1 in registers (twiddle indices compile-time, table in
@@ -29,19 +29,20 @@ namespace cg {
 
 int fft_plan(int batch, int H, int W, cufftType type, cufftHandle *out);
 
-__constant__ float2 c_tw32[32];    // exp(+2 pi i t / 32)
-__constant__ double2 c_tw32d[32];  // the same in FP64 (complex128 tables)
+__constant__ float2 c_tw24[24];    // exp(+2 pi i t / 24) (complex64 tables)
+__constant__ double2 c_tw32d[32];  // exp(+2 pi i t / 32) (complex128 tables)
 
 namespace {
 
-// the complex type of each precision
+// the complex type of each precision, and its transforms' edge
 template <typename R> struct Cx;
 template <> struct Cx<float> {
   typedef float2 T;
-  static __device__ __forceinline__ T tw(int i) { return c_tw32[i]; }
+  static constexpr int N = 24;
 };
 template <> struct Cx<double> {
   typedef double2 T;
+  static constexpr int N = 32;
   static __device__ __forceinline__ T tw(int i) { return c_tw32d[i]; }
 };
 
@@ -83,33 +84,33 @@ __device__ __forceinline__ void idft32_dif(T (&x)[32]) {
   dif_stage<1>(x);
 }
 
-// FA: akern [nk][16][16] zero-padded to [nk][32][32] and scaled by 1/1024
-template <typename T>
+// FA: akern [nk][16][16] zero-padded to [nk][N][N] and scaled by 1/N^2
+template <typename T, int N>
 __global__ void k_pad_akern(const T *__restrict__ akern, int nk, T *__restrict__ fa) {
-  const int64_t total = (int64_t)nk * 1024;
+  const int64_t total = (int64_t)nk * (N * N);
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e >> 10), r = (int)((e >> 5) & 31), c = (int)(e & 31);
+    const int k = (int)(e / (N * N)), m = (int)(e - (int64_t)k * (N * N)), r = m / N, c = m % N;
     T v;
     v.x = v.y = 0;
     if (r < 16 && c < 16) {
       v = akern[((int64_t)k * 16 + r) * 16 + c];
-      v.x *= (decltype(v.x))(1.0 / 1024.0);
-      v.y *= (decltype(v.x))(1.0 / 1024.0);
+      v.x *= (decltype(v.x))(1.0 / (N * N));
+      v.y *= (decltype(v.x))(1.0 / (N * N));
     }
     fa[e] = v;
   }
 }
 
-// FW: W [nWQ][S][S] (FP64) zero-padded to [nWQ][32][32] (rounded to FP32 for
+// FW: W [nWQ][S][S] (FP64) zero-padded to [nWQ][N][N] (rounded to FP32 for
 // complex64 tables)
-template <typename T>
+template <typename T, int N>
 __global__ void k_pad_w(const double2 *__restrict__ W, int64_t nwq, int S, T *__restrict__ fw) {
-  const int64_t total = nwq * 1024;
+  const int64_t total = nwq * (N * N);
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t g = e >> 10;
-    const int r = (int)((e >> 5) & 31), c = (int)(e & 31);
+    const int64_t g = e / (N * N);
+    const int m = (int)(e - g * (N * N)), r = m / N, c = m % N;
     T v;
     v.x = v.y = 0;
     if (r < S && c < S) {
@@ -185,23 +186,34 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 1) k_aw_fftconv(
   }
 }
 
-// The complex64 form with 16-point register transforms (fft32.h) and one
-// transpose through shared memory in place of the shuffled row pass: per
-// sub-kernel about 800 warp instructions against 1,794.  Column pass (lane =
-// column k2): the 32-point inverse transform over k1 as two 16-point
-// transforms of the even and odd rows, Y[n] = E[n mod 16] + w32^n O[n mod 16]
-// (w32^(n + 16) = -w32^n), evaluated for the 16 kept rows n = o .. o + 15
-// only; they go to shared memory.  Row pass: lane 2r + h takes kept row r and
-// the outputs n2 = 2m + h: Out[2m + h] = DFT16_m[(z[k] + (-1)^h z[k + 16])
-// w32^(k h)], of which the 8 kept ones (n2 in o .. o + 15) are stored.
+// The complex64 form: 24-point circular convolutions in place of 32-point ones.
+// Of the 16 + S - 1 points of the full convolution only the 16 from o =
+// (S - 1) / 2 are kept, so the wrapped-around rest may fall on the others: a
+// period of 24 suffices (the last point, 14 + S, lands on S - 10 < o), and the
+// spectra, which bound this kernel (L1, then L2: read once per sub-kernel), are
+// 576 points instead of 1024.
+//
+// Column pass (lane < 24 = column k2): the inverse transform over k1 as three
+// 8-point register transforms of the rows k1 = c mod 3 (fft32.h), Y[n] = sum_c
+// w24^(c n) F_c[n mod 8], formed for the 16 kept rows only; they go to shared
+// memory.  Row pass: lane 2r + h takes kept row r and the outputs n2 = 2m + h,
+// the 12-point transforms of u[k] = (z[k] + (-1)^h z[k + 12]) w24^(k h): three
+// 4-point ones of k = b mod 3, Out[m] = sum_b w12^(b m) G_b[m mod 4], for the
+// nine m that either half keeps (the halves differ by one m when o is odd).  The
+// 16 x 16 result leaves through shared memory, so that its stores are whole
+// lines.
+//
+// 6000 keys of 256 sub-kernels, S 16: 1.38 ms against 2.21 with 32 points, 8-byte
+// stores scattered over half sectors and 1,058 warp instructions per sub-kernel
+// (852 now); error against 64 bits 3.8e-7 against 4.9e-7.
 template <int S>
 __global__ void __launch_bounds__(256, 3) k_aw_fftconv_f(
     const float2 *__restrict__ fa, const float2 *__restrict__ fw, int nW, int QQ,
     const int32_t *__restrict__ wi, float2 *__restrict__ out, int32_t *status) {
   using f32::cf;
-  __shared__ float2 sfa[32][33];
-  __shared__ float2 srow[8][16][33];  // per warp: the kept rows of the column pass
-  constexpr int o = (S - 1) / 2;
+  constexpr int N = 24, o = (S - 1) / 2, RP = N + 1;  // RP: pitch of the kept rows
+  __shared__ float2 sfa[N][N];
+  __shared__ float2 srow[8][16 * RP];  // per warp: the kept rows, then the result
   const int k = blockIdx.x;
   const int w = wi[k];
   if (w < 0 || w >= nW) {
@@ -209,49 +221,70 @@ __global__ void __launch_bounds__(256, 3) k_aw_fftconv_f(
     return;
   }
   if ((status[ST_RANGE] | status[ST_INDEX]) != 0) return;
-  for (int t = threadIdx.x; t < 1024; t += blockDim.x)
-    sfa[t >> 5][t & 31] = fa[(int64_t)k * 1024 + t];
+  for (int t = threadIdx.x; t < N * N; t += blockDim.x)
+    (&sfa[0][0])[t] = fa[(int64_t)k * (N * N) + t];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = lane >> 1, h = lane & 1;
-  auto mul = [](cf a, float2 b) { return cf{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; };
+  const int r = lane >> 1, h = lane & 1, col = lane < N ? lane : N - 1;
+  float2 *rows = srow[warp];
+  auto mul = [](cf a, float2 b) {
+    return cf{fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x)};
+  };
+  auto mac = [](cf s, cf a, float2 b) {  // s + a b
+    return cf{fmaf(-a.y, b.y, fmaf(a.x, b.x, s.x)), fmaf(a.y, b.x, fmaf(a.x, b.y, s.y))};
+  };
   for (int f = warp; f < QQ; f += 8) {
-    const float2 *src = fw + ((int64_t)w * QQ + f) * 1024;
-    cf e[16], od[16];
+    const float2 *src = fw + ((int64_t)w * QQ + f) * (N * N) + col;
+    {
+      cf F[3][8];
 #pragma unroll
-    for (int b = 0; b < 16; ++b) {
-      const float2 x0 = src[(2 * b) * 32 + lane], a0 = sfa[2 * b][lane];
-      const float2 x1 = src[(2 * b + 1) * 32 + lane], a1 = sfa[2 * b + 1][lane];
-      e[b] = mul(cf{a0.x, a0.y}, x0);
-      od[b] = mul(cf{a1.x, a1.y}, x1);
-    }
-    f32::dft16(e, 1);  // inverse: exp(+2 pi i / 16); output q in slot out_slot(4, q)
-    f32::dft16(od, 1);
+      for (int c = 0; c < 3; ++c) {
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      const int n = o + t, q = n < 16 ? n : n - 16;
-      const cf E = e[f32::out_slot(4, q)], O = mul(od[f32::out_slot(4, q)], c_tw32[q]);
-      const cf y = n < 16 ? f32::cf_add(E, O) : f32::cf_sub(E, O);
-      srow[warp][t][lane] = make_float2(y.x, y.y);
+        for (int a = 0; a < 8; ++a) {
+          const float2 x = __ldg(&src[(3 * a + c) * N]), y = sfa[3 * a + c][col];
+          F[c][a] = mul(cf{y.x, y.y}, x);
+        }
+        f32::dft8(F[c], 1);  // inverse: exp(+2 pi i / 8); output q in slot out_slot(3, q)
+      }
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        const int n = o + t, q = f32::out_slot(3, n & 7);
+        const cf y = mac(mac(F[0][q], F[1][q], c_tw24[n]), F[2][q], c_tw24[2 * n % N]);
+        if (lane < N) rows[t * RP + lane] = make_float2(y.x, y.y);
+      }
     }
     __syncwarp();
-    cf u[16];
+    cf G[3][4];
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      const float2 z0 = srow[warp][r][kk], z1 = srow[warp][r][kk + 16];
-      const cf sum = {z0.x + z1.x, z0.y + z1.y}, dif = {z0.x - z1.x, z0.y - z1.y};
-      u[kk] = h ? mul(dif, c_tw32[kk]) : sum;
-    }
-    __syncwarp();  // srow is rewritten by the next sub-kernel
-    f32::dft16(u, 1);
-    float2 *dst = out + ((int64_t)k * QQ + f) * 256 + r * 16;
-    constexpr int m0e = (o + 1) >> 1, m0o = o >> 1;  // first kept m for h = 0 and 1
+    for (int b = 0; b < 3; ++b) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int me = m0e + j, mo = m0o + j;  // n2 = 2 me, or 2 mo + 1
-      const cf v = h ? u[f32::out_slot(4, mo)] : u[f32::out_slot(4, me)];
-      dst[(h ? 2 * mo + 1 : 2 * me) - o] = make_float2(v.x, v.y);
+      for (int a = 0; a < 4; ++a) {
+        const int kk = 3 * a + b;
+        const float2 z0 = rows[r * RP + kk], z1 = rows[r * RP + kk + 12];
+        const cf sum = {z0.x + z1.x, z0.y + z1.y}, dif = {z0.x - z1.x, z0.y - z1.y};
+        G[b][a] = h ? (kk ? mul(dif, c_tw24[kk]) : dif) : sum;
+      }
+      f32::dft4(G[b], 1);
     }
+    __syncwarp();  // the rows have been read
+    // out n2 = 2 m + h for m = m0 .. m0 + 8; this lane's eight from n2 >= o
+    constexpr int m0 = o >> 1;
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const int m = m0 + j;
+      const cf v = mac(mac(G[0][m & 3], G[1][m & 3], c_tw24[2 * m % N]), G[2][m & 3],
+                       c_tw24[4 * m % N]);
+      const int n = 2 * m + h - o;
+      if (n >= 0 && n < 16) rows[r * 17 + n] = make_float2(v.x, v.y);
+    }
+    __syncwarp();
+    float2 *dst = out + ((int64_t)k * QQ + f) * 256;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const int e = t * 32 + lane;
+      dst[e] = rows[(e >> 4) * 17 + (e & 15)];
+    }
+    __syncwarp();  // rewritten by the next sub-kernel
   }
 }
 
@@ -276,32 +309,33 @@ int aw_fft_run(const typename Cx<R>::T *akern, int nk, const void *W, int nW, in
   CG_REQUIRE(aw_fft_supported(16, S), "FFT AW convolution needs 16 x 16 kernels, S <= 16");
   if (ws_bytes < aw_fft_workspace_bytes(nk, nW, Q))
     return set_error(CG_ERR_WORKSPACE, "AW FFT convolution workspace too small");
-  T tw[32];
-  for (int t = 0; t < 32; ++t) {
-    tw[t].x = (R)std::cos(2.0 * M_PI * t / 32.0);
-    tw[t].y = (R)std::sin(2.0 * M_PI * t / 32.0);
+  constexpr int N = Cx<R>::N;
+  T tw[N];
+  for (int t = 0; t < N; ++t) {
+    tw[t].x = (R)std::cos(2.0 * M_PI * t / N);
+    tw[t].y = (R)std::sin(2.0 * M_PI * t / N);
   }
   if (sizeof(R) == 4)
-    CG_CUDA(cudaMemcpyToSymbolAsync(c_tw32, tw, sizeof(tw), 0, cudaMemcpyHostToDevice, st));
+    CG_CUDA(cudaMemcpyToSymbolAsync(c_tw24, tw, sizeof(tw), 0, cudaMemcpyHostToDevice, st));
   else
     CG_CUDA(cudaMemcpyToSymbolAsync(c_tw32d, tw, sizeof(tw), 0, cudaMemcpyHostToDevice, st));
   T *fa = (T *)ws;
-  T *fw = fa + (size_t)nk * 1024;
+  T *fw = fa + (size_t)nk * (N * N);
   const int64_t nwq = (int64_t)nW * Q * Q;
-  const unsigned gb = (unsigned)std::min<int64_t>(((int64_t)nk * 1024 + 255) / 256,
+  const unsigned gb = (unsigned)std::min<int64_t>(((int64_t)nk * (N * N) + 255) / 256,
                                                   (int64_t)num_sms() * 16);
-  k_pad_akern<T><<<gb, 256, 0, st>>>(akern, nk, fa);
+  k_pad_akern<T, N><<<gb, 256, 0, st>>>(akern, nk, fa);
   CG_LAUNCH("AW FFT pad A");
-  const unsigned gw = (unsigned)std::min<int64_t>((nwq * 1024 + 255) / 256,
+  const unsigned gw = (unsigned)std::min<int64_t>((nwq * (N * N) + 255) / 256,
                                                   (int64_t)num_sms() * 16);
-  k_pad_w<T><<<gw, 256, 0, st>>>((const double2 *)W, nwq, S, fw);
+  k_pad_w<T, N><<<gw, 256, 0, st>>>((const double2 *)W, nwq, S, fw);
   CG_LAUNCH("AW FFT pad W");
   cufftHandle plan;
   int rc;
   for (int pass = 0; pass < 2; ++pass) {
     const int batch = pass ? (int)nwq : nk;
     T *data = pass ? fw : fa;
-    if ((rc = fft_plan(batch, 32, 32, sizeof(R) == 4 ? CUFFT_C2C : CUFFT_Z2Z, &plan))) return rc;
+    if ((rc = fft_plan(batch, N, N, sizeof(R) == 4 ? CUFFT_C2C : CUFFT_Z2Z, &plan))) return rc;
     if (cufftSetStream(plan, st) != CUFFT_SUCCESS)
       return set_error(CG_ERR_CUDA, "cufftSetStream failed");
     const cufftResult r =
