@@ -85,12 +85,12 @@ def _store(sig, entry):
 
 
 def candidates(S, quick=False):
-    """Launch shapes to try: the warp layout over tile edge, work-item size and
+    """Launch shapes to try: the automatic choices; the warp layout over tile edge, work-item size and
     warps per CTA; the owner layout over tile edge, rows per thread and groups;
     the lane layout (S <= 16) over tile edge, work-item size and degridder."""
     tiles = [t for t in ((32, 48) if quick else (16, 24, 32, 48, 64)) if t >= min(S, 16)]
     chunks = (0, 1024) if quick else (0, 512, 2048)
-    out = []
+    out = [{"tile": 0, "chunk": 0, "rows": 0, "groups": 0, "layout": 0}]  # automatic
     if S <= 16:
         # the lane layout, each with the tiled degridder (dvis 0) and the ring
         # degridder (dvis 3)

@@ -264,6 +264,7 @@ struct cg_plan {
   int64_t max_items;
   int chunk;    // visibilities per work item
   int outer;    // window edge of the separable gridder (grid_outer.cu), 0: another gridder
+  int lane_odd; // odd supports on the lane layout's tiles, gridded by the lane kernel
   int lean;     // plan_geometry: the choices that need the least workspace
   int slice_stride;  // lane layout: elements between S x S slices of the table it reads
   int64_t kpad_slices;  // lane layout, slices padded to a 16-byte multiple: slices to copy

@@ -810,20 +810,21 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   int gsize = 0, ngroups = 0;
   bool shared = false;
   if (p->outer) return outer_launch(p, kt, vv, nullptr, weight, mode, gg, s);
-  const int layout = layout_for(p->kd);
-  // Automatic, another gridder than the plan's layout names: taps straight into
-  // the grid while few visibilities meet in a cell (L2 takes atomics on one
-  // address in turn) and, for supports that fill the lane gridder's lanes, few
-  // visibilities in all (direct / lane or warp gridder, us: S 9, 2M on 2048^2: 383 /
-  // 437, on 300^2: 685 / 432; S 8, 2M on 2048^2: 299 / 362; S 6, 500k: 63 / 100; S 12,
-  // 2M: 607 / 579; S 16, 500k: 241 / 172, 50k on 1024^2: 44 / 55; S 15, 1M: 441 / 458).
+  const bool automatic = t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0;
+  const bool lane = layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0);
+  // Automatic: taps straight into the grid while few visibilities meet in a cell
+  // (L2 takes atomics on one address in turn), and, where the lane kernel can
+  // take its place, few visibilities in all (direct / lane / warp gridder, us: S 8,
+  // 150k on 1024^2: 32 / 42; 500k on 2048^2: 70 / 73; 2M: 300 / 202; S 12, 500k: 146 /
+  // 152, 2M: 586 / 455; S 16, 60k: 38 / 46, 150k: 79 / 64; S 6, 3M on 4096^2: 296 / 354,
+  // 2M on 2048^2: 223 / 221; S 9, 2M: 382 / 301 / 453, on 300^2: 685 / - / 432).  A
+  // wait limit of 0 keeps to the lane kernel (lane_launch).
   const double rho = (double)p->n / ((double)p->H * (double)p->W * (double)p->layers);
-  if (t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0 && S <= 16 && rho < 1.5 &&
-      (S <= 11 || layout != CG_LAYOUT_LANE || p->n < 100000))
+  const bool few = !lane || (S <= 6 ? rho < 0.4 : p->n < (S == 16 ? 120000 : 450000));
+  if (automatic && S <= 16 && rho < 1.5 && few && !(lane && wait_cycles() == 0))
     return direct_grid_launch(p, kt, vv, weight, mode, gg, s);
-  if (layout == CG_LAYOUT_LANE)
-    return lane_launch(p, kt, vv, weight, mode, gg, nullptr, nullptr, 0, false, s);
-  if (layout != CG_LAYOUT_OWNER) {
+  if (lane) return lane_launch(p, kt, vv, weight, mode, gg, nullptr, nullptr, 0, false, s);
+  if (layout_for(p->kd) != CG_LAYOUT_OWNER) {
     const int need = (S * S + 31) / 32;
     int maxt = 1;
     while (maxt < need) maxt *= 2;
@@ -933,14 +934,13 @@ int cg_degrid(const cg_plan *p, const void *ktab, const void *grid, void *out,
   //    16.1M visibilities, 12.4 GB table: 3.67 ms, tiled 3.91, direct 4.56;
   //    1.35M, 4.1 GB: 0.387 both; 1.75M on 8192^2, 1.8 GB: direct 0.43, ring
   //    0.73; below that direct leads).
-  //  - S 13 to 15, 4-D, some hundred visibilities to a tile: rows that do not
-  //    fill the lanes (S 15, 3M visibilities on 4096^2: tiled 592, direct 647
-  //    us; 300k on 2048^2: 95 against 85).
+  //  - S 14 and 15, 4-D, dense tiles: rows that do not fill the lanes (S 15, 2M
+  //    visibilities on 2048^2: tiled 380, direct 428 us; 300k: 98 against 85).
   const int64_t slices = (int64_t)p->kd.G * p->kd.Q * (p->kd.sep ? 1 : p->kd.Q);
   const int64_t table = slices * p->kd.S * (p->kd.sep ? 1 : p->kd.S) * (int64_t)sizeof(float2);
   const int64_t per_tile = p->n / std::max(p->ntx * p->nty * p->layers, 1);
   const bool streams = lane && table > ((int64_t)4 << 30) && per_tile >= 16;
-  const bool ragged = !p->kd.sep && p->kd.S >= 13 && p->kd.S <= 15 && per_tile >= 400;
+  const bool ragged = !p->kd.sep && (p->kd.S == 14 || p->kd.S == 15) && per_tile >= 100;
   if (dvis == 3 || (dvis == 0 && streams)) {
     const int rc = ring_degrid_launch(p, (const float2 *)ktab, (const float2 *)grid,
                                       (float2 *)out, s);
@@ -1003,7 +1003,7 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
     return outer_launch(p, (const float2 *)ktab, (const float2 *)vis_in, (const float2 *)vis_out,
                         nullptr, residual ? 3 : 0, (float2 *)grid_out, s);
   }
-  if (layout_for(p->kd) == CG_LAYOUT_LANE)
+  if (layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0))
     return lane_launch(p, (const float2 *)ktab, (const float2 *)vis_in, nullptr, 0,
                        (float2 *)grid_out, (const float2 *)grid_in, (float2 *)vis_out, residual,
                        true, s);

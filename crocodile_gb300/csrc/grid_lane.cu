@@ -399,9 +399,22 @@ int lane_launch(const cg_plan *p, const float2 *ktab, const float2 *vis, const f
   const int KS = p->kd.sep ? S : p->slice_stride;
   const int prc = padded_table(p, ktab, s);
   if (prc) return prc;
-  const bool bulk = !p->kd.sep && (KS * 8) % 16 == 0 && ((uintptr_t)ktab & 15) == 0;
-
   const cg_tuning t = tuning();
+  // Streaming the slices through shared memory writes and reads them there beside
+  // the window's read-modify-write, and the stages' room costs warps: taps by
+  // loads, one visibility ahead, in CTAs of 4 warps (20 to an SM, against 14 in
+  // one) are faster wherever the table is found in L2 or lightly used, and in the
+  // fused pass always.  Streamed / loaded, us, S 16: w-projection 2M, 4096^2, 604 /
+  // 485, fused 926 / 741; AW 1.75M, 8192^2, 1.8 GB, 694 / 646; dense tiles and a
+  // table of gigabytes: AW 2M, 4096^2, 1.6 GB, 598 / 615 (fused 934 / 812), 16.1M, 12 GB,
+  // 4116 / 4273 (fused 6381 / 5712).  A lane layout asked for by the tuning streams,
+  // and so does a wait limit of 0, whose time-outs only the streams have.
+  const int64_t table = (int64_t)p->kd.G * p->kd.Q * p->kd.Q * SS * (int64_t)sizeof(float2);
+  const int64_t per_tile = p->n / std::max(p->ntx * p->nty * p->layers, 1);
+  const bool stream = t.layout == CG_LAYOUT_LANE || wait_cycles() == 0 ||
+                      (!fused && table > ((int64_t)1 << 30) && per_tile >= 16);
+  const bool bulk = stream && !p->kd.sep && (KS * 8) % 16 == 0 && ((uintptr_t)ktab & 15) == 0;
+
   LaneArgs P;
   P.ktab = ktab;
   P.vis = vis;
@@ -435,7 +448,8 @@ int lane_launch(const cg_plan *p, const float2 *ktab, const float2 *vis, const f
   CG_REQUIRE(fit >= 1, "lane-layout window does not fit in shared memory (%zu bytes per warp)",
              off);
   const int warps = std::min(fit, t.groups > 0 ? t.groups
-                                               : (int)std::max<size_t>(1, (220u << 10) / off));
+                                  : bulk       ? (int)std::max<size_t>(1, (220u << 10) / off)
+                                               : 4);
   void *fn = p->kd.sep ? (fused ? lane_kernel_for<true, false, true>(maxt, SS, p->pitch)
                                 : lane_kernel_for<true, false, false>(maxt, SS, p->pitch))
                        : bulk ? (fused ? lane_kernel_for<false, true, true>(maxt, SS, p->pitch)

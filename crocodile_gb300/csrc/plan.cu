@@ -636,11 +636,22 @@ static int outer_edge(const cg_plan &p, int &T) {
   return 24;
 }
 
+// 4-D tables of odd support under no tuning and no requested tile: the lane
+// layout's 16-cell tiles (layout_for gives the lane layout to even supports,
+// whose slices it can stream), for the lane kernel with taps by loads.
+static bool lane_odd(const cg_plan &p) {
+  const cg_tuning t = tuning();
+  return !p.lean && !p.kd.sep && p.kd.S <= 16 && p.kd.S % 2 == 1 && p.tile_req == 0 &&
+         t.tile == 0 && t.layout == 0 && (int64_t)p.kd.G * p.kd.Q * p.kd.Q < INT32_MAX;
+}
+
 static void plan_geometry(cg_plan &p) {
   if (p.mode == CG_PLAN_TILED) {
     int outer_T = 0;
     p.outer = outer_edge(p, outer_T);
-    p.T = p.outer ? outer_T : tile_edge(p.kd, p.tile_req);
+    p.lane_odd = lane_odd(p);
+    const bool lane = p.lane_odd || layout_for(p.kd) == CG_LAYOUT_LANE;
+    p.T = p.outer ? outer_T : p.lane_odd ? 16 : tile_edge(p.kd, p.tile_req);
     p.ntx = (p.W + p.T - 1) / p.T;
     p.nty = (p.H + p.T - 1) / p.T;
     // Morton blocks of up to 32 x 32 tiles (no larger than the grid needs)
@@ -656,7 +667,7 @@ static void plan_geometry(cg_plan &p) {
     // in-tile coordinate shifted by subshift is always below 2^sublog.
     int full = 0;
     while ((4 << full) < p.T) ++full;
-    p.sublog = p.outer || layout_for(p.kd) == CG_LAYOUT_LANE ? 0 : full;
+    p.sublog = p.outer || lane ? 0 : full;
     p.subshift = 2 + full - p.sublog;
     // keep the histogram (4 B per bucket) within 2^24 buckets: coarser sub-tiles
     // for very large grid stacks
@@ -683,7 +694,7 @@ static void plan_geometry(cg_plan &p) {
     };
     p.chunk = t.chunk > 0 ? t.chunk
               : p.outer   ? clamp(per_warp, 32, 256)
-              : layout_for(p.kd) == CG_LAYOUT_LANE
+              : lane
                   ? (p.lean ? 512 : clamp(per_warp, 64, 512))
                   : (int)std::min<int64_t>(
                         2048, std::max<int64_t>(256, p.n / (int64_t)(num_sms() * 16) + 1));

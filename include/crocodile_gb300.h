@@ -108,7 +108,8 @@ typedef struct {
  * visibility, shared-memory atomics), CG_LAYOUT_OWNER (threads own window
  * cells by position mod S and keep running sums in registers) or
  * CG_LAYOUT_LANE (one warp per work item with a private window, lanes own
- * cells by position mod S, kernel slices streamed by bulk copies; S <= 16;
+ * cells by position mod S, kernel slices streamed by bulk copies when this
+ * layout is asked for; S <= 16;
  * also selects the lane form of cg_degrid_grid; odd S * S slices stream
  * from a padded copy of the table in the plan's workspace); rows: row
  * residues per owner-layout thread (1..8), or bulk-copy stages per
@@ -123,9 +124,12 @@ typedef struct {
  * S <= 16, 16-byte slices) through the ring degridder: the item's window in
  * shared memory, each warp's slices by bulk copies through a 2-stage ring
  * (others as 0).  All of them but 1 sum a visibility's taps in the same order.
- * layout 0 picks CG_LAYOUT_LANE (with 16-cell tiles) for
- * non-separable tables with even S <= 16, whose slices stream by bulk
- * copies as they are, and CG_LAYOUT_WARP otherwise.  Process-wide. */
+ * layout 0 lets each plan and call choose: non-separable tables, S <= 16, get
+ * 16-cell tiles and the lane kernel (its slices by loads, or by bulk copies
+ * where the table is large and the tiles dense), or taps added straight to the
+ * grid where visibilities are few; separable tables, S <= 16, the gridder with
+ * its window in registers or again the direct one; wider supports
+ * CG_LAYOUT_WARP.  Process-wide. */
 #define CG_LAYOUT_WARP 1
 #define CG_LAYOUT_OWNER 2
 #define CG_LAYOUT_LANE 3

@@ -204,3 +204,36 @@ def test_pad_even(env, S, G):
     want = torch.nn.functional.pad(torch.view_as_real(t), (0, 0, 1, 0, 1, 0))
     assert p.S == S + 1
     assert torch.equal(torch.view_as_real(p.table).reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("S", [1, 3, 6, 8, 9, 11, 12, 15, 16])
+def test_grid_lane_loads(env, S):
+    """4-D tables on dense visibilities (the lane kernel with taps by loads, odd
+    supports on its tiles too), grids that end inside a tile and a stack, gridding and
+    the fused pass against the oracle.  Tolerance 3e-6: a few hundred complex64
+    products summed per cell."""
+    torch, L, E, _, O = env
+    for N, layers in ((81, 1), (48, 2)):
+        n = 3 * N * N
+        rng, uvw, gcf, src = _case(S + N, n, S, 2, False, G=2)
+        vis = (rng.normal(size=n) + 1j * rng.normal(size=n)).astype(numpy.complex64)
+        lay = rng.integers(0, layers, n).astype(numpy.int32)
+        kt = E.KernelTable.from_gcf(gcf, 1, E.CF)
+        plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32),
+                      layers=None if layers == 1 else (layers, lay))
+        assert plan.info()["tile"] == 16
+        v = E.cuda_tensor(vis, E.CF)
+        got = plan.grid(kt, v, torch.zeros((layers, N, N), dtype=E.CF, device="cuda"))
+        model = E.cuda_tensor(_grids(torch, rng, N, layers), E.CF)
+        out = torch.zeros_like(got)
+        d = plan.degrid_grid(kt, model, v, out, residual=True).cpu().numpy()
+        plan.check()
+        mh = model.cpu().numpy().astype(complex)
+        for p in range(layers):
+            s = lay == p
+            dw = O.convdegrid(gcf, mh[p], uvw[s, :2], src[s])
+            want, res = (numpy.zeros((N, N), dtype=complex) for _ in range(2))
+            O.convgrid(gcf, want, uvw[s, :2], src[s], vis[s])
+            O.convgrid(gcf, res, uvw[s, :2], src[s], vis[s] - dw)
+            for a, b in ((got[p].cpu().numpy(), want), (d[s], dw), (out[p].cpu().numpy(), res)):
+                assert numpy.linalg.norm(a - b) <= 3e-6 * numpy.linalg.norm(b)
