@@ -164,16 +164,39 @@ __global__ void __launch_bounds__(OUTER_THREADS) k_grid_outer(TiledArgs A, Outer
       b += 32;
       continue;
     }
+    bool finite = true;
 #pragma unroll
     for (int r = 0; r < RY; ++r)
 #pragma unroll
-      for (int c = 0; c < CX; ++c) {
-        const float2 a = acc[r][c];
-        const int gy = org.wy0 + ly + r, gx = org.wx0 + lx + LX * c;
-        if ((a.x != 0.f || a.y != 0.f) && gy < A.H && gx < A.W)
-          atomicAdd(&O.grid[org.layer_off + (size_t)gy * A.W + gx], a);
-        acc[r][c] = make_float2(0.f, 0.f);
+      for (int c = 0; c < CX; ++c)
+        finite = finite && fabsf(acc[r][c].x) < INFINITY && fabsf(acc[r][c].y) < INFINITY;
+    if (__all_sync(0xffffffffu, finite)) {
+#pragma unroll
+      for (int r = 0; r < RY; ++r)
+#pragma unroll
+        for (int c = 0; c < CX; ++c) {
+          const float2 a = acc[r][c];
+          const int gy = org.wy0 + ly + r, gx = org.wx0 + lx + LX * c;
+          if ((a.x != 0.f || a.y != 0.f) && gy < A.H && gx < A.W)
+            atomicAdd(&O.grid[org.layer_off + (size_t)gy * A.W + gx], a);
+        }
+    } else {
+      // a NaN or infinity, which the zeros around a footprint would spread over
+      // the window: this item's taps one by one
+      for (int j = 0; j < w.count; ++j) {
+        const VisRec q = A.recs[w.start + j];
+        const float2 u = value(A.perm[w.start + j]);
+        for (int t = lane; t < S * S; t += 32) {
+          const int dy = t / S, dx = t - dy * S;
+          const float2 f = cmul(O.ktab[q.k0 * S + dy], O.ktab[q.k1 * S + dx]);
+          atomicAdd(&O.grid[org.layer_off + (size_t)(q.y0 + dy) * A.W + q.x0 + dx], cmul(f, u));
+        }
       }
+    }
+#pragma unroll
+    for (int r = 0; r < RY; ++r)
+#pragma unroll
+      for (int c = 0; c < CX; ++c) acc[r][c] = make_float2(0.f, 0.f);
     it += nw;
     if (it >= nitems) return;
     w = wn;

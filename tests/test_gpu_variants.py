@@ -237,3 +237,28 @@ def test_grid_lane_loads(env, S):
             O.convgrid(gcf, res, uvw[s, :2], src[s], vis[s] - dw)
             for a, b in ((got[p].cpu().numpy(), want), (d[s], dw), (out[p].cpu().numpy(), res)):
                 assert numpy.linalg.norm(a - b) <= 3e-6 * numpy.linalg.norm(b)
+
+
+@pytest.mark.parametrize("S", [1, 9, 16])
+@pytest.mark.parametrize("bad", [complex("nan"), complex("inf")])
+def test_grid_separable_not_finite(env, S, bad):
+    """A visibility that is not finite: only its footprint's cells are lost, also where
+    the gridder keeps its window in registers (dense visibilities); the others as
+    ever, 3e-6 as for test_grid_separable_dense."""
+    torch, L, E, _, O = env
+    N, n = 96, 60000
+    rng, uvw, gcf, src = _case(S, n, S, 2, True, G=2)
+    vis = (rng.normal(size=n) + 1j * rng.normal(size=n)).astype(numpy.complex64)
+    vis[777] = bad
+    kt = E.KernelTable.from_gcf(gcf, 1, E.CF)
+    plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32))
+    got = plan.grid(kt, E.cuda_tensor(vis, E.CF),
+                    torch.zeros((N, N), dtype=E.CF, device="cuda")).cpu().numpy()
+    plan.check()
+    want = numpy.zeros((N, N), dtype=complex)
+    with numpy.errstate(invalid="ignore"):
+        O.convgrid(gcf, want, uvw[:, :2], src, vis)
+    ok = numpy.isfinite(want)
+    assert ok.sum() == N * N - S * S
+    numpy.testing.assert_array_equal(numpy.isfinite(got), ok)
+    assert numpy.linalg.norm(got[ok] - want[ok]) <= 3e-6 * numpy.linalg.norm(want[ok])
