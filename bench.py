@@ -13,7 +13,7 @@ Q 8, 101 w-kernels.
 One step = plan (bit-exact FP64 cell assignment, tile sort, work list) + FP32
 tiled gridding + FP32 tiled degridding of all visibilities, inputs resident
 in HBM.  The same line reports the plain FP64 form (complex128, FP64
-atomics, one launch per w-plane), FP32-vs-FP64 errors, the fused
+atomics, in the order of the w-planes), FP32-vs-FP64 errors, the fused
 degrid+grid pass, end to end with host buffers, the roofline of the dominant
 kernel, the other configurations and a single-core CPU baseline.
 
@@ -417,7 +417,7 @@ class WProjGpu(GpuWorkload):
         self.kt = E.KernelTable(E.w_kernels(w.theta, self.wlist, npff, self.S, self.Q,
                                             dtype=E.CF).reshape(-1), False, self.Q, self.S)
         self._alloc_ws()
-        self.groups_desc = "one launch per w-plane (%d)" % self.nk
+        self.groups_desc = "in the order of the w-planes (%d)" % self.nk
 
     def tune_kidx(self):
         return self.E.w_bins(self.uvw, self.wstep, self.st)[0]
@@ -465,7 +465,7 @@ class AWGpu(GpuWorkload):
                                       phase_ms=getattr(self, "phase_ms", None))
         self.kt, self.rows = self.op.ktab, self.op.rows
         self._alloc_ws()
-        self.groups_desc = "one launch per w-plane (%d)" % self.op.nbins
+        self.groups_desc = "in the order of the w-planes (%d)" % self.op.nbins
 
     def tune_kidx(self):
         return self.rows
@@ -486,7 +486,7 @@ class AWGpu(GpuWorkload):
 
     def plain(self, steps):
         """(ms per plain FP64 step, FP32-vs-FP64 errors): the same AW kernels held as
-        complex128, FP64 atomics, one launch per w-plane."""
+        complex128, FP64 atomics, in the order of the w-planes."""
         E, torch, op, w = self.E, self.torch, self.op, self.w
         torch.cuda.synchronize()
         t0 = time.perf_counter()

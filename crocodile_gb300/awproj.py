@@ -25,7 +25,7 @@ class AWProjection:
     uvw [n, 3] (wavelengths), a1, a2 [n] antenna indices, beams [nant, F, F]
     complex far fields of the antennas (A-kernel = kernel_oversample(beam, 1,
     SA)), wstep: w-bin width, w-kernels w_kernel(theta, wbin, NpixFF, S, Q).
-    fp64=True also prepares the plain FP64 form (one launch per w-plane).
+    fp64=True also prepares the plain FP64 form (in the order of the w-planes).
     phase_ms: a dict that receives the host time of each set-up phase (the
     device synchronised at every phase boundary), for profiling."""
 
@@ -77,7 +77,7 @@ class AWProjection:
 
     def enable_fp64(self):
         """Prepare the plain FP64 form: the same AW kernels held as complex128 and a
-        groups plan with one launch per w-plane."""
+        groups plan in the order of the w-planes."""
         st = self.status
         Q, SA = self.ktab.Q, self.ktab.S
         self.ktab64 = E.KernelTable(E.aw_kernels(*self._aw_args, dtype=E.CD,

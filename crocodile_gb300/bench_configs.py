@@ -270,7 +270,7 @@ def measure_aw(steps=5, nvis=None, fp64=True):
             "plain_fp64_mvis_s": n / ms64 / 1e3, "speedup": ms64 / ms,
             "fused_ms": ms_fused, "fused_mvis_s": n / ms_fused / 1e3,
             "fused_speedup": ms64 / ms_fused,
-            "plain_form": "complex128, FP64 atomics, one launch per w-plane (%d)" % op.nbins,
+            "plain_form": "complex128, FP64 atomics, in the order of the w-planes (%d)" % op.nbins,
             "rel_err_grid": _rel(g, g64), "rel_err_degrid": _rel(out["v"], out["v64"])}
 
 

@@ -2,13 +2,14 @@
 //
 // The plain form is the accuracy and speed comparator of the FP32 tiled
 // path: complex128 data, one thread per (visibility, tap) with FP64
-// atomicAdd into the grid, one launch per kernel group (w-plane or AW
-// group), no tiling, no shared memory, no register accumulation.  It
+// atomicAdd into the grid in the order of the kernel groups (w-planes or AW
+// groups), no tiling, no shared memory, no register accumulation.  It
 // consumes a CG_PLAN_GROUPS plan, whose records are the same bit-exact cell
 // assignment as the tiled path.  Replaces convgrid/convdegrid
 // (crocodile/synthesis.py:464-503) at full reference precision.
 //
 // Boxcar gridding replaces grid/degrid (synthesis.py:389-416).
+#include <algorithm>
 #include "cg_internal.cuh"
 
 namespace cg {
@@ -189,6 +190,20 @@ static PlainArgs plain_args(const cg_plan *p) {
   return A;
 }
 
+// The visibilities of one layer's grid: its kernel groups are neighbouring
+// buckets, so one launch takes them all.  A launch per group left the GPU with
+// some thousand visibilities at a time (50,000 visibilities in 31 groups, S 9,
+// FP64 w_cache_imaging and w_cache_predict together: 853 us, and 379 without
+// those launches and, with one grid, without the groups' ranges on the host).
+static void plain_range(const cg_plan *p, int layer, int64_t &start, int64_t &count) {
+  start = 0;
+  count = p->n;  // (with errors fewer are sorted, and the kernels return)
+  if (p->layers == 1) return;
+  const int g0 = layer * p->gper, g1 = g0 + p->gper - 1;
+  start = p->h_offsets[g0];
+  count = p->h_offsets[g1] + p->h_counts[g1] - start;
+}
+
 }  // namespace cg
 
 using namespace cg;
@@ -202,13 +217,16 @@ int cg_grid_fp64(const cg_plan *p, const void *ktab, const void *vis, void *grid
   CG_REQUIRE(ktab && vis && grid, "NULL argument");
   PlainArgs A = plain_args(p);
   const int SS = p->kd.S * p->kd.S;
-  for (int g = 0; g < p->nbuckets; ++g) {
-    const int c = p->h_counts[g];
-    if (!c) continue;
-    const int64_t threads = (int64_t)c * SS;
-    double *layer_grid = (double *)grid + 2 * (size_t)(g / p->gper) * p->H * p->W;
-    k_grid_plain<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        A, p->h_offsets[g], c, (const double2 *)ktab, (const double2 *)vis, layer_grid);
+  const int64_t most = (int64_t)INT32_MAX * 256 / SS;  // to a launch
+  for (int l = 0; l < p->layers; ++l) {
+    int64_t start, c;
+    plain_range(p, l, start, c);
+    double *layer_grid = (double *)grid + 2 * (size_t)l * p->H * p->W;
+    for (; c > 0; start += most, c -= most) {
+      const int m = (int)std::min(c, most);
+      k_grid_plain<<<(unsigned)(((int64_t)m * SS + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+          A, (int)start, m, (const double2 *)ktab, (const double2 *)vis, layer_grid);
+    }
   }
   CG_LAUNCH("grid_fp64");
   return CG_OK;
@@ -220,13 +238,14 @@ int cg_degrid_fp64(const cg_plan *p, const void *ktab, const void *grid, void *o
   if (p->n == 0) return CG_OK;
   CG_REQUIRE(ktab && grid && out, "NULL argument");
   PlainArgs A = plain_args(p);
-  for (int g = 0; g < p->nbuckets; ++g) {
-    const int c = p->h_counts[g];
+  for (int l = 0; l < p->layers; ++l) {
+    int64_t start, c;
+    plain_range(p, l, start, c);
     if (!c) continue;
-    const double2 *layer_grid = (const double2 *)grid + (size_t)(g / p->gper) * p->H * p->W;
-    const int64_t threads = (int64_t)c * PLAIN_LANES;
+    const double2 *layer_grid = (const double2 *)grid + (size_t)l * p->H * p->W;
+    const int64_t threads = c * PLAIN_LANES;
     k_degrid_plain<<<(unsigned)((threads + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
-        A, p->h_offsets[g], c, (const double2 *)ktab, layer_grid, (double2 *)out);
+        A, (int)start, (int)c, (const double2 *)ktab, layer_grid, (double2 *)out);
   }
   CG_LAUNCH("degrid_fp64");
   return CG_OK;

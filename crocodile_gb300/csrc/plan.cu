@@ -902,7 +902,8 @@ size_t plan_workspace_least(const cg_kernel_desc *kd, int H, int W, int64_t n) {
   return std::min(need, layout_of(p).total);
 }
 
-// Heap plan; the groups form also copies the group ranges to the host.
+// Heap plan; the groups form of a stack of grids also copies the group ranges to
+// the host.
 static int plan_create_heap(cg_plan **out, int mode, const cg_kernel_desc *kd, int H, int W,
                             const double *uvw, int64_t stride, double lam, const int32_t *kidx,
                             double wstep, int kmin, int layers, const int32_t *layer,
@@ -918,7 +919,7 @@ static int plan_create_heap(cg_plan **out, int mode, const cg_kernel_desc *kd, i
     delete p;
     return rc;
   }
-  if (mode == CG_PLAN_GROUPS) {
+  if (mode == CG_PLAN_GROUPS && layers > 1) {
     p->h_counts = (int32_t *)malloc((size_t)p->nbuckets * 4);
     p->h_offsets = (int32_t *)malloc((size_t)p->nbuckets * 4);
     cudaError_t e = cudaSuccess;

@@ -180,7 +180,7 @@ class Plan:
         """wbins=(wstep, kmin): take each visibility's kernel group from its w bin
         (round(w / wstep) - kmin) inside the plan's coordinate pass.
         layers=(L, layer): grid visibility i into grid layer[i] of a stack of L grids.
-        groups=(G, group): plain form only, one launch per group[i] in [0, G).
+        groups=(G, group): plain form only, in the order of group[i] in [0, G).
         tile: this plan's grid tile edge (0: the tuning / automatic choice).
         kidx may be a WBins, which stands for wbins."""
         require_cuda()

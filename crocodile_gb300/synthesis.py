@@ -13,7 +13,7 @@ Precision: the default ``precision="fp32"`` grids complex64 visibilities with
 FP32 products and accumulation in the tiled persistent kernels, while cell
 assignment and w binning stay bit-exact FP64 and kernels are generated in
 FP64.  ``precision="fp64"`` selects the plain complex128 form (FP64 atomics,
-one launch per kernel group).  Drivers accept ``precision=`` as an extra
+in the order of the kernel groups).  Drivers accept ``precision=`` as an extra
 keyword; ``set_precision`` changes the module default.
 
 Small host-side helpers that only reshape or describe arrays (coordinates,

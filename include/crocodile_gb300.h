@@ -167,7 +167,7 @@ int cg_fft_timeouts(int32_t *count, int reset);
 typedef struct cg_plan cg_plan;
 
 #define CG_PLAN_TILED 0  /* FP32 tiled gridder/degridder (cg_grid, cg_degrid) */
-#define CG_PLAN_GROUPS 1 /* plain FP64 form, one launch per kernel group */
+#define CG_PLAN_GROUPS 1 /* plain FP64 form, in the order of the kernel groups */
 
 size_t cg_plan_workspace_bytes(int mode, int64_t n, int H, int W,
                                const cg_kernel_desc *kd);
@@ -201,7 +201,7 @@ typedef struct {
   int kmin;
   /* CG_PLAN_GROUPS only: launch group per visibility (device int32 [n]) in
    * [0, ngroups), e.g. the w-plane, when each visibility's kernel row (kidx)
-   * is finer than the launches (AW kernels: one launch per w-plane). */
+   * is finer than that order (AW kernels: by w-plane). */
   const int32_t *group;
   int ngroups;
   /* Tiled mode: grid tile edge for this plan (multiple of 4, <= 64), or 0 for
@@ -306,7 +306,7 @@ int cg_grid_noalloc(const cg_kernel_desc *kd, int H, int W, const double *uvw,
                     int32_t *d_status, cg_stream_t stream);
 
 /* Plain FP64 form of the same two operations (c128 data, FP64 atomics,
- * one launch per kernel group): the accuracy and speed comparator.
+ * in the order of the kernel groups): the accuracy and speed comparator.
  * Needs a CG_PLAN_GROUPS plan. */
 int cg_grid_fp64(const cg_plan *plan, const void *ktab_c128,
                  const void *vis_c128, void *grid_c128, cg_stream_t stream);

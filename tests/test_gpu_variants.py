@@ -262,3 +262,34 @@ def test_grid_separable_not_finite(env, S, bad):
     assert ok.sum() == N * N - S * S
     numpy.testing.assert_array_equal(numpy.isfinite(got), ok)
     assert numpy.linalg.norm(got[ok] - want[ok]) <= 3e-6 * numpy.linalg.norm(want[ok])
+
+
+@pytest.mark.parametrize("layers,n", [(1, 1), (1, 500), (4, 3), (4, 500)])
+def test_plain_fp64_stack(env, layers, n):
+    """The plain form's launches, one to each grid of a stack (some grids without a
+    visibility, kernels without one, a last block with idle threads).  Tolerance as
+    for test_plain_fp64_degrid, n terms to a cell at most."""
+    torch, L, E, _, O = env
+    N, S, G = 64, 5, 3
+    rng, uvw, gcf, src = _case(n, n, S, 2, True, G=G)
+    vis = rng.normal(size=n) + 1j * rng.normal(size=n)
+    lay = rng.integers(0, layers, n).astype(numpy.int32)
+    lay[lay == 2] = 0
+    src[src == 1] = 0
+    kt = E.KernelTable.from_gcf(gcf, 1, E.CD)
+    plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32), mode=L.CG_PLAN_GROUPS,
+                  layers=None if layers == 1 else (layers, lay))
+    v = E.cuda_tensor(vis, E.CD)
+    grid = plan.grid_fp64(kt, v, torch.zeros((layers, N, N), dtype=E.CD, device="cuda"))
+    model = E.cuda_tensor(rng.normal(size=(layers, N, N)) * (1 + 2j), E.CD)
+    d = plan.degrid_fp64(kt, model).cpu().numpy()
+    plan.check()
+    tol = 4 * (max(n, S * S) + 8) * S * 2.0 ** -53
+    for p in range(layers):
+        s = lay == p
+        want = numpy.zeros((N, N), dtype=complex)
+        O.convgrid(gcf, want, uvw[s, :2], src[s], vis[s])
+        dw = O.convdegrid(gcf, model[p].cpu().numpy(), uvw[s, :2], src[s])
+        for a, b in ((grid[p].cpu().numpy(), want), (d[s], dw)):
+            if b.size:
+                assert numpy.abs(a - b).max() <= tol * max(numpy.abs(b).max(), 1.0)
