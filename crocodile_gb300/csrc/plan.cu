@@ -287,6 +287,149 @@ __global__ void k_plan_items(int ntiles, int sublog, const int32_t *__restrict__
   }
 }
 
+// The whole of the above (bucket scan, item counts, their scan, items) in one
+// block for small grids, where launches are most of a plan's time.
+static constexpr int PLAN_SMALL_BUCKETS = 16384;
+
+__device__ __forceinline__ void write_items(int tile, int off, int count, int chunk, int base,
+                                            WorkItem *items) {
+  for (int j = 0; j * chunk < count; ++j) {
+    WorkItem w;
+    w.tile = tile;
+    w.start = off + j * chunk;
+    w.count = min(chunk, count - j * chunk);
+    w.pad = 0;
+    items[base + j] = w;
+  }
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_plan_small(
+    int nbuckets, int ntiles, int sublog, const int32_t *__restrict__ counts, int chunk,
+    int32_t *__restrict__ offsets, WorkItem *__restrict__ items, int32_t *__restrict__ nitems) {
+  __shared__ int s_warp[33];
+  int carry = 0;
+  for (int b0 = 0; b0 < nbuckets; b0 += SCAN_TILE) {
+    const int base = b0 + threadIdx.x * SCAN_PER_THREAD;
+    int v[SCAN_PER_THREAD], sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) {
+      v[k] = base + k < nbuckets ? counts[base + k] : 0;
+      sum += v[k];
+    }
+    int run = carry + block_exclusive_scan(sum, s_warp, total);
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) {
+      if (base + k < nbuckets) offsets[base + k] = run;
+      run += v[k];
+    }
+    carry += total;
+  }
+  const int n = carry;
+  carry = 0;
+  __syncthreads();  // the offsets of every bucket
+  for (int t0 = 0; t0 < ntiles; t0 += SCAN_THREADS) {
+    const int t = t0 + threadIdx.x;
+    int off = 0, c = 0, total;
+    if (t < ntiles) {
+      const int next = (t + 1) << (2 * sublog);
+      off = offsets[t << (2 * sublog)];
+      c = (next < nbuckets ? offsets[next] : n) - off;
+    }
+    const int m = (c + chunk - 1) / chunk;
+    const int at = carry + block_exclusive_scan(m, s_warp, total);
+    write_items(t, off, c, chunk, at, items);
+    carry += total;
+  }
+  if (threadIdx.x == 0) *nitems = carry;
+}
+
+// Larger grids whose buckets are tiles: both scans as one (counts in the lower
+// half of a 64-bit value, items in the upper), each block its SCAN_TILE buckets,
+// the last block to finish the blocks' totals; then the items.
+__device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned long long v,
+                                                                     unsigned long long *s_warp,
+                                                                     unsigned long long &total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  unsigned long long inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    const unsigned long long w = lane < nw ? s_warp[lane] : 0;
+    unsigned long long winc = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, winc, o);
+      if (lane >= o) winc += t;
+    }
+    if (lane < nw) s_warp[lane] = winc - w;
+    if (lane == 31) s_warp[32] = winc;
+  }
+  __syncthreads();
+  total = s_warp[32];
+  const unsigned long long r = s_warp[warp] + inc - v;
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
+    int nbuckets, const int32_t *__restrict__ counts, int chunk, int32_t *__restrict__ offsets,
+    int32_t *__restrict__ ioff, unsigned long long *sums, int32_t *done,
+    int32_t *__restrict__ nitems) {
+  __shared__ unsigned long long s_warp[33];
+  __shared__ bool s_last;
+  const int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
+  unsigned long long v[SCAN_PER_THREAD], sum = 0, total;
+#pragma unroll
+  for (int k = 0; k < SCAN_PER_THREAD; ++k) {
+    const int c = base + k < nbuckets ? counts[base + k] : 0;
+    v[k] = (unsigned long long)c | (unsigned long long)((c + chunk - 1) / chunk) << 32;
+    sum += v[k];
+  }
+  unsigned long long run = block_exclusive_scan64(sum, s_warp, total);
+#pragma unroll
+  for (int k = 0; k < SCAN_PER_THREAD; ++k) {
+    if (base + k < nbuckets) {
+      offsets[base + k] = (int32_t)run;
+      ioff[base + k] = (int32_t)(run >> 32);
+    }
+    run += v[k];
+  }
+  if (threadIdx.x == 0) {
+    sums[blockIdx.x] = total;
+    __threadfence();
+    s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  unsigned long long carry = 0;
+  for (int b0 = 0; b0 < (int)gridDim.x; b0 += SCAN_THREADS) {
+    const int b = b0 + threadIdx.x;
+    const unsigned long long x = b < (int)gridDim.x ? __ldcg(&sums[b]) : 0;
+    const unsigned long long e = carry + block_exclusive_scan64(x, s_warp, total);
+    if (b < (int)gridDim.x) sums[b] = e;
+    carry += total;
+  }
+  if (threadIdx.x == 0) *nitems = (int32_t)(carry >> 32);
+}
+
+__global__ void k_plan_finish(int nbuckets, const int32_t *__restrict__ counts, int chunk,
+                              int32_t *__restrict__ offsets, const int32_t *__restrict__ ioff,
+                              const unsigned long long *__restrict__ sums,
+                              WorkItem *__restrict__ items) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nbuckets) return;
+  const unsigned long long s = sums[t / SCAN_TILE];
+  const int off = offsets[t] + (int32_t)s;
+  offsets[t] = off;
+  write_items(t, off, counts[t], chunk, ioff[t] + (int32_t)(s >> 32), items);
+}
+
 __global__ void k_frac_coords(const double *uvw, int64_t stride, double lam,
                               int64_t n, int H, int W, int Q, AxisConst ax, AxisConst ay,
                               int32_t *x, int32_t *xf, int32_t *y, int32_t *yf,
@@ -636,13 +779,24 @@ static int outer_edge(const cg_plan &p, int &T) {
   return 24;
 }
 
-// 4-D tables of odd support under no tuning and no requested tile: the lane
-// layout's 16-cell tiles (layout_for gives the lane layout to even supports,
-// whose slices it can stream), for the lane kernel with taps by loads.
-static bool lane_odd(const cg_plan &p) {
+// Under no tuning and no requested tile, supports up to 16 get the lane layout's
+// 16-cell tiles where layout_for names the warp layout: 4-D tables of odd
+// support, for the lane kernel with taps by loads, and separable ones that the
+// direct kernels grid, which need no order inside a tile.  Not for stacks of so
+// many tiles that their numbers would run out.
+static bool small_tiles(const cg_plan &p) {
   const cg_tuning t = tuning();
-  return !p.lean && !p.kd.sep && p.kd.S <= 16 && p.kd.S % 2 == 1 && p.tile_req == 0 &&
-         t.tile == 0 && t.layout == 0 && (int64_t)p.kd.G * p.kd.Q * p.kd.Q < INT32_MAX;
+  const int64_t tiles = (int64_t)((p.W + 15) / 16) * ((p.H + 15) / 16) * p.layers;
+  return !p.lean && p.kd.S <= 16 && p.tile_req == 0 && t.tile == 0 && t.layout == 0 &&
+         tiles <= (1 << 24);
+}
+static bool lane_odd(const cg_plan &p) {
+  return small_tiles(p) && !p.kd.sep && p.kd.S % 2 == 1 &&
+         (int64_t)p.kd.G * p.kd.Q * p.kd.Q < INT32_MAX;
+}
+static bool direct_sep(const cg_plan &p) {
+  return small_tiles(p) && p.kd.sep && !p.outer &&
+         (double)p.n < 1.5 * (double)p.H * (double)p.W * (double)p.layers;
 }
 
 static void plan_geometry(cg_plan &p) {
@@ -651,7 +805,8 @@ static void plan_geometry(cg_plan &p) {
     p.outer = outer_edge(p, outer_T);
     p.lane_odd = lane_odd(p);
     const bool lane = p.lane_odd || layout_for(p.kd) == CG_LAYOUT_LANE;
-    p.T = p.outer ? outer_T : p.lane_odd ? 16 : tile_edge(p.kd, p.tile_req);
+    const bool flat = p.outer || lane || direct_sep(p);  // no order inside a tile
+    p.T = p.outer ? outer_T : flat && small_tiles(p) ? 16 : tile_edge(p.kd, p.tile_req);
     p.ntx = (p.W + p.T - 1) / p.T;
     p.nty = (p.H + p.T - 1) / p.T;
     // Morton blocks of up to 32 x 32 tiles (no larger than the grid needs)
@@ -667,7 +822,7 @@ static void plan_geometry(cg_plan &p) {
     // in-tile coordinate shifted by subshift is always below 2^sublog.
     int full = 0;
     while ((4 << full) < p.T) ++full;
-    p.sublog = p.outer || lane ? 0 : full;
+    p.sublog = flat ? 0 : full;
     p.subshift = 2 + full - p.sublog;
     // keep the histogram (4 B per bucket) within 2^24 buckets: coarser sub-tiles
     // for very large grid stacks
@@ -734,6 +889,7 @@ static Layout layout_of(const cg_plan &p) {
   L.rank = o;    o = align256(o + n * 4);
   L.recs = o;    o = align256(o + n * sizeof(VisRec));
   L.perm = o;    o = align256(o + n * 4);
+  L.ctr = o;     o = align256(o + 4 * 4);  // before the counts: zeroed with them
   L.counts = o;  o = align256(o + (size_t)p.nbuckets * 4);
   L.offsets = o; o = align256(o + (size_t)p.nbuckets * 4);
   L.scan = o;    o = align256(o + scan_scratch_words(p.nbuckets) * 4);
@@ -741,7 +897,6 @@ static Layout layout_of(const cg_plan &p) {
   const size_t nt = p.mode == CG_PLAN_TILED ? (size_t)p.ntiles : 0;  // items per tile, scanned
   L.tnch = o;    o = align256(o + nt * 4);
   L.tioff = o;   o = align256(o + nt * 4);
-  L.ctr = o;     o = align256(o + 4 * 4);
   L.kpad = o;    o = align256(o + (size_t)p.kpad_slices * p.slice_stride * sizeof(float2));
   L.total = o;
   return L;
@@ -813,8 +968,7 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   p->ticket = ctr + 1;
   p->status = d_status;
   // everything later kernels accumulate into starts at zero on every call
-  CG_CUDA(cudaMemsetAsync(p->counts, 0, (size_t)p->nbuckets * 4, s));
-  CG_CUDA(cudaMemsetAsync(ctr, 0, 16, s));
+  CG_CUDA(cudaMemsetAsync(ctr, 0, (char *)(p->counts + p->nbuckets) - (char *)ctr, s));
   if (n == 0) return CG_OK;
   CoordParams P;
   P.uvw = uvw;
@@ -854,22 +1008,43 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   const int blocks = (int)((n + 255) / 256);
   k_plan_coords<<<blocks, 256, 0, s>>>(P);
   CG_LAUNCH("coords");
-  rc = launch_scan(p->counts, p->offsets, p->nbuckets, (int32_t *)(ws + L.scan), s);
-  if (rc) return rc;
-  k_plan_scatter<<<blocks, 256, 0, s>>>(n, rec_tmp, key, rank, p->offsets, p->recs, p->perm);
-  CG_LAUNCH("plan sort");
-  if (mode == CG_PLAN_TILED) {
-    int32_t *tnch = (int32_t *)(ws + L.tnch), *tioff = (int32_t *)(ws + L.tioff);
-    const unsigned tb = (unsigned)((p->ntiles + 255) / 256);
-    k_plan_item_counts<<<tb, 256, 0, s>>>(p->ntiles, p->sublog, p->counts, p->offsets, p->chunk,
-                                          tnch);
-    CG_LAUNCH("plan item counts");
-    // the bucket scan's scratch is free again (ntiles <= nbuckets)
-    rc = launch_scan(tnch, tioff, p->ntiles, (int32_t *)(ws + L.scan), s);
+  // Buckets' offsets and, tiled, the work list: one block for small grids, two
+  // launches where the buckets are tiles, else the separate passes.  A plan of
+  // 1000 visibilities on 256^2 took eight launches, one on 1531^2 eleven; now four
+  // and five (conv_imaging + conv_predict there: 286 -> 266 us, 370 -> 340 us).
+  const bool tiled = mode == CG_PLAN_TILED;
+  const int scan_blocks = (p->nbuckets + SCAN_TILE - 1) / SCAN_TILE;
+  if (tiled && p->nbuckets <= PLAN_SMALL_BUCKETS) {
+    k_plan_small<<<1, SCAN_THREADS, 0, s>>>(p->nbuckets, p->ntiles, p->sublog, p->counts, p->chunk,
+                                            p->offsets, p->items, p->nitems);
+    CG_LAUNCH("plan offsets and items");
+  } else if (tiled && p->sublog == 0) {
+    unsigned long long *sums = (unsigned long long *)(ws + L.scan);
+    int32_t *tioff = (int32_t *)(ws + L.tioff);
+    k_plan_scan<<<scan_blocks, SCAN_THREADS, 0, s>>>(p->nbuckets, p->counts, p->chunk, p->offsets,
+                                                     tioff, sums, ctr + 3, p->nitems);
+    CG_LAUNCH("plan scan");
+    k_plan_finish<<<(p->nbuckets + 255) / 256, 256, 0, s>>>(p->nbuckets, p->counts, p->chunk,
+                                                            p->offsets, tioff, sums, p->items);
+    CG_LAUNCH("plan items");
+  } else {
+    rc = launch_scan(p->counts, p->offsets, p->nbuckets, (int32_t *)(ws + L.scan), s);
     if (rc) return rc;
-    k_plan_items<<<tb, 256, 0, s>>>(p->ntiles, p->sublog, p->counts, p->offsets, p->chunk, tnch,
-                                    tioff, p->items, p->nitems);
+    if (tiled) {
+      int32_t *tnch = (int32_t *)(ws + L.tnch), *tioff = (int32_t *)(ws + L.tioff);
+      const unsigned tb = (unsigned)((p->ntiles + 255) / 256);
+      k_plan_item_counts<<<tb, 256, 0, s>>>(p->ntiles, p->sublog, p->counts, p->offsets, p->chunk,
+                                            tnch);
+      CG_LAUNCH("plan item counts");
+      // the bucket scan's scratch is free again (ntiles <= nbuckets)
+      rc = launch_scan(tnch, tioff, p->ntiles, (int32_t *)(ws + L.scan), s);
+      if (rc) return rc;
+      k_plan_items<<<tb, 256, 0, s>>>(p->ntiles, p->sublog, p->counts, p->offsets, p->chunk, tnch,
+                                      tioff, p->items, p->nitems);
+      CG_LAUNCH("plan items");
+    }
   }
+  k_plan_scatter<<<blocks, 256, 0, s>>>(n, rec_tmp, key, rank, p->offsets, p->recs, p->perm);
   CG_LAUNCH("plan sort");
   return CG_OK;
 }

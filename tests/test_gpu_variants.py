@@ -293,3 +293,36 @@ def test_plain_fp64_stack(env, layers, n):
         for a, b in ((grid[p].cpu().numpy(), want), (d[s], dw)):
             if b.size:
                 assert numpy.abs(a - b).max() <= tol * max(numpy.abs(b).max(), 1.0)
+
+
+@pytest.mark.parametrize("N,S,sep,layers,n", [
+    (24, 7, True, 1, 1), (256, 8, True, 1, 1000), (1531, 9, False, 1, 4000),
+    (2047, 8, True, 1, 3), (2100, 8, False, 1, 300000), (129, 17, True, 1, 5000),
+    (1500, 17, False, 1, 9000), (640, 8, False, 12, 20000)])
+def test_plan_lists(env, N, S, sep, layers, n):
+    """The plan's offsets and items in one block (up to 16384 buckets), in two launches
+    (tiles as buckets) and in separate passes (sub-tiles): every visibility sorted
+    once, its record as assigned, the buckets' counts in order; then gridded ones,
+    which need every item once: small whole numbers, exact in complex64."""
+    torch, L, E, _, O = env
+    rng, uvw, gcf, src = _case(N + n, n, S, 2, sep, G=2)
+    gcf = numpy.ones_like(gcf)
+    lay = rng.integers(0, layers, n).astype(numpy.int32)
+    kt = E.KernelTable.from_gcf(gcf, 1, E.CF)
+    plan = E.Plan(uvw, 1.0, (N, N), kt, src[:, 0].astype(numpy.int32),
+                  layers=None if layers == 1 else (layers, lay))
+    vis = rng.integers(-4, 5, n).astype(numpy.complex64)
+    got = plan.grid(kt, E.cuda_tensor(vis, E.CF),
+                    torch.zeros((layers, N, N), dtype=E.CF, device="cuda")).cpu().numpy()
+    plan.check()
+    recs, perm, counts = (t.cpu().numpy() for t in plan.export())
+    x, _, y, _ = O.frac_coords((N, N), 2, uvw[:, :2])
+    numpy.testing.assert_array_equal(numpy.sort(perm), numpy.arange(n))
+    numpy.testing.assert_array_equal(recs[:, 0], (x - S // 2)[perm])
+    numpy.testing.assert_array_equal(recs[:, 1], (y - S // 2)[perm])
+    assert counts.sum() == n
+    want = numpy.zeros((layers, N + S, N + S))
+    numpy.add.at(want, (lay, y - S // 2, x - S // 2), vis.real)
+    for axis in (1, 2):  # the footprints: S cells on from the corner
+        want = sum(numpy.roll(want, t, axis) for t in range(S))
+    numpy.testing.assert_array_equal(got.real, want[:, :N, :N])
