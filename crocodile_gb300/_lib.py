@@ -74,8 +74,11 @@ SIGNATURES = {
                             P]),
     "cg_aw_keys": (c_int, [P, c_int64, P, P, c_int64, c_int, c_double, c_int, c_int, P, P, P]),
     "cg_wstack_combine": (c_int, [P, c_int, c_int, c_double, P, P, P, P, P]),
+    "cg_wstack_image": (c_int, [P, c_int, c_int, c_double, P, P, P, P, P]),
     "cg_tower_keys": (c_int, [P, c_int64, c_int64, c_double, c_int, c_double, P, P, P, P, P, P]),
     "cg_towers_combine": (c_int, [P, c_int, c_int, c_double, P, P, c_int, P, P, P]),
+    "cg_towers_image": (c_int, [P, c_int, c_int, c_double, P, P, c_int, P, P, P]),
+    "cg_towers_layers": (c_int, [P, c_int, c_int, c_double, P, P, c_int, P, P, P]),
     "cg_towers_add": (c_int, [P, c_int, c_int, P, c_int, P, P]),
     "cg_towers_cut": (c_int, [P, c_int, P, c_int, c_int, P, P]),
     "cg_towers_expand": (c_int, [P, c_int, c_double, P, P, c_int, P, P, P]),

@@ -776,6 +776,402 @@ int dispatch_rows(int logw, const RowIO &io, int64_t nrows, int sign, cudaStream
   return set_error(CG_ERR_ARG, "FP32 FFT: unsupported row length 2^%d", logw);
 }
 
+// ---------------------------------------------------------------- stacks of w-planes
+// Sums over w-planes in image space (w-stacking, w-towers) read each plane's
+// inverse transform once, times the plane's factor.  Made by the column pass
+// itself, in registers, they spare the planes' last write and the read of it:
+// the pass then reads the stack and writes one plane per sum.
+struct StackLayer {
+  int plane;
+  float wh, wl;  // the plane's w as hi + lo
+  int pad;
+};
+
+// The planes of a sum, in order: all of them, or (counts) those that hold
+// visibilities, whose number goes to first[1] and 0 to first[0].
+__global__ void k_stack_layers(int layers, const double *__restrict__ w,
+                               const int32_t *__restrict__ counts, StackLayer *__restrict__ out,
+                               int32_t *__restrict__ first) {
+  int kept = 0;
+  for (int b = 0; b < layers; b += blockDim.x) {
+    const int L = b + (int)threadIdx.x;
+    const bool in = L < layers && (!counts || counts[L] != 0);
+    int at = L;
+    if (counts) {  // one warp
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      at = kept + __popc(m & ((1u << threadIdx.x) - 1));
+      kept += __popc(m);
+    }
+    if (!in) continue;
+    const double x = w[L];
+    const float hi = (float)x;
+    out[at] = StackLayer{L, hi, (float)(x - (double)hi), 0};
+  }
+  if (counts && threadIdx.x == 0) {
+    first[0] = 0;
+    first[1] = kept;
+  }
+}
+
+// ph = 1 - sqrt(1 - l^2 - m^2) as hi + lo at (i, j) <= N / 2, l, m = theta *
+// coordinates2(N); the other quadrants mirror it.  It is bound by FP64, so a
+// 32 x 32 tile also serves its transpose (l and m change places).
+__global__ void k_w_phase(int N, double theta, float2 *__restrict__ ph, int32_t *status) {
+  if (blockIdx.y > blockIdx.x) return;
+  __shared__ float2 tile[32][33];
+  const int half = N / 2, M = half + 1;
+  const int j = blockIdx.x * 32 + threadIdx.x;
+  const double l = __dmul_rn(theta, centred_coord(j, half, N));
+  const double l2 = __dmul_rn(l, l);
+  int bad = 0;
+  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
+    const int i = blockIdx.y * 32 + y;
+    const double m = __dmul_rn(theta, centred_coord(i, half, N));
+    const double r2 = __dadd_rn(l2, __dmul_rn(m, m));
+    if (i < M && j < M && !(r2 < 1.0)) bad = 1;
+    const double p = 1.0 - sqrt(1.0 - r2);
+    const float hi = (float)p;
+    const float2 v = make_float2(hi, (float)(p - (double)hi));
+    tile[y][threadIdx.x] = v;
+    if (i < M && j < M) ph[(int64_t)i * M + j] = v;
+  }
+  if (bad && status) atomicAdd(&status[ST_RANGE], 1);
+  if (blockIdx.x == blockIdx.y) return;
+  __syncthreads();
+  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
+    const int i = blockIdx.x * 32 + y, k = blockIdx.y * 32 + threadIdx.x;
+    if (i < M && k < M) ph[(int64_t)i * M + k] = tile[threadIdx.x][y];
+  }
+}
+
+// exp(2 pi i w ph).  The turns are a double-float product, reduced to a fraction of
+// a turn and then to an eighth on either side of a quarter turn, g.  There sin(2
+// pi g) / g and cos(2 pi g) are their best polynomials in g^2 (Remez exchange; off
+// by 3e-9 and 1e-10 before rounding), and the quarter's number, in the low bits of
+// the rounding sum, swaps them and sets the signs.  All errors together stay
+// below 1.2e-7 (8.6e-8 over 2M arguments of one turn; sincospif, made for any
+// argument, took 3 % more of a whole w-stacking or w-towers call).
+__device__ __forceinline__ void w_factor(float wh, float wl, float2 ph, float &cs, float &sn) {
+  const float hi = wh * ph.x;
+  const float lo = fmaf(wl, ph.x, fmaf(wh, ph.y, fmaf(wh, ph.x, -hi)));
+  const float f = (hi - rintf(hi)) + lo;
+  const float t = fmaf(4.f, f, 12582912.f);  // 1.5 x 2^23: rounds to whole quarters
+  const float g = fmaf(-0.25f, t - 12582912.f, f), z = g * g;
+  const float s = g * fmaf(fmaf(fmaf(-75.4020680f, z, 81.5925536f), z, -41.3416626f), z, 6.28318529f);
+  const float c =
+      fmaf(fmaf(fmaf(fmaf(59.2867640f, z, -85.4450344f), z, 64.9393391f), z, -19.7392087f), z, 1.f);
+  const unsigned q = __float_as_uint(t);
+  const bool odd = q & 1;
+  sn = __uint_as_float(__float_as_uint(odd ? c : s) ^ ((q << 30) & 0x80000000u));
+  cs = __uint_as_float(__float_as_uint(odd ? s : c) ^ (((q + 1) << 30) & 0x80000000u));
+}
+
+// The quadrant's row or column of index i of a centred (or, rolled, of an
+// unshifted) plane
+__device__ __forceinline__ int w_mirror(int i, int half, bool rolled) {
+  const int k = rolled ? (i < half ? i + half : i - half) : i;
+  return min(k, 2 * half - k);
+}
+
+struct StackArgs {
+  int W, H1, tiles, nj;  // tiles of C columns, nj lines (first rows) per tile
+  int half;
+  bool rolled;
+  const int32_t *first;  // layers [first[c], first[c + 1]) of the list make sum c
+  const StackLayer *list;
+  const float2 *ph;
+  float2 *out;
+  int64_t plane;  // elements of an output plane
+  float scale;
+  __device__ void unit(int64_t u, int C, int &c, int &j, int &col0) const {
+    const int64_t per = (int64_t)tiles * nj;
+    c = (int)(u / per);
+    const int r = (int)(u - c * per);
+    j = r / tiles;
+    col0 = (r - j * tiles) * C;
+  }
+};
+
+template <int LOGL, int C>
+struct StackShape {
+  static constexpr int L = 1 << LOGL, THREADS = C * (L / 16);
+  // 128 registers a thread (sums, phases and the line's values): 512 threads per SM
+  static constexpr int MINB = 512 / THREADS;
+  static constexpr size_t tile_bytes() { return (size_t)L * C * sizeof(float2); }
+  static constexpr size_t smem() {
+    return 128 + 2 * tile_bytes() + (size_t)tw_entries(LOGL) * sizeof(float2) + 16;
+  }
+};
+
+// sum over planes p of X_p / exp(2 pi i w_p ph), X_p the column pass's output
+// (pass B of the four-step columns, or whole columns): a unit (sum, line of rows,
+// tile of C columns) takes its planes in turn, each plane's tile one tensor copy,
+// double-buffered, and keeps the sum and the phases of its elements in
+// registers.  Bound by issue (the factors beside the transform) at about the rate
+// HBM reads the stack.  8 planes of 4096^2, transform and sum: 1.42 ms apart, 1.26
+// so; w_stack_imaging of 32 planes 7.38 -> 6.44 ms; 1200 layers of 256^2 in 200
+// sums: 0.66 and 0.52 ms.  Waits are bounded as in k_fft32_step_tma.
+template <int LOGL, int C>
+__global__ void __launch_bounds__(StackShape<LOGL, C>::THREADS, StackShape<LOGL, C>::MINB)
+    k_fft32_stack(const __grid_constant__ CUtensorMap tmap, StackArgs A, int64_t units,
+                  const float2 *__restrict__ tw, int sign, long long wait) {
+  using TS = StackShape<LOGL, C>;
+  constexpr int L = TS::L, T = L / 16, NS = (LOGL + 3) / 4;
+  extern __shared__ unsigned char f32_tsm[];
+  float2 *tiles = (float2 *)(((uintptr_t)f32_tsm + 127) & ~(uintptr_t)127);
+  float2 *stw = tiles + 2 * L * C;
+  uint64_t *bar = (uint64_t *)(stw + tw_entries(LOGL));
+  const int c = threadIdx.x % C, t = threadIdx.x / C;
+  for (int k = threadIdx.x; k < tw_entries(LOGL); k += TS::THREADS) stw[k] = tw[k];
+  if (threadIdx.x == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  const SmTw<LOGL> twf{stw};
+  auto issue = [&](int64_t u, int q, int b) {  // one thread
+    int s, j, col0;
+    A.unit(u, C, s, j, col0);
+    tma_load_4d(tiles + b * L * C, &tmap, col0, 0, j, A.list[q].plane, &bar[b],
+                (uint32_t)TS::tile_bytes());
+  };
+  // the place after (u, q): the unit's next plane, or the next unit that has one
+  auto advance = [&](int64_t &u, int &q, int &end) {
+    if (++q < end) return;
+    for (u += gridDim.x; u < units; u += gridDim.x) {
+      int s, j, col0;
+      A.unit(u, C, s, j, col0);
+      q = A.first[s];
+      end = A.first[s + 1];
+      if (q < end) return;
+    }
+  };
+  int64_t pu = (int64_t)blockIdx.x - gridDim.x;  // thread 0: the next tile to ask for
+  int pq = 0, pend = 0, it = 0;
+  if (threadIdx.x == 0) {
+    advance(pu, pq, pend);
+    if (pu < units) issue(pu, pq, 0);
+  }
+  for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+    int s, j, col0;
+    A.unit(u, C, s, j, col0);
+    const int col = col0 + c, q1 = A.first[s + 1];
+    float2 acc[16], ph[16];
+    const int mj = w_mirror(col, A.half, A.rolled);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const int mi = w_mirror(j + A.H1 * (t + r * T), A.half, A.rolled);
+      ph[r] = __ldg(&A.ph[(int64_t)mi * (A.half + 1) + mj]);
+      acc[r] = make_float2(0.f, 0.f);
+    }
+    for (int q = A.first[s]; q < q1; ++q, ++it) {
+      const int b = it & 1;
+      bool next = false;
+      // the other tile's last reads were before the previous plane's last barrier
+      if (threadIdx.x == 0) {
+        advance(pu, pq, pend);
+        next = pu < units;
+        if (next) issue(pu, pq, b ^ 1);
+      }
+      const bool ok = tile_wait(&bar[b], (it >> 1) & 1, wait);
+      if (__syncthreads_or(!ok)) {
+        if (threadIdx.x == 0) {
+          atomicAdd(&g_fft32_timeouts, 1);
+          mbar_wait_cycles(&bar[b], (it >> 1) & 1, FFT_WAIT_CYCLES);
+          if (next) mbar_wait_cycles(&bar[b ^ 1], ((it + 1) >> 1) & 1, FFT_WAIT_CYCLES);
+        }
+        __syncthreads();
+        return;
+      }
+      float2 *buf = tiles + b * L * C;
+      auto lds = [&](int e) {
+        const float2 v = buf[e * C + c];
+        return cf{v.x, v.y};
+      };
+      auto sts = [&](int e, cf v) { buf[e * C + c] = make_float2(v.x, v.y); };
+      const StackLayer w = A.list[q];
+      cf v[16];
+      stage_load(LOGL, 0, t, lds, twf, v);
+      __syncthreads();  // all reads before any write
+      stage_dft(LOGL, 0, sign, v);
+      stage_store(LOGL, 0, t, sts, v);
+#pragma unroll
+      for (int st = 1; st < NS; ++st) {
+        __syncthreads();
+        stage_load(LOGL, st, t, lds, twf, v);
+        __syncthreads();
+        stage_dft(LOGL, st, sign, v);
+        if (st + 1 < NS) stage_store(LOGL, st, t, sts, v);
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {  // outputs t + r T
+        const cf g = v[out_slot(4, r)];
+        float cs, sn;
+        w_factor(w.wh, w.wl, ph[r], cs, sn);
+        acc[r].x += g.x * cs + g.y * sn;  // g / (cs + i sn)
+        acc[r].y += g.y * cs - g.x * sn;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const int row = j + A.H1 * (t + r * T);
+      const float sc = (row + col) & 1 ? -A.scale : A.scale;
+      A.out[s * A.plane + (int64_t)row * A.W + col] = make_float2(acc[r].x * sc, acc[r].y * sc);
+    }
+  }
+}
+
+// The reverse: rows of every layer's image, the chunk's image (unshifted) over
+// exp(2 pi i w ph), transformed on their way out, so that the layers are written
+// once.  A unit is a group of rows of one chunk, whose image and phases stay in
+// registers over the chunk's layers.  1200 layers of 256^2: 0.67 ms apart, 0.52 so.
+template <int LOGN>
+__global__ void __launch_bounds__(256, 2)
+    k_fft32_rows_stack(const float2 *__restrict__ images, StackArgs A, int64_t units,
+                       float2 *__restrict__ stack, const float2 *__restrict__ tw, int sign) {
+  constexpr int N = 1 << LOGN, T = N / 16, LPC = 256 / T, P = N + N / 32;
+  constexpr int NS = (LOGN + 3) / 4;
+  static_assert(T <= 32, "a row is one warp's");
+  extern __shared__ float2 f32_sm[];
+  const int line = threadIdx.x / T, t = threadIdx.x % T;
+  float2 *buf = f32_sm + line * P;
+  float2 *stw = f32_sm + LPC * P;
+  for (int k = threadIdx.x; k < tw_entries(LOGN); k += 256) stw[k] = tw[k];
+  __syncthreads();
+  const SmTw<LOGN> twf{stw};
+  auto lds = [&](int e) {
+    const float2 x = buf[pad(e)];
+    return cf{x.x, x.y};
+  };
+  auto sts = [&](int e, cf x) { buf[pad(e)] = make_float2(x.x, x.y); };
+  constexpr int logr = stage_logr(LOGN, 0), R = 1 << logr, NR = N >> logr;
+  for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
+    const int c = (int)(u / (N / LPC));
+    const int row = (int)(u - (int64_t)c * (N / LPC)) * LPC + line;
+    const float2 *src = images + ((int64_t)c * N + row) * N;
+    const int mi = w_mirror(row, A.half, true);
+    float2 a[16], ph[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {  // slot q = m R + r: element t + m T + r N / R
+      const int e = t + (q >> logr) * T + (q & (R - 1)) * NR;
+      const float sc = (row + e) & 1 ? -A.scale : A.scale;
+      a[q] = src[e];
+      a[q].x *= sc;
+      a[q].y *= sc;
+      ph[q] = __ldg(&A.ph[(int64_t)mi * (A.half + 1) + w_mirror(e, A.half, true)]);
+    }
+    const int q1 = A.first[c + 1];
+    for (int q = A.first[c]; q < q1; ++q) {
+      const StackLayer w = A.list[q];
+      cf v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        float cs, sn;
+        w_factor(w.wh, w.wl, ph[k], cs, sn);
+        v[k] = cf{a[k].x * cs + a[k].y * sn, a[k].y * cs - a[k].x * sn};
+      }
+      stage_dft(LOGN, 0, sign, v);
+      __syncwarp();  // the previous layer's last reads
+      stage_store(LOGN, 0, t, sts, v);
+      float2 *dst = stack + ((int64_t)w.plane * N + row) * N;
+#pragma unroll
+      for (int st = 1; st < NS; ++st) {
+        __syncwarp();
+        stage_load(LOGN, st, t, lds, twf, v);
+        __syncwarp();
+        stage_dft(LOGN, st, sign, v);
+        if (st + 1 < NS)
+          stage_store(LOGN, st, t, sts, v);
+        else
+          stage_store(LOGN, st, t, [&](int e, cf x) { dst[e] = make_float2(x.x, x.y); }, v);
+      }
+    }
+  }
+}
+
+// The layer list, the ranges of a sum over all planes, and the phases of a stack,
+// in scratch of the library's pool.
+struct StackScratch {
+  StackLayer *list;
+  int32_t *first;
+  float2 *ph;
+};
+
+int stack_scratch(int layers, int N, double theta, const double *w, const int32_t *counts,
+                  int32_t *status, StackScratch *out, cudaStream_t st) {
+  const int64_t M = N / 2 + 1;
+  const size_t head = ((size_t)layers * sizeof(StackLayer) + 8 + 255) & ~(size_t)255;
+  cudaMemPool_t pool;
+  int rc = scratch_pool(&pool);
+  if (rc) return rc;
+  char *p = nullptr;
+  CG_CUDA(cudaMallocFromPoolAsync((void **)&p, head + (size_t)(M * M) * sizeof(float2), pool, st));
+  out->list = (StackLayer *)p;
+  out->first = (int32_t *)(out->list + layers);
+  out->ph = (float2 *)(p + head);
+  k_stack_layers<<<1, counts ? 32 : 1024, 0, st>>>(layers, w, counts, out->list, out->first);
+  const unsigned tiles = (unsigned)((M + 31) / 32);
+  k_w_phase<<<dim3(tiles, tiles), dim3(32, 8), 0, st>>>(N, theta, out->ph, status);
+  if (cudaPeekAtLastError() != cudaSuccess) {
+    cudaFreeAsync(p, st);
+    CG_LAUNCH("w-plane stack set-up");
+  }
+  return CG_OK;
+}
+
+template <int LOGL, int C>
+int launch_stack(const CUtensorMap &map, const StackArgs &A, int64_t units, int sign,
+                 cudaStream_t st) {
+  using TS = StackShape<LOGL, C>;
+  const float2 *tw;
+  int rc = twiddles(LOGL, sign, &tw);
+  if (rc) return rc;
+  CG_CUDA(cudaFuncSetAttribute(k_fft32_stack<LOGL, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)TS::smem()));
+  int per_sm = 0;
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft32_stack<LOGL, C>,
+                                                        TS::THREADS, TS::smem()));
+  CG_REQUIRE(per_sm > 0, "FP32 FFT stack columns do not fit on an SM (smem %zu)", TS::smem());
+  const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * per_sm);
+  k_fft32_stack<LOGL, C><<<grid, TS::THREADS, TS::smem(), st>>>(map, A, units, tw, sign,
+                                                                wait_cycles());
+  CG_LAUNCH("FP32 FFT stack columns");
+  return CG_OK;
+}
+
+// Tensor map of a stack's column tiles: (W, H2, H1, planes), boxes of C columns by
+// H2 rows.  false: not describable.
+bool stack_map(CUtensorMap *map, const float2 *in, int W, int H1, int H2, int planes, int C) {
+  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (!enc || ((uintptr_t)in & 15)) return false;
+  const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)H2, (cuuint64_t)H1, (cuuint64_t)planes};
+  const cuuint64_t strides[3] = {(cuuint64_t)W * 8, (cuuint64_t)H2 * W * 8,
+                                 (cuuint64_t)H1 * H2 * W * 8};
+  const cuuint32_t box[4] = {(cuuint32_t)C, (cuuint32_t)H2, 1, 1};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, (void *)in, dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int LOGN>
+int launch_rows_stack(const float2 *images, const StackArgs &A, int nchunks, float2 *stack, int sign,
+                      cudaStream_t st) {
+  constexpr int N = 1 << LOGN, LPC = 4096 / N;
+  const float2 *tw;
+  int rc = twiddles(LOGN, sign, &tw);
+  if (rc) return rc;
+  const size_t smem = (size_t)(LPC * (N + N / 32) + tw_entries(LOGN)) * sizeof(float2);
+  CG_CUDA(cudaFuncSetAttribute(k_fft32_rows_stack<LOGN>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t units = (int64_t)nchunks * (N / LPC);
+  const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * 2);
+  k_fft32_rows_stack<LOGN><<<grid, 256, smem, st>>>(images, A, units, stack, tw, sign);
+  CG_LAUNCH("FP32 FFT stack rows");
+  return CG_OK;
+}
+
 }  // namespace f32
 
 // Sides the hand-written FP32 transform takes: powers of two 64..8192 (H may
@@ -887,6 +1283,101 @@ int fft32_image(const float2 *grid_premod, int H, int W, float *image, float *ma
   f32::ColImageIO io{grid_premod, image, W, H, (H / 2 + W / 2) & 1,
                      (float)(1.0 / ((double)H * W))};
   return f32::dispatch_cols(lh, io, 1, W, 1, max_out, st);
+}
+
+// The centred inverse transform of every plane with visibilities and their sum
+// over exp(2 pi i w ph), in one: rows, pass A in place, then k_fft32_stack as pass
+// B.  *used = false (and nothing done) where that does not apply: sides without
+// the four-step columns, whose single column pass would have too few units to
+// fill the GPU with the planes inside each.
+int fft32_wstack(float2 *planes, int layers, int N, double theta, const double *mean_w,
+                 const int32_t *counts, float2 *image, int32_t *status, cudaStream_t st,
+                 bool *used) {
+  *used = false;
+  if (!fft32_supported(N, N) || N < f32::STEP_MIN) return CG_OK;
+  int l1, l2;
+  f32::step_split(f32::log2_exact(N), l1, l2);
+  CUtensorMap map;
+  if (!f32::stack_map(&map, planes, N, 1 << l1, 1 << l2, layers, 32)) return CG_OK;
+  *used = true;
+  const float2 *twH;
+  int rc = f32::twiddles_full(l1 + l2, 1, &twH);
+  if (rc) return rc;
+  f32::RowIO rio{planes, N, N, 1, 0, 0, 1.f};
+  if ((rc = f32::dispatch_rows(l1 + l2, rio, (int64_t)layers * N, 1, st))) return rc;
+  f32::StepShape sa{N, 1 << l1, 1 << l2, N / 32, 1 << l2, (int64_t)N * N};
+  f32::StepA sA{sa, planes, planes, twH};
+  const int64_t ua = (int64_t)layers * sa.nj * sa.tiles;
+  bool tma;
+  rc = f32::launch_step_tma(l1, sA, planes, N, 1 << l1, 1 << l2, layers, true, ua, 1, nullptr, st,
+                            &tma);
+  if (!rc && !tma) rc = f32::launch_step(l1, sA, ua, 1, nullptr, st);
+  if (rc) return rc;
+  f32::StackScratch sc;
+  if ((rc = f32::stack_scratch(layers, N, theta, mean_w, counts, status, &sc, st))) return rc;
+  f32::StackArgs A{N,      1 << l1, N / 32, 1 << l1, N / 2, false, sc.first, sc.list, sc.ph,
+                   image, (int64_t)N * N, (float)(1.0 / ((double)N * N))};
+  const int64_t units = (int64_t)A.tiles * A.nj;
+  rc = l2 == 5 ? f32::launch_stack<5, 32>(map, A, units, 1, st)
+               : f32::launch_stack<6, 32>(map, A, units, 1, st);
+  const cudaError_t fe = cudaFreeAsync(sc.list, st);
+  if (rc) return rc;
+  CG_CUDA(fe);
+  return CG_OK;
+}
+
+// The raw inverse transforms of a stack of S x S layers and their sums by chunk,
+// as cg_towers_combine forms them.  Sides 64 to 256 (a tile's rows fit a copy box);
+// a wait limit of 0 keeps to the passes that wait for nothing.
+int fft32_towers_sum(float2 *stack, int layers, int S, double theta, const double *layer_w,
+                     const int32_t *chunk_first, int nchunks, float2 *out, int32_t *status,
+                     cudaStream_t st, bool *used) {
+  *used = false;
+  if (!fft32_supported(S, S) || S > 256 || wait_cycles() == 0) return CG_OK;
+  const int C = S == 256 ? 16 : 32;
+  CUtensorMap map;
+  if (!f32::stack_map(&map, stack, S, 1, S, layers, C)) return CG_OK;
+  *used = true;
+  f32::RowIO rio{stack, S, S, 0, 0, 0, 1.f};
+  const int ls = f32::log2_exact(S);
+  int rc = f32::dispatch_rows(ls, rio, (int64_t)layers * S, 1, st);
+  if (rc) return rc;
+  f32::StackScratch sc;
+  if ((rc = f32::stack_scratch(layers, S, theta, layer_w, nullptr, status, &sc, st))) return rc;
+  f32::StackArgs A{S,   1,   S / C, 1, S / 2, true, chunk_first, sc.list, sc.ph,
+                   out, (int64_t)S * S, 1.0f / (float)((int64_t)S * S)};
+  const int64_t units = (int64_t)nchunks * A.tiles;
+  rc = ls == 6   ? f32::launch_stack<6, 32>(map, A, units, 1, st)
+       : ls == 7 ? f32::launch_stack<7, 32>(map, A, units, 1, st)
+                 : f32::launch_stack<8, 16>(map, A, units, 1, st);
+  const cudaError_t fe = cudaFreeAsync(sc.list, st);
+  if (rc) return rc;
+  CG_CUDA(fe);
+  return CG_OK;
+}
+
+// The reverse: cg_towers_expand and the raw forward transform of its layers.
+int fft32_towers_layers(const float2 *images, int layers, int S, double theta,
+                        const double *layer_w, const int32_t *chunk_first, int nchunks,
+                        float2 *stack, int32_t *status, cudaStream_t st, bool *used) {
+  *used = false;
+  if (!fft32_supported(S, S) || S > 512) return CG_OK;  // a row to a warp
+  *used = true;
+  f32::StackScratch sc;
+  int rc = f32::stack_scratch(layers, S, theta, layer_w, nullptr, status, &sc, st);
+  if (rc) return rc;
+  f32::StackArgs A{S,       1, 0, 1, S / 2, true, chunk_first, sc.list, sc.ph,
+                   nullptr, 0, 1.0f / (float)((int64_t)S * S)};
+  const int ls = f32::log2_exact(S);
+  rc = ls == 6   ? f32::launch_rows_stack<6>(images, A, nchunks, stack, -1, st)
+       : ls == 7 ? f32::launch_rows_stack<7>(images, A, nchunks, stack, -1, st)
+       : ls == 8 ? f32::launch_rows_stack<8>(images, A, nchunks, stack, -1, st)
+                 : f32::launch_rows_stack<9>(images, A, nchunks, stack, -1, st);
+  const cudaError_t fe = cudaFreeAsync(sc.list, st);
+  if (rc) return rc;
+  CG_CUDA(fe);
+  f32::ColIO cio{stack, S, S, 0, 0, 1.f};
+  return f32::dispatch_cols(ls, cio, layers, S, -1, nullptr, st);
 }
 
 }  // namespace cg

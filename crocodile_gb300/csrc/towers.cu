@@ -22,6 +22,14 @@
 
 namespace cg {
 
+// fft32.cu
+int fft32_towers_sum(float2 *stack, int layers, int S, double theta, const double *layer_w,
+                     const int32_t *chunk_first, int nchunks, float2 *out, int32_t *status,
+                     cudaStream_t st, bool *used);
+int fft32_towers_layers(const float2 *images, int layers, int S, double theta,
+                        const double *layer_w, const int32_t *chunk_first, int nchunks,
+                        float2 *stack, int32_t *status, cudaStream_t st, bool *used);
+
 __device__ __forceinline__ int64_t floor_div_ll(int64_t a, int64_t b) {
   int64_t q, r;
   q = a / b;
@@ -388,6 +396,37 @@ int cg_towers_combine(const void *stack_c64, int layers, int S, double theta,
       d_status);
   CG_LAUNCH("w-towers combine");
   return CG_OK;
+}
+
+int cg_towers_image(void *stack_c64, int layers, int S, double theta, const double *layer_w,
+                    const int32_t *chunk_first, int nchunks, void *out_c64, int32_t *d_status,
+                    cg_stream_t stream) {
+  CG_REQUIRE(stack_c64 && layer_w && chunk_first && out_c64 && layers >= 1 && S >= 2 &&
+                 S % 2 == 0 && nchunks >= 1,
+             "bad w-towers image arguments (even sub-grid size)");
+  bool used;
+  int rc = fft32_towers_sum((float2 *)stack_c64, layers, S, theta, layer_w, chunk_first, nchunks,
+                            (float2 *)out_c64, d_status, (cudaStream_t)stream, &used);
+  if (rc || used) return rc;
+  if ((rc = cg_fft_raw(stack_c64, layers, S, S, 1, 1, stream))) return rc;
+  return cg_towers_combine(stack_c64, layers, S, theta, layer_w, chunk_first, nchunks, out_c64,
+                           d_status, stream);
+}
+
+int cg_towers_layers(const void *images_c64, int layers, int S, double theta,
+                     const double *layer_w, const int32_t *chunk_first, int nchunks,
+                     void *stack_c64, int32_t *d_status, cg_stream_t stream) {
+  CG_REQUIRE(images_c64 && layer_w && chunk_first && stack_c64 && layers >= 1 && S >= 2 &&
+                 S % 2 == 0 && nchunks >= 1,
+             "bad w-towers layers arguments (even sub-grid size)");
+  bool used;
+  int rc = fft32_towers_layers((const float2 *)images_c64, layers, S, theta, layer_w, chunk_first,
+                               nchunks, (float2 *)stack_c64, d_status, (cudaStream_t)stream, &used);
+  if (rc || used) return rc;
+  if ((rc = cg_towers_expand(images_c64, S, theta, layer_w, chunk_first, nchunks, stack_c64,
+                             d_status, stream)))
+    return rc;
+  return cg_fft_raw(stack_c64, layers, S, S, 1, 0, stream);
 }
 
 int cg_towers_add(const void *sub_c64, int nchunks, int S, const int32_t *origin, int N,

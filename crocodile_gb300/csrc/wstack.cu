@@ -7,7 +7,8 @@
 //
 // The planes are gridded in one launch into a stack of grids (a layered
 // plan), transformed as one batch of centred inverse FFTs, and combined here
-// in one pass over the stack.  w_kernel_function (crocodile/synthesis.py:273-293) is
+// in one pass over the stack, or from 2048^2 in the transform's last pass
+// (fft32.cu).  w_kernel_function (crocodile/synthesis.py:273-293) is
 // exp(2 pi i w ph) with ph = 1 - sqrt(1 - l^2 - m^2); ph is computed in FP64
 // once per pixel, the turns w ph of each plane are formed in double-float
 // arithmetic and reduced to a fraction of a turn before the FP32 sincospi,
@@ -15,6 +16,11 @@
 #include "cg_internal.cuh"
 
 namespace cg {
+
+// fft32.cu
+int fft32_wstack(float2 *planes, int layers, int N, double theta, const double *mean_w,
+                 const int32_t *counts, float2 *image, int32_t *status, cudaStream_t st,
+                 bool *used);
 
 // Mean of w over each layer's visibilities (the plan's sorted order keeps a
 // layer's visibilities contiguous).  Grid (chunk, layer): every block sums up
@@ -190,6 +196,21 @@ int cg_wstack_combine(const void *planes_c64, int layers, int N, double theta,
       d_status);
   CG_LAUNCH("w-stack combine");
   return CG_OK;
+}
+
+int cg_wstack_image(void *planes_c64, int layers, int N, double theta, const double *mean_w,
+                    const int32_t *counts, void *image_c64, int32_t *d_status,
+                    cg_stream_t stream) {
+  CG_REQUIRE(planes_c64 && mean_w && counts && image_c64 && layers >= 1 && N >= 2 && N % 2 == 0,
+             "bad w-stacking arguments (even image size)");
+  CG_REQUIRE(layers <= 4096, "at most 4096 w-planes");
+  bool used;
+  int rc = fft32_wstack((float2 *)planes_c64, layers, N, theta, mean_w, counts, (float2 *)image_c64,
+                        d_status, (cudaStream_t)stream, &used);
+  if (rc || used) return rc;
+  if ((rc = cg_fft(planes_c64, layers, N, N, 1, 1, nullptr, stream))) return rc;
+  return cg_wstack_combine(planes_c64, layers, N, theta, mean_w, counts, image_c64, d_status,
+                           stream);
 }
 
 }  // extern "C"

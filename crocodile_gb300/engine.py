@@ -414,6 +414,18 @@ def wstack_combine(planes, theta, mean_w, counts, status):
     return out
 
 
+def wstack_image(planes, theta, mean_w, counts, status):
+    """wstack_combine of the planes' centred inverse transforms; consumes the planes."""
+    layers, N = planes.shape[0], planes.shape[-1]
+    if N % 2:
+        fft_(planes, True)
+        return wstack_combine(planes, theta, mean_w, counts, status)
+    out = torch.empty((N, N), dtype=CF, device="cuda")
+    L.call("cg_wstack_image", _p(planes), layers, N, float(theta), _p(mean_w), _p(counts),
+           _p(out), _p(status.t), stream())
+    return out
+
+
 # --------------------------------------------------------------------------
 # imaging helpers
 
@@ -635,6 +647,29 @@ def towers_combine(stack, theta, layer_w, chunk_first, status):
     out = torch.empty((nchunks, S, S), dtype=CF, device="cuda")
     L.call("cg_towers_combine", _p(stack), int(stack.shape[0]), S, float(theta), _p(lw),
            _p(cf), nchunks, _p(out), _p(status.t), stream())
+    return out
+
+
+def towers_image(stack, theta, layer_w, chunk_first, status):
+    """towers_combine of the layers' inverse fft_raw; consumes the stack."""
+    S = stack.shape[-1]
+    lw = cuda_tensor(layer_w, torch.float64)
+    cf = cuda_tensor(chunk_first, torch.int32)
+    nchunks = int(cf.shape[0]) - 1
+    out = torch.empty((nchunks, S, S), dtype=CF, device="cuda")
+    L.call("cg_towers_image", _p(stack), int(stack.shape[0]), S, float(theta), _p(lw), _p(cf),
+           nchunks, _p(out), _p(status.t), stream())
+    return out
+
+
+def towers_layers(images, theta, layer_w, chunk_first, status):
+    """The forward fft_raw of towers_expand's layers."""
+    S = images.shape[-1]
+    lw = cuda_tensor(layer_w, torch.float64)
+    cf = cuda_tensor(chunk_first, torch.int32)
+    out = torch.empty((int(lw.shape[0]), S, S), dtype=CF, device="cuda")
+    L.call("cg_towers_layers", _p(images), int(lw.shape[0]), S, float(theta), _p(lw), _p(cf),
+           int(cf.shape[0]) - 1, _p(out), _p(status.t), stream())
     return out
 
 

@@ -929,7 +929,7 @@ def w_stack_imaging(theta, lam, uvw, src, vis, kv, plane, precision=None, per_pl
         else:
             raise ValueError("gridder must be 'auto', 'tiled' or 'sparse'")
         mean_w, counts = plan.layer_mean_w()
-        E.fft_(planes, True)
+        image = E.wstack_image(planes, theta, mean_w, counts, st)
     else:
         mean_w = torch.zeros(layers, dtype=torch.float64, device="cuda")
         counts = torch.zeros(layers, dtype=torch.int32, device="cuda")
@@ -946,7 +946,7 @@ def w_stack_imaging(theta, lam, uvw, src, vis, kv, plane, precision=None, per_pl
             m, c = sub.layer_mean_w()
             mean_w[p], counts[p] = m[0], c[0]
             E.fft_(planes[p], True)
-    image = E.wstack_combine(planes, theta, mean_w, counts, st)
+        image = E.wstack_combine(planes, theta, mean_w, counts, st)
     st.check()
     return _host(image, like=uvw)
 
@@ -1014,8 +1014,7 @@ def w_towers_imaging(theta, lam, uvw, src, vis, subgrid_size, margin, wincrement
         raise ValueError("gridder must be 'auto', 'tiled' or 'sparse'")
     # unshifted transforms: the centring rolls, signs and 1/s^2 are folded into
     # the combine and add passes
-    E.fft_raw(stack, True)
-    sub = E.towers_combine(stack, theta, plane * float(wincrement), chunk_first, st)
+    sub = E.towers_image(stack, theta, plane * float(wincrement), chunk_first, st)
     del stack
     E.fft_raw(sub, False)
     E.towers_add(sub, origin, grid)
@@ -1149,9 +1148,8 @@ def w_towers_predict(theta, lam, uvw, src, guv, subgrid_size, margin, wincrement
                                E.CF)
     images = E.towers_cut(grid_t, origin, s)
     E.fft_raw(images, True)
-    stack = E.towers_expand(images, theta, plane * float(wincrement), chunk_first, st)
+    stack = E.towers_layers(images, theta, plane * float(wincrement), chunk_first, st)
     del images
-    E.fft_raw(stack, False)
     plan = E.Plan(rel, s / theta, (s, s), ktab, kidx, status=st, layers=(len(used), row),
                   tile=tile)
     out = plan.degrid(ktab, stack)

@@ -434,6 +434,12 @@ int cg_plan_layer_mean_w(const cg_plan *plan, const double *uvw, int64_t stride,
 int cg_wstack_combine(const void *planes_c64, int layers, int N, double theta,
                       const double *mean_w, const int32_t *counts,
                       void *image_c64, int32_t *d_status, cg_stream_t stream);
+/* The inverse centred cg_fft of the planes and cg_wstack_combine in one (even N),
+ * for sides 2048 to 8192 (powers of two) with the sum formed in the last pass of
+ * the transform; the planes are left undefined. */
+int cg_wstack_image(void *planes_c64, int layers, int N, double theta, const double *mean_w,
+                    const int32_t *counts, void *image_c64, int32_t *d_status,
+                    cg_stream_t stream);
 
 /* w-towers: w-stacking on sub-grids (examples/grid/grid.c:482-710,
  * examples/notebooks/wtowers.ipynb code cell 16).  Visibility i falls into
@@ -468,6 +474,16 @@ int cg_towers_add(const void *sub_c64, int nchunks, int S, const int32_t *origin
  * w_kernel_function(l, m, layer_w[L]), rolled and sign-modulated so that an
  * unshifted forward cg_fft_raw of the stack gives the centred sub-grids, which a
  * layered plan's cg_degrid then degrids with the residual-w kernels. */
+/* cg_towers_image: the unshifted inverse cg_fft_raw of the gridded layers and
+ * cg_towers_combine in one (the stack is left undefined); cg_towers_layers:
+ * cg_towers_expand and the forward cg_fft_raw of its layers in one.  For sides 64
+ * to 256 (512: layers) the factors are applied in the transforms' own passes. */
+int cg_towers_image(void *stack_c64, int layers, int S, double theta, const double *layer_w,
+                    const int32_t *chunk_first, int nchunks, void *out_c64, int32_t *d_status,
+                    cg_stream_t stream);
+int cg_towers_layers(const void *images_c64, int layers, int S, double theta,
+                     const double *layer_w, const int32_t *chunk_first, int nchunks,
+                     void *stack_c64, int32_t *d_status, cg_stream_t stream);
 int cg_towers_cut(const void *grid_c64, int N, const int32_t *origin, int nchunks, int S,
                   void *out_c64, cg_stream_t stream);
 int cg_towers_expand(const void *images_c64, int S, double theta, const double *layer_w,

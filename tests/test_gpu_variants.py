@@ -326,3 +326,57 @@ def test_plan_lists(env, N, S, sep, layers, n):
     for axis in (1, 2):  # the footprints: S cells on from the corner
         want = sum(numpy.roll(want, t, axis) for t in range(S))
     numpy.testing.assert_array_equal(got.real, want[:, :N, :N])
+
+
+def _near(a, b, tol=1e-6):
+    """Within tol of b's norm: the same products summed in the same order, with a
+    few roundings of 2^-24 to each."""
+    a, b = a.cpu().numpy(), b.cpu().numpy()
+    assert numpy.linalg.norm(a - b) <= tol * numpy.linalg.norm(b)
+
+
+@pytest.mark.parametrize("N,held", [(64, [1, 0, 2]), (96, [3]), (2048, [0, 0]), (2048, [5]),
+                                    (2048, [0, 7, 1, 0, 2]), (4096, [1, 1, 0, 9]), (8192, [0, 4, 1])])
+def test_wstack_image(env, N, held):
+    """Planes summed in the transform's last pass (from 2048), some or all of them
+    without visibilities, against the transform and the sum by themselves."""
+    torch, L, E, _, O = env
+    g = torch.Generator(device="cuda").manual_seed(N + len(held))
+    planes = torch.randn((len(held), N, N), dtype=E.CF, device="cuda", generator=g)
+    w = torch.linspace(-700.0, 900.0, len(held), dtype=torch.float64, device="cuda")
+    counts = torch.tensor(held, dtype=torch.int32, device="cuda")
+    st = E.Status()
+    want = E.wstack_combine(E.fft_(planes.clone(), True), 0.3, w, counts, st)
+    got = E.wstack_image(planes.clone(), 0.3, w, counts, st)
+    st.check()
+    _near(got, want)
+    assert E.fft_timeouts() == 0
+    E.wstack_image(planes, 1.5, w, counts, st)  # l^2 + m^2 >= 1 in the corners
+    with pytest.raises(Exception):
+        st.check()
+
+
+@pytest.mark.parametrize("S", [64, 96, 128, 256, 512])
+def test_towers_stack(env, S):
+    """Layers summed by chunk in the transform's last pass (sides 64 to 256), and the
+    reverse in its first (to 512), chunks of one layer, of many and of none, against
+    the transforms and sums by themselves."""
+    torch, L, E, _, O = env
+    first = numpy.array([0, 1, 1, 4, 4 + 3 * 1024 // S, 4 + 3 * 1024 // S + 2], numpy.int32)
+    n = int(first[-1])
+    g = torch.Generator(device="cuda").manual_seed(S)
+    stack = torch.randn((n, S, S), dtype=E.CF, device="cuda", generator=g)
+    w = numpy.random.default_rng(S).uniform(-3000, 3000, n)
+    st = E.Status()
+    want = E.towers_combine(E.fft_raw(stack.clone(), True), 0.2, w, first, st)
+    _near(E.towers_image(stack.clone(), 0.2, w, first, st), want)
+    images = torch.randn((len(first) - 1, S, S), dtype=E.CF, device="cuda", generator=g)
+    want = E.fft_raw(E.towers_expand(images, 0.2, w, first, st), False)
+    _near(E.towers_layers(images, 0.2, w, first, st), want)
+    st.check()
+    assert E.fft_timeouts() == 0
+    for call, x in ((E.towers_image, stack), (E.towers_layers, images)):
+        st = E.Status()
+        call(x, 1.5, w, first, st)
+        with pytest.raises(Exception):
+            st.check()
