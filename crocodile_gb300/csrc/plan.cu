@@ -288,8 +288,10 @@ __global__ void k_plan_items(int ntiles, int sublog, const int32_t *__restrict__
 }
 
 // The whole of the above (bucket scan, item counts, their scan, items) in one
-// block for small grids, where launches are most of a plan's time.
-static constexpr int PLAN_SMALL_BUCKETS = 16384;
+// block for small grids, where launches are most of a plan's time: up to 16384
+// buckets in the place of five launches (27 us against 12 and their gaps), up to
+// 4096 where two can do it (16384 tiles: 27 us against 10).
+static constexpr int PLAN_SMALL_BUCKETS = 16384, PLAN_SMALL_TILES = 4096;
 
 __device__ __forceinline__ void write_items(int tile, int off, int count, int chunk, int base,
                                             WorkItem *items) {
@@ -1014,7 +1016,7 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   // and five (conv_imaging + conv_predict there: 286 -> 266 us, 370 -> 340 us).
   const bool tiled = mode == CG_PLAN_TILED;
   const int scan_blocks = (p->nbuckets + SCAN_TILE - 1) / SCAN_TILE;
-  if (tiled && p->nbuckets <= PLAN_SMALL_BUCKETS) {
+  if (tiled && p->nbuckets <= (p->sublog ? PLAN_SMALL_BUCKETS : PLAN_SMALL_TILES)) {
     k_plan_small<<<1, SCAN_THREADS, 0, s>>>(p->nbuckets, p->ntiles, p->sublog, p->counts, p->chunk,
                                             p->offsets, p->items, p->nitems);
     CG_LAUNCH("plan offsets and items");
