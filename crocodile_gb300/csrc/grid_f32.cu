@@ -692,6 +692,7 @@ template <bool SEP, int S>
 __global__ void __launch_bounds__(256, 4) k_grid_direct(DirectArgs D, int mode,
                                                         const float2 *__restrict__ ktab,
                                                         const float2 *__restrict__ vis,
+                                                        const float2 *__restrict__ sub,
                                                         const float *__restrict__ weight,
                                                         float2 *__restrict__ grid) {
   const TiledArgs &A = D.A;
@@ -714,6 +715,10 @@ __global__ void __launch_bounds__(256, 4) k_grid_direct(DirectArgs D, int mode,
           const float wt = weight[src];
           val.x *= wt;
           val.y *= wt;
+        } else if (mode == 3) {  // the residual of a degridding just done
+          const float2 d = sub[src];
+          val.x -= d.x;
+          val.y -= d.y;
         }
       }
     }
@@ -782,11 +787,20 @@ static DirectArgs direct_args(const cg_plan *p) {
 }
 
 static int direct_grid_launch(const cg_plan *p, const float2 *ktab, const float2 *vis,
-                              const float *weight, int mode, float2 *grid, cudaStream_t s) {
+                              const float2 *sub, const float *weight, int mode, float2 *grid,
+                              cudaStream_t s) {
   void *fn = p->kd.sep ? grid_direct_for<true>(p->kd.S) : grid_direct_for<false>(p->kd.S);
   DirectArgs D = direct_args(p);
-  void *args[] = {&D, &mode, &ktab, &vis, &weight, &grid};
+  void *args[] = {&D, &mode, &ktab, &vis, &sub, &weight, &grid};
   return direct_launch(p, fn, args, s);
+}
+
+// Whether a call takes the direct gridder by itself.  A wait limit of 0 keeps to the
+// lane kernel (lane_launch) where that would run.
+static bool direct_wanted(const cg_plan *p, bool lane) {
+  const cg_tuning t = tuning();
+  return t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0 && direct_fits(*p) &&
+         !(lane && wait_cycles() == 0);
 }
 
 static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
@@ -810,19 +824,13 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   int gsize = 0, ngroups = 0;
   bool shared = false;
   if (p->outer) return outer_launch(p, kt, vv, nullptr, weight, mode, gg, s);
-  const bool automatic = t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0;
   const bool lane = layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0);
-  // Automatic: taps straight into the grid while few visibilities meet in a cell
-  // (L2 takes atomics on one address in turn), and, where the lane kernel can
-  // take its place, few visibilities in all (direct / lane / warp gridder, us: S 8,
-  // 150k on 1024^2: 32 / 42; 500k on 2048^2: 70 / 73; 2M: 300 / 202; S 12, 500k: 146 /
-  // 152, 2M: 586 / 455; S 16, 60k: 38 / 46, 150k: 79 / 64; S 6, 3M on 4096^2: 296 / 354,
-  // 2M on 2048^2: 223 / 221; S 9, 2M: 382 / 301 / 453, on 300^2: 685 / - / 432).  A
-  // wait limit of 0 keeps to the lane kernel (lane_launch).
-  const double rho = (double)p->n / ((double)p->H * (double)p->W * (double)p->layers);
-  const bool few = !lane || (S <= 6 ? rho < 0.4 : p->n < (S == 16 ? 120000 : 450000));
-  if (automatic && S <= 16 && rho < 1.5 && few && !(lane && wait_cycles() == 0))
-    return direct_grid_launch(p, kt, vv, weight, mode, gg, s);
+  // Taps straight into the grid while visibilities are few (direct_fits: accuracy
+  // sets the line, and below it this is the fastest too, direct / lane / warp
+  // gridder, us: S 8, 30k on 512^2: 11 / 24 / 23; S 16: 22 / 32 / 53; 60k on 4096^2, S 8:
+  // 13 / 56 / 53).
+  if (direct_wanted(p, lane))
+    return direct_grid_launch(p, kt, vv, nullptr, weight, mode, gg, s);
   if (lane) return lane_launch(p, kt, vv, weight, mode, gg, nullptr, nullptr, 0, false, s);
   if (layout_for(p->kd) != CG_LAYOUT_OWNER) {
     const int need = (S * S + 31) / 32;
@@ -895,7 +903,7 @@ int cg_grid_sparse(const cg_plan *p, const void *ktab, const void *vis, void *gr
   if (p->n == 0) return CG_OK;
   CG_REQUIRE(ktab && vis && grid, "NULL argument");
   if (p->kd.S <= 16)
-    return direct_grid_launch(p, (const float2 *)ktab, (const float2 *)vis, nullptr, 0,
+    return direct_grid_launch(p, (const float2 *)ktab, (const float2 *)vis, nullptr, nullptr, 0,
                               (float2 *)grid, (cudaStream_t)stream);
   const int SS = p->kd.S * p->kd.S;
   const int need = (SS + 31) / 32;
@@ -988,22 +996,27 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
   cudaStream_t s = (cudaStream_t)stream;
   const int S = p->kd.S;
   const cg_tuning t = tuning();
-  // Separable tables, small tiles: a block per tile has too little to do in one
-  // traversal, and the table is small, so reading it twice costs nothing.  Not
-  // in place: the second pass reads what the first would have overwritten.
+  const bool lane = layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0);
+  // Degrid, then grid, by the kernels that do each best: few visibilities (a tile's
+  // windows of both grids cost more than they hold; 60k on 4096^2, S 8, separable:
+  // 173 us in one traversal, 22 so), and separable tables on the register-window
+  // gridder's small tiles, whose table is small, so reading it twice costs nothing.
+  // Not in place: the second pass reads what the first would have overwritten.
+  const bool direct = direct_wanted(p, lane);
   const char *vi0 = (const char *)vis_in, *vo0 = (const char *)vis_out;
   const size_t vbytes = (size_t)p->n * sizeof(float2);
   const bool apart = !vis_in || !vis_out || vi0 + vbytes <= vo0 || vo0 + vbytes <= vi0;
-  if (p->outer && apart && (vis_out || !residual)) {
+  if ((p->outer || direct) && apart && (vis_out || !residual)) {
     if (vis_out) {
       const int rc = cg_degrid(p, ktab, grid_in, vis_out, stream);
       if (rc) return rc;
     }
     if (!vis_in) return CG_OK;
-    return outer_launch(p, (const float2 *)ktab, (const float2 *)vis_in, (const float2 *)vis_out,
-                        nullptr, residual ? 3 : 0, (float2 *)grid_out, s);
+    const auto launch = p->outer ? outer_launch : direct_grid_launch;
+    return launch(p, (const float2 *)ktab, (const float2 *)vis_in, (const float2 *)vis_out,
+                  nullptr, residual ? 3 : 0, (float2 *)grid_out, s);
   }
-  if (layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0))
+  if (lane)
     return lane_launch(p, (const float2 *)ktab, (const float2 *)vis_in, nullptr, 0,
                        (float2 *)grid_out, (const float2 *)grid_in, (float2 *)vis_out, residual,
                        true, s);

@@ -759,12 +759,12 @@ static int tile_edge(const cg_kernel_desc &kd, int req) {
 
 // Window edge of the register-window gridder for separable tables
 // (grid_outer.cu) and its tile edge T (window >= T + S - 1), or 0 where another
-// gridder runs: its cost per visibility hardly depends on S, and its flush per
-// tile is spread over the tile's visibilities, so it takes wide supports, and
-// narrow ones where visibilities are dense (direct gridder / this one, us: S 8,
-// 0.24 visibilities per cell, 1M: 159 / 124, 0.06: 136 / 176; S 13, 0.06: 297 /
-// 243; S 16, 0.05, 200k: 101 / 81; S 6, 0.24: 97 / 125, 1.0: 120 / 111).  Stacks of
-// grids, requested or tuned tiles and tuned layouts keep the other gridders.
+// gridder runs: the direct one for few visibilities (direct_fits), the one with
+// shared-memory tiles for the narrowest supports unless visibilities are dense
+// (its time goes with S, the window's flush does not; plan and grid, warp gridder
+// / this one, us: S 3, 1M on 2048^2: 153 / 181, S 5: 174 / 179, on 4096^2: 200 / 183,
+// S 6: 210 / 172, S 8: 239 / 170, on 4096^2: 259 / 218).  Stacks of grids, requested
+// or tuned tiles and tuned layouts keep the other gridders.
 static int outer_edge(const cg_plan &p, int &T) {
   const cg_tuning t = tuning();
   const int S = p.kd.S;
@@ -772,33 +772,28 @@ static int outer_edge(const cg_plan &p, int &T) {
       t.layout > 0 || (int64_t)p.kd.G * p.kd.Q * S >= INT32_MAX)
     return 0;
   const double rho = (double)p.n / ((double)p.H * (double)p.W);
-  if (rho < (S >= 10 ? 0.03 : S >= 7 ? 0.1 : 1.5)) return 0;
-  if (S <= 9) {
-    T = S <= 5 ? 12 : 8;
-    return 16;
-  }
-  T = S <= 13 ? 12 : 8;
-  return 24;
+  if (direct_fits(p) || (S <= 4 && rho < 1.5)) return 0;
+  // larger tiles where they fit the window and are not full: fewer flushes, but
+  // more visibilities to a counter of the plan (S 5, 1M on 1024^2: plan 117 us with
+  // tiles of 12, 74 with 8, gridder 99 with either)
+  T = rho < 0.25 && (S <= 5 || (S >= 10 && S <= 13)) ? 12 : 8;
+  return S <= 9 ? 16 : 24;
 }
 
-// Under no tuning and no requested tile, supports up to 16 get the lane layout's
-// 16-cell tiles where layout_for names the warp layout: 4-D tables of odd
-// support, for the lane kernel with taps by loads, and separable ones that the
-// direct kernels grid, which need no order inside a tile.  Not for stacks of so
-// many tiles that their numbers would run out.
-static bool small_tiles(const cg_plan &p) {
-  const cg_tuning t = tuning();
-  const int64_t tiles = (int64_t)((p.W + 15) / 16) * ((p.H + 15) / 16) * p.layers;
-  return !p.lean && p.kd.S <= 16 && p.tile_req == 0 && t.tile == 0 && t.layout == 0 &&
-         tiles <= (1 << 24);
-}
+// 4-D tables of odd support, which layout_for gives to the warp layout, get the
+// lane layout's 16-cell tiles under no tuning and no requested tile, for the lane
+// kernel with taps by loads: not for the narrowest, nor where tiles are nearly
+// empty (plan and grid, warp gridder / lane kernel, us: S 9, 123k on 1531^2: 94 / 81,
+// 2M on 4096^2: 541 / 467, 400k: 172 / 168; S 7, 2M: 422 / 419, 545 / 578 fused).  Not for
+// stacks of so many tiles that their numbers would run out.
 static bool lane_odd(const cg_plan &p) {
-  return small_tiles(p) && !p.kd.sep && p.kd.S % 2 == 1 &&
+  const cg_tuning t = tuning();
+  const int S = p.kd.S;
+  const int64_t tiles = (int64_t)((p.W + 15) / 16) * ((p.H + 15) / 16) * p.layers;
+  const double cells = (double)p.H * (double)p.W * (double)p.layers;
+  return !p.lean && !p.kd.sep && S >= 9 && S <= 16 && S % 2 == 1 && p.tile_req == 0 &&
+         t.tile == 0 && t.layout == 0 && tiles <= (1 << 24) && (double)p.n >= 0.04 * cells &&
          (int64_t)p.kd.G * p.kd.Q * p.kd.Q < INT32_MAX;
-}
-static bool direct_sep(const cg_plan &p) {
-  return small_tiles(p) && p.kd.sep && !p.outer &&
-         (double)p.n < 1.5 * (double)p.H * (double)p.W * (double)p.layers;
 }
 
 static void plan_geometry(cg_plan &p) {
@@ -807,8 +802,11 @@ static void plan_geometry(cg_plan &p) {
     p.outer = outer_edge(p, outer_T);
     p.lane_odd = lane_odd(p);
     const bool lane = p.lane_odd || layout_for(p.kd) == CG_LAYOUT_LANE;
-    const bool flat = p.outer || lane || direct_sep(p);  // no order inside a tile
-    p.T = p.outer ? outer_T : flat && small_tiles(p) ? 16 : tile_edge(p.kd, p.tile_req);
+    const cg_tuning t = tuning();
+    // no order inside a tile (for few visibilities it is not worth its buckets)
+    const bool flat =
+        p.outer || lane || (!p.lean && t.layout == 0 && t.tile == 0 && direct_fits(p));
+    p.T = p.outer ? outer_T : p.lane_odd ? 16 : tile_edge(p.kd, p.tile_req);
     p.ntx = (p.W + p.T - 1) / p.T;
     p.nty = (p.H + p.T - 1) / p.T;
     // Morton blocks of up to 32 x 32 tiles (no larger than the grid needs)
@@ -817,11 +815,10 @@ static void plan_geometry(cg_plan &p) {
     const int nby = (p.nty + (1 << p.tblog) - 1) >> p.tblog;
     p.tpl = (p.nbx * nby) << (2 * p.tblog);
     p.ntiles = p.tpl * p.layers;
-    const cg_tuning t = tuning();
     // 4x4-cell sub-tiles, 2^sublog per tile edge (4 << full >= T), except for the
     // lane layout and the separable gridder, whose private windows need no order
-    // inside a tile (tile buckets only).  The sub-tile edge is 1 << subshift cells, so that an
-    // in-tile coordinate shifted by subshift is always below 2^sublog.
+    // inside a tile (tile buckets only), and few visibilities.  The sub-tile edge is 1 <<
+    // subshift cells, so that an in-tile coordinate shifted by subshift is always below 2^sublog.
     int full = 0;
     while ((4 << full) < p.T) ++full;
     p.sublog = flat ? 0 : full;
