@@ -186,8 +186,8 @@ __global__ void k_plan_coords(CoordParams P) {
       }
       int g = 0;
       if (P.wstep != 0.0) {
-        const double j = w_bin_fast(P.uvw[i * P.stride + 2], P.wstep, P.inv_wstep) - P.kmin;
-        g = (j >= 0.0 && j < (double)P.nk) ? (int)j : -1;
+        const long long j = w_bin_fast(P.uvw[i * P.stride + 2], P.wstep, P.inv_wstep) - P.kmin;
+        g = (j >= 0 && j < P.nk) ? (int)j : -1;
       } else if (P.kidx) {
         g = P.kidx[i];
       }
@@ -457,8 +457,8 @@ __global__ void k_w_bins(const double *uvw, int64_t stride, int64_t n, double ws
   int lo = INT32_MAX, hi = INT32_MIN, bad = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const double k = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep);
-    if (!(k > -1.0e9 && k < 1.0e9)) {
+    const long long k = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep);
+    if (!(k > -1000000000 && k < 1000000000)) {
       ++bad;
       kidx[i] = 0;
     } else {
@@ -483,9 +483,8 @@ __global__ void k_w_bins_fixed(const double *uvw, int64_t stride, int64_t n, dou
                                int32_t *status) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double k = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep);
-  const double j = k - (double)kmin;
-  if (!(j >= 0.0 && j < (double)nk)) {
+  const long long j = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep) - kmin;
+  if (!(j >= 0 && j < nk)) {
     atomicAdd(&status[ST_INDEX], 1);
     kidx[i] = 0;
     return;
@@ -539,13 +538,15 @@ __global__ void k_uvw_ranges(const double *__restrict__ uvw, int64_t stride, int
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const double x = p[c];
-      const unsigned long long b = order_bits(x), m = x != x ? ~order_bits(-INFINITY) : ~b;
+      const unsigned long long b = order_bits(x);
+      const bool nan = (unsigned long long)__double_as_longlong(x) << 1 > 0x7FFull << 53;
+      const unsigned long long m = nan ? ~order_bits(-INFINITY) : ~b;
       hi = b > hi ? b : hi;
       lo = m > lo ? m : lo;
     }
     if (wstep != 0.0) {
-      const double k = w_bin_fast(p[2], wstep, inv_wstep);
-      if (k > -1.0e9 && k < 1.0e9) {
+      const long long k = w_bin_fast(p[2], wstep, inv_wstep);
+      if (k > -1000000000 && k < 1000000000) {
         const uint32_t b = (uint32_t)(int)k ^ 0x80000000u;
         whi = max(whi, b);
         wlo = max(wlo, ~b);
@@ -706,8 +707,8 @@ __global__ void k_row_keys(const double *__restrict__ uvw, int64_t stride, int64
                            int32_t *__restrict__ key, int32_t *status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double j = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep) - (double)kmin;
-  bool ok = j >= 0.0 && j < (double)nbins;
+  const long long j = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep) - kmin;
+  bool ok = j >= 0 && j < nbins;
   int64_t k = ok ? (int64_t)j : 0;
   for (int c = 0; c < C.ncols; ++c) {
     const int v = cols[i * C.ncols + c] - C.mins[c];
@@ -730,9 +731,9 @@ __global__ void k_aw_keys(const double *__restrict__ uvw, int64_t stride,
                           int nbins, int32_t *__restrict__ key, int32_t *status) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double j = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep) - (double)kmin;
+  const long long j = w_bin_fast(uvw[i * stride + 2], wstep, inv_wstep) - kmin;
   const int p = a1[i], q = a2[i];
-  if (!(j >= 0.0 && j < (double)nbins) || p < 0 || p >= nant || q < 0 || q >= nant) {
+  if (!(j >= 0 && j < nbins) || p < 0 || p >= nant || q < 0 || q >= nant) {
     atomicAdd(&status[ST_INDEX], 1);
     key[i] = 0;
     return;

@@ -42,32 +42,36 @@ __device__ __forceinline__ int64_t floor_div_ll(int64_t a, int64_t b) {
 // in w_bin_fast: F = round(t * (1/C) * 2^20) from one FMA decides unless the
 // quotient lies within FIX_MARGIN units of an integer, where the exact
 // quotient is formed.  |t / C| < 2^30 on the fast path.
-__device__ __forceinline__ double floor_div_fast(double t, double C, double invC) {
+static __device__ __noinline__ long long floor_div_exact(double t, double C) {
+  return whole_bin(floor(__ddiv_rn(t, C)));
+}
+__device__ __forceinline__ long long floor_div_fast(double t, double C, double invC) {
   const double e = fma(t, invC, FIX_MAGIC);
   const long long F = (long long)((unsigned long long)__double_as_longlong(e) - FIX_MAGIC_BITS);
   if (F > -(1ll << 50) && F < (1ll << 50)) {
     const long long fr = F & (FIX_ONE - 1);
-    if (fr > FIX_MARGIN && fr < FIX_ONE - FIX_MARGIN) return (double)(F >> FIX_BITS);
+    if (fr > FIX_MARGIN && fr < FIX_ONE - FIX_MARGIN) return F >> FIX_BITS;
   }
-  return floor(__ddiv_rn(t, C));
+  return floor_div_exact(t, C);
 }
 
 // Pass 1: bins (ub, vb, wp) of every visibility, their ranges, and the bins
 // stored as three int32 at the start of the visibility's rel row (pass 2
 // reads them back before overwriting the row).
 __global__ void k_tower_bounds(const double *__restrict__ uvw, int64_t stride, int64_t n,
-                               double theta, int C, double invC, double winc, double inv_winc,
+                               double theta, double C, double invC, double winc, double inv_winc,
                                int32_t *mm, double *__restrict__ rel, int32_t *status) {
   int mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
   int bad = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double *row = uvw + i * stride;
-    const double fu = floor_div_fast(__dmul_rn(row[0], theta), (double)C, invC);
-    const double fv = floor_div_fast(__dmul_rn(row[1], theta), (double)C, invC);
-    const double fw = w_bin_fast(row[2], winc, inv_winc);
+    const long long fu = floor_div_fast(__dmul_rn(row[0], theta), C, invC);
+    const long long fv = floor_div_fast(__dmul_rn(row[1], theta), C, invC);
+    const long long fw = w_bin_fast(row[2], winc, inv_winc);
     int32_t *bins = (int32_t *)(rel + 3 * i);
-    if (!(fabs(fu) < 1e9 && fabs(fv) < 1e9 && fabs(fw) < 1e9)) {  // NaN too
+    constexpr long long MOST = 1000000000;
+    if (!(llabs(fu) < MOST && llabs(fv) < MOST && llabs(fw) < MOST)) {  // NO_BIN too
       ++bad;
       bins[0] = bins[1] = bins[2] = INT32_MIN;
       continue;
