@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(512) k_lane(TiledArgs A, LaneArgs P) {
     const int t = lane + 32 * i;
     tdy[i] = STEP ? lane / S + i * (32 / S) : t / S;
     tdx[i] = STEP ? lane % S : t - tdy[i] * S;
-    own[i] = FULLT || t < SS;
+    own[i] = FULLT || (SC && 32 * i + 31 < SC * SC) || t < SS;
     soff[i] = STEP ? (lane / S) * pitch + lane % S + i * (32 / S) * pitch : tdy[i] * pitch + tdx[i];
     goff[i] = tdy[i] * A.W + tdx[i];
   }
@@ -262,7 +262,8 @@ __global__ void __launch_bounds__(512) k_lane(TiledArgs A, LaneArgs P) {
                      org.wx0 + (m.x & 0xffff);
 #pragma unroll
         for (int i = 0; i < MAXT; ++i)
-          if (own[i]) atomicAdd(&gp[(size_t)tdy[i] * A.W + tdx[i]], cmul(kc[i], u));
+          if (own[i])  // (offsets kept for grid_in, or made of constants)
+            atomicAdd(&gp[FUSED || STEP ? goff[i] : tdy[i] * A.W + tdx[i]], cmul(kc[i], u));
       } else {
         // distinct taps of one visibility are distinct cells: plain read-modify-write
 #pragma unroll
@@ -371,8 +372,23 @@ static int padded_table(const cg_plan *p, const float2 *&ktab, cudaStream_t s) {
   return CG_OK;
 }
 
+// Taps by loads, supports 8 to 15 on 16-cell tiles (pitch S + 16): support and
+// taps per lane fixed at compile time, where they were rounded up to a power of two
+// and every tap checked (2M visibilities, 4096^2, grid / fused, us: S 9 354 / 580 ->
+// 335 / 535, S 12 522 / 876 -> 375 / 615, S 15 608 / 986 -> 502 / 811).
+template <bool FUSED, int S = 15>
+static void *lane_fixed_for(int support) {
+  if (support == S)
+    return (void *)k_lane<false, false, FUSED, (S * S + 31) / 32, S * S % 32 == 0, S, S + 16>;
+  if constexpr (S > 8) return lane_fixed_for<FUSED, S - 1>(support);
+  return nullptr;
+}
+
 template <bool SEP, bool BULK, bool FUSED>
-static void *lane_kernel_for(int maxt, int SS, int pitch) {
+static void *lane_kernel_for(int maxt, int S, int pitch) {
+  const int SS = S * S;
+  if (!SEP && !BULK && pitch == S + 16)
+    if (void *fn = lane_fixed_for<FUSED>(S)) return fn;
   if (maxt == 8 && SS == 256 && pitch == 32) return (void *)k_lane<SEP, BULK, FUSED, 8, true, 16, 32>;
   if (maxt == 8 && SS == 256 && pitch == 48) return (void *)k_lane<SEP, BULK, FUSED, 8, true, 16, 48>;
   if (maxt == 8 && SS == 256) return (void *)k_lane<SEP, BULK, FUSED, 8, true>;
@@ -450,12 +466,12 @@ int lane_launch(const cg_plan *p, const float2 *ktab, const float2 *vis, const f
   const int warps = std::min(fit, t.groups > 0 ? t.groups
                                   : bulk       ? (int)std::max<size_t>(1, (220u << 10) / off)
                                                : 4);
-  void *fn = p->kd.sep ? (fused ? lane_kernel_for<true, false, true>(maxt, SS, p->pitch)
-                                : lane_kernel_for<true, false, false>(maxt, SS, p->pitch))
-                       : bulk ? (fused ? lane_kernel_for<false, true, true>(maxt, SS, p->pitch)
-                                       : lane_kernel_for<false, true, false>(maxt, SS, p->pitch))
-                              : (fused ? lane_kernel_for<false, false, true>(maxt, SS, p->pitch)
-                                       : lane_kernel_for<false, false, false>(maxt, SS, p->pitch));
+  void *fn = p->kd.sep ? (fused ? lane_kernel_for<true, false, true>(maxt, S, p->pitch)
+                                : lane_kernel_for<true, false, false>(maxt, S, p->pitch))
+                       : bulk ? (fused ? lane_kernel_for<false, true, true>(maxt, S, p->pitch)
+                                       : lane_kernel_for<false, true, false>(maxt, S, p->pitch))
+                              : (fused ? lane_kernel_for<false, false, true>(maxt, S, p->pitch)
+                                       : lane_kernel_for<false, false, false>(maxt, S, p->pitch));
   CG_REQUIRE(fn, "no lane-layout kernel for support %d", S);
   const size_t smem = (size_t)warps * off;
   const int threads = 32 * warps;

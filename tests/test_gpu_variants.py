@@ -213,7 +213,7 @@ def test_pad_even(env, S, G):
     assert torch.equal(torch.view_as_real(p.table).reshape(want.shape), want)
 
 
-@pytest.mark.parametrize("S", [2, 4, 6, 8, 9, 11, 12, 15, 16])
+@pytest.mark.parametrize("S", [2, 4, 6, 8, 9, 10, 11, 12, 13, 14, 15, 16])
 def test_grid_lane_loads(env, S):
     """4-D tables on dense visibilities (the lane kernel with taps by loads, odd
     supports on its tiles too), grids that end inside a tile and a stack, gridding and
