@@ -62,6 +62,11 @@ def _host(t, like=None, dtype=None):
         # conversion; larger results convert on the host, in less device memory
         t = t.to(E.CD if t.is_complex() else torch.float64 if t.is_floating_point() else
                  torch.int64 if t.dtype in (torch.int8, torch.int16, torch.int32) else t.dtype)
+        # into numpy's memory: torch's leaves the C heap handing pages of such sizes back
+        # on each call (do_imaging + do_predict at 1500^2: 4.2 against 2.1 ms)
+        a = numpy.empty(tuple(t.shape), dtype=torch.empty(0, dtype=t.dtype).numpy().dtype)
+        torch.from_numpy(a).copy_(t)
+        return a
     a = t.cpu().numpy()
     if dtype is not None:
         return a.astype(dtype)
