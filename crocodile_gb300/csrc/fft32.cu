@@ -220,9 +220,12 @@ __global__ void __launch_bounds__(RowShape<LOGN>::TPC, RowShape<LOGN>::MINB)
 }
 
 // Tiles of C columns of one plane (units = planes * W / C), T = H / 16
-// threads per column, thread (t, c) with c fastest for coalesced rows.
+// threads per column, thread (t, c) with c fastest for coalesced rows.  64
+// registers, so that a second CTA's loads run under the stages of the first
+// (rows and columns of a stack, one CTA of 128 registers / two, us: 2371 x 256^2
+// 903 / 838, 600 x 512^2 1144 / 939, 150 x 1024^2 1309 / 1164).
 template <int LOGH, int C, class IO>
-__global__ void __launch_bounds__(COL_THREADS) k_fft32_cols(IO io, int64_t nplanes, int W,
+__global__ void __launch_bounds__(COL_THREADS, 2) k_fft32_cols(IO io, int64_t nplanes, int W,
                                                             const float2 *__restrict__ tw,
                                                             int sign, float *max_out) {
   constexpr int H = 1 << LOGH, T = H / 16;
@@ -740,7 +743,11 @@ int launch_cols(const IO &io, int64_t nplanes, int W, int sign, float *max_out, 
   CG_CUDA(cudaFuncSetAttribute(k_fft32_cols<LOGH, C, IO>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t units = nplanes * (W / C);
-  const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * 2);
+  int per_sm = 0;
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fft32_cols<LOGH, C, IO>, C * T,
+                                                        smem));
+  CG_REQUIRE(per_sm > 0, "FP32 FFT columns do not fit on an SM (smem %zu)", smem);
+  const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * per_sm);
   k_fft32_cols<LOGH, C, IO><<<grid, C * T, smem, st>>>(io, nplanes, W, tw, sign, max_out);
   CG_LAUNCH("FP32 FFT columns");
   return CG_OK;
