@@ -240,6 +240,80 @@ __global__ void k_aw_akern(const double2 *__restrict__ A, int SA,
   }
 }
 
+// The FP32 form for SA = 16, the size of the FFT form's kernels: 64 threads per AW
+// kernel, four rows of one column of outputs each, so that a column of A[a2],
+// zero-padded in shared memory, slides through registers past them: 35 loads for
+// 64 complex products where every output on its own takes 128 and tests every
+// index.  Bound by FP32 issue: 6,000 AW kernels 124 -> 72 us, and the table's error
+// against 64 bits 4e-7 -> 2e-7.
+template <int SA>
+__global__ void __launch_bounds__(256) k_aw_akern_f(const double2 *__restrict__ A,
+                                                    const int32_t *__restrict__ a1,
+                                                    const int32_t *__restrict__ a2, int nk, int nA,
+                                                    float2 *__restrict__ akern, int32_t *status) {
+  constexpr int RB = 4, TPK = SA * SA / RB, KPB = 256 / TPK, P = 2 * SA - 1, o = (SA - 1) / 2;
+  static_assert(SA % RB == 0 && 256 % TPK == 0, "whole row blocks and kernels per CTA");
+  __shared__ float2 su[KPB][SA * SA], sv[KPB][P * P];
+  const int g = threadIdx.x / TPK, t = threadIdx.x % TPK;
+  const int k = blockIdx.x * KPB + g;
+  bool ok = k < nk;
+  if (ok) {
+    const int i1 = a1[k], i2 = a2[k];
+    if (i1 < 0 || i1 >= nA || i2 < 0 || i2 >= nA) {
+      if (t == 0) atomicAdd(&status[ST_INDEX], 1);
+      ok = false;
+    } else {
+      const double2 *u = A + (size_t)i1 * SA * SA, *v = A + (size_t)i2 * SA * SA;
+      for (int e = t; e < SA * SA; e += TPK) su[g][e] = make_float2((float)u[e].x, (float)u[e].y);
+      for (int e = t; e < P * P; e += TPK) {
+        const int y = e / P - (SA - 1 - o), x = e % P - (SA - 1 - o);
+        float2 r = make_float2(0.f, 0.f);
+        if (y >= 0 && y < SA && x >= 0 && x < SA) {
+          const double2 d = v[y * SA + x];
+          r = make_float2((float)d.x, (float)d.y);
+        }
+        sv[g][e] = r;
+      }
+    }
+  }
+  __syncthreads();
+  if (!ok) return;
+  const int j = t % SA, i0 = t / SA * RB;
+  float2 sum[RB];
+#pragma unroll
+  for (int r = 0; r < RB; ++r) sum[r] = make_float2(0.f, 0.f);
+  for (int q = 0; q < SA; ++q) {  // columns summed by themselves: shorter chains of roundings
+    float2 acc[RB];
+#pragma unroll
+    for (int r = 0; r < RB; ++r) acc[r] = make_float2(0.f, 0.f);
+    // same[i, j] += u[p, q] v[i - p, j - q] (padded indices), i = i0 .. i0 + RB - 1
+    const float2 *col = sv[g] + i0 * P + j - q + SA - 1;
+    float2 w[SA + RB - 1];
+#pragma unroll
+    for (int y = 0; y < SA + RB - 1; ++y) w[y] = col[y * P];
+#pragma unroll
+    for (int p = 0; p < SA; ++p) {
+      const float2 u = su[g][p * SA + q];
+#pragma unroll
+      for (int r = 0; r < RB; ++r) {
+        const float2 v = w[r - p + SA - 1];
+        acc[r].x = fmaf(u.x, v.x, acc[r].x);
+        acc[r].x = fmaf(-u.y, v.y, acc[r].x);
+        acc[r].y = fmaf(u.x, v.y, acc[r].y);
+        acc[r].y = fmaf(u.y, v.x, acc[r].y);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      sum[r].x += acc[r].x;
+      sum[r].y += acc[r].y;
+    }
+  }
+  float2 *dst = akern + (size_t)k * SA * SA + i0 * SA + j;
+#pragma unroll
+  for (int r = 0; r < RB; ++r) dst[r * SA] = sum[r];
+}
+
 template <typename C>
 __global__ void k_aw_conv(const float2 *__restrict__ akern, int SA,
                           const float2 *__restrict__ Wk, int nW, int Q, int S,
@@ -595,8 +669,12 @@ int cg_aw_kernels(const void *A, int nA, int SA, const void *Wk, int nW, int Q, 
   if (sh_a > 48 * 1024)
     CG_CUDA(cudaFuncSetAttribute(k_aw_akern<float, float2>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh_a));
-  k_aw_akern<float, float2><<<nk, 256, sh_a, st>>>((const double2 *)A, SA, a1, a2, nA, akern,
+  if (SA == 16)
+    k_aw_akern_f<16><<<(nk + 3) / 4, 256, 0, st>>>((const double2 *)A, a1, a2, nk, nA, akern,
                                                    d_status);
+  else
+    k_aw_akern<float, float2><<<nk, 256, sh_a, st>>>((const double2 *)A, SA, a1, a2, nA, akern,
+                                                     d_status);
   CG_LAUNCH("aw akern");
   if (fft_form)  // complex64 tables: the FFT form
     return aw_fft_launch(akern, nk, Wk, nW, Q, S, wi, out, 1,

@@ -387,3 +387,22 @@ def test_towers_stack(env, S):
         call(x, 1.5, w, first, st)
         with pytest.raises(Exception):
             st.check()
+
+
+@pytest.mark.parametrize("nk", [1, 3, 4, 6])
+def test_aw_akern_blocks(env, nk):
+    """A1 * A2 by four kernels to a block: part-filled last blocks, and one bad index
+    that loses its own kernel's call only.  Tolerance 2e-6 of the norm against the
+    complex128 form: sums of 256 products, twice."""
+    torch, L, E, _, O = env
+    rng = numpy.random.default_rng(nk)
+    A = rng.normal(size=(5, 16, 16)) + 1j * rng.normal(size=(5, 16, 16))
+    W = rng.normal(size=(2, 2, 2, 16, 16)) + 1j * rng.normal(size=(2, 2, 2, 16, 16))
+    a1, a2 = rng.integers(0, 5, (2, nk)).astype(numpy.int32)
+    wi = rng.integers(0, 2, nk).astype(numpy.int32)
+    _near(E.aw_kernels(A, W, a1, a2, wi, dtype=E.CF).to(E.CD),
+          E.aw_kernels(A, W, a1, a2, wi, dtype=E.CD), 2e-6)
+    a1[-1] = 5
+    with pytest.raises(Exception):
+        E.aw_kernels(A, W, a1, a2, wi, dtype=E.CF)
+        torch.cuda.synchronize()
