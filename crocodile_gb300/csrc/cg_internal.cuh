@@ -296,6 +296,18 @@ struct cg_plan {
 
 // Internal entry points shared across translation units.
 namespace cg {
+// Records that a plan sorted: all n, or fewer where coordinates or indices were
+// refused.  The rest of recs and perm is never written, and the status block that
+// tells of the refusal is the caller's to reset, so kernels that walk the sorted
+// order itself end here.
+struct SortedEnd {
+  const int32_t *offset, *count;  // of the last bucket
+  __device__ __forceinline__ int operator()() const { return *offset + *count; }
+};
+inline SortedEnd sorted_end(const cg_plan *p) {
+  return {p->offsets + p->nbuckets - 1, p->counts + p->nbuckets - 1};
+}
+
 // Few enough visibilities to add their taps one by one to the grid in memory
 // (k_grid_direct): the sum in a cell rounds with each, so its error grows with the
 // root of the number of its taps, where the other gridders sum a tile's share

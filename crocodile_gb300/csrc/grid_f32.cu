@@ -602,7 +602,7 @@ static void *grid_warp_kernel_for(int maxt) {
 // against 479; 4M visibilities on 32 stacked 4096^2 grids: 0.60 against 2.06 ms.
 struct DirectArgs {
   TiledArgs A;
-  int64_t n;
+  SortedEnd end;
   int layered;  // grids of a stack: by work item, which knows its layer
 };
 
@@ -613,8 +613,9 @@ __device__ __forceinline__ void direct_batches(const DirectArgs &D, F f) {
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   if (!D.layered) {
-    for (int64_t b = gw * 32; b < D.n; b += nw * 32)
-      f((int)b, (int)min((int64_t)32, D.n - b), (size_t)0);
+    const int64_t n = D.end();
+    for (int64_t b = gw * 32; b < n; b += nw * 32)
+      f((int)b, (int)min((int64_t)32, n - b), (size_t)0);
     return;
   }
   const int nitems = *D.A.nitems;
@@ -781,7 +782,7 @@ static int direct_launch(const cg_plan *p, void *fn, void **args, cudaStream_t s
 static DirectArgs direct_args(const cg_plan *p) {
   DirectArgs D;
   D.A = tiled_args(p);
-  D.n = p->n;
+  D.end = sorted_end(p);
   D.layered = p->layers > 1;
   return D;
 }

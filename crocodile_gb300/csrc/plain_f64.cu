@@ -26,6 +26,7 @@ struct PlainArgs {
   const VisRec *recs;
   const int32_t *perm;
   const int32_t *status;
+  SortedEnd end;
   int W, S, Q, sep;
 };
 
@@ -45,6 +46,7 @@ __global__ void k_grid_plain(PlainArgs A, int start, int count,
   if (any_failed(A.status)) return;
   const int SS = A.S * A.S;
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  count = min(count, A.end() - start);
   if (idx >= (int64_t)count * SS) return;
   const int j = (int)(idx / SS), t = (int)(idx - (int64_t)j * SS);
   const int dy = t / A.S, dx = t - dy * A.S;
@@ -80,6 +82,8 @@ __global__ void k_degrid_plain(PlainArgs A, int start, int count,
   if (any_failed(A.status)) return;
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int sub = threadIdx.x % PLAIN_LANES;
+  count = min(count, A.end() - start);
+  if (count <= 0) return;
   const bool live = t0 / PLAIN_LANES < count;
   const int j = live ? (int)(t0 / PLAIN_LANES) : count - 1;  // the shuffles need whole warps
   const int S = A.S;
@@ -183,6 +187,7 @@ static PlainArgs plain_args(const cg_plan *p) {
   A.recs = p->recs;
   A.perm = p->perm;
   A.status = p->status;
+  A.end = sorted_end(p);
   A.W = p->W;
   A.S = p->kd.S;
   A.Q = p->kd.Q;
@@ -197,7 +202,7 @@ static PlainArgs plain_args(const cg_plan *p) {
 // those launches and, with one grid, without the groups' ranges on the host).
 static void plain_range(const cg_plan *p, int layer, int64_t &start, int64_t &count) {
   start = 0;
-  count = p->n;  // (with errors fewer are sorted, and the kernels return)
+  count = p->n;  // (the kernels end at the last one sorted)
   if (p->layers == 1) return;
   const int g0 = layer * p->gper, g1 = g0 + p->gper - 1;
   start = p->h_offsets[g0];
