@@ -438,10 +438,17 @@ __global__ void __launch_bounds__(32 * (1 << (LOGL - 4)), step_minb(LOGL))
 // 0, plane), pass B's (32, H2, 1, 1) at (col0, 0, k1, plane).  Every wait is
 // bounded by the process-wide wait limit (cg_set_wait_limit; 0 polls once
 // without blocking); on expiry the CTA counts the timeout in
-// g_fft32_timeouts (cg_fft_timeouts), waits for its copies in flight (at
-// most the default limit each) and stops, leaving its units' output undefined.
+// g_fft32_timeouts (cg_fft_timeouts) and, for calls that have one, in the status
+// block, waits for its copies in flight (at most the default limit each) and
+// stops, leaving its units' output undefined.
 constexpr long long FFT_WAIT_CYCLES = 4000000000ll;
 __device__ int g_fft32_timeouts;
+
+// by one thread of the CTA that gave up
+__device__ __forceinline__ void count_timeout(int32_t *status) {
+  atomicAdd(&g_fft32_timeouts, 1);
+  if (status) atomicAdd(&status[ST_TIMEOUT], 1);
+}
 
 __device__ __forceinline__ bool tile_wait(uint64_t *bar, uint32_t parity, long long cycles) {
   return cycles ? mbar_wait_cycles(bar, parity, cycles) : mbar_test(bar, parity);
@@ -460,7 +467,7 @@ template <int LOGL, class IO>
 __global__ void __launch_bounds__(TmaShape<LOGL>::THREADS, step_minb(LOGL))
     k_fft32_step_tma(const __grid_constant__ CUtensorMap tmap, IO io, int64_t units,
                      int box_a, const float2 *__restrict__ tw, int sign, float *max_out,
-                     long long wait) {
+                     long long wait, int32_t *status) {
   using TS = TmaShape<LOGL>;
   constexpr int L = TS::L, T = L / 16, C = TS::C, NS = (LOGL + 3) / 4;
   extern __shared__ unsigned char f32_tsm[];
@@ -498,7 +505,7 @@ __global__ void __launch_bounds__(TmaShape<LOGL>::THREADS, step_minb(LOGL))
       // let this tile's copy and the next one's land before the CTA (and its
       // shared memory) goes away
       if (threadIdx.x == 0) {
-        atomicAdd(&g_fft32_timeouts, 1);
+        count_timeout(status);
         mbar_wait_cycles(&bar[b], (it >> 1) & 1, FFT_WAIT_CYCLES);
         if (next) mbar_wait_cycles(&bar[b ^ 1], ((it + 1) >> 1) & 1, FFT_WAIT_CYCLES);
       }
@@ -601,7 +608,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 template <int LOGL, class IO>
 int launch_step_tma_as(const IO &io, const float2 *in, int W, int H1, int H2, int64_t nplanes,
                        bool box_a, int64_t units, int sign, float *max_out, cudaStream_t st,
-                       bool *used) {
+                       bool *used, int32_t *status) {
   using TS = TmaShape<LOGL>;
   *used = false;
   const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
@@ -629,7 +636,7 @@ int launch_step_tma_as(const IO &io, const float2 *in, int W, int H1, int H2, in
   if (per_sm < 1) return CG_OK;
   const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * per_sm);
   k_fft32_step_tma<LOGL, IO><<<grid, TS::THREADS, smem, st>>>(map, io, units, box_a ? 1 : 0, tw,
-                                                              sign, max_out, wait_cycles());
+                                                              sign, max_out, wait_cycles(), status);
   CG_LAUNCH("FP32 FFT column step (TMA)");
   *used = true;
   return CG_OK;
@@ -638,17 +645,17 @@ int launch_step_tma_as(const IO &io, const float2 *in, int W, int H1, int H2, in
 template <class IO>
 int launch_step_tma(int logl, const IO &io, const float2 *in, int W, int H1, int H2,
                     int64_t nplanes, bool box_a, int64_t units, int sign, float *max_out,
-                    cudaStream_t st, bool *used) {
+                    cudaStream_t st, bool *used, int32_t *status = nullptr) {
   switch (logl) {
     case 5:
       return launch_step_tma_as<5>(io, in, W, H1, H2, nplanes, box_a, units, sign, max_out, st,
-                                   used);
+                                   used, status);
     case 6:
       return launch_step_tma_as<6>(io, in, W, H1, H2, nplanes, box_a, units, sign, max_out, st,
-                                   used);
+                                   used, status);
     case 7:
       return launch_step_tma_as<7>(io, in, W, H1, H2, nplanes, box_a, units, sign, max_out, st,
-                                   used);
+                                   used, status);
   }
   *used = false;
   return CG_OK;
@@ -921,7 +928,7 @@ struct StackShape {
 template <int LOGL, int C>
 __global__ void __launch_bounds__(StackShape<LOGL, C>::THREADS, StackShape<LOGL, C>::MINB)
     k_fft32_stack(const __grid_constant__ CUtensorMap tmap, StackArgs A, int64_t units,
-                  const float2 *__restrict__ tw, int sign, long long wait) {
+                  const float2 *__restrict__ tw, int sign, long long wait, int32_t *status) {
   using TS = StackShape<LOGL, C>;
   constexpr int L = TS::L, T = L / 16, NS = (LOGL + 3) / 4;
   extern __shared__ unsigned char f32_tsm[];
@@ -984,7 +991,7 @@ __global__ void __launch_bounds__(StackShape<LOGL, C>::THREADS, StackShape<LOGL,
       const bool ok = tile_wait(&bar[b], (it >> 1) & 1, wait);
       if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) {
-          atomicAdd(&g_fft32_timeouts, 1);
+          count_timeout(status);
           mbar_wait_cycles(&bar[b], (it >> 1) & 1, FFT_WAIT_CYCLES);
           if (next) mbar_wait_cycles(&bar[b ^ 1], ((it + 1) >> 1) & 1, FFT_WAIT_CYCLES);
         }
@@ -1129,7 +1136,7 @@ int stack_scratch(int layers, int N, double theta, const double *w, const int32_
 
 template <int LOGL, int C>
 int launch_stack(const CUtensorMap &map, const StackArgs &A, int64_t units, int sign,
-                 cudaStream_t st) {
+                 int32_t *status, cudaStream_t st) {
   using TS = StackShape<LOGL, C>;
   const float2 *tw;
   int rc = twiddles(LOGL, sign, &tw);
@@ -1142,7 +1149,7 @@ int launch_stack(const CUtensorMap &map, const StackArgs &A, int64_t units, int 
   CG_REQUIRE(per_sm > 0, "FP32 FFT stack columns do not fit on an SM (smem %zu)", TS::smem());
   const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * per_sm);
   k_fft32_stack<LOGL, C><<<grid, TS::THREADS, TS::smem(), st>>>(map, A, units, tw, sign,
-                                                                wait_cycles());
+                                                                wait_cycles(), status);
   CG_LAUNCH("FP32 FFT stack columns");
   return CG_OK;
 }
@@ -1317,7 +1324,7 @@ int fft32_wstack(float2 *planes, int layers, int N, double theta, const double *
   const int64_t ua = (int64_t)layers * sa.nj * sa.tiles;
   bool tma;
   rc = f32::launch_step_tma(l1, sA, planes, N, 1 << l1, 1 << l2, layers, true, ua, 1, nullptr, st,
-                            &tma);
+                            &tma, status);
   if (!rc && !tma) rc = f32::launch_step(l1, sA, ua, 1, nullptr, st);
   if (rc) return rc;
   f32::StackScratch sc;
@@ -1325,8 +1332,8 @@ int fft32_wstack(float2 *planes, int layers, int N, double theta, const double *
   f32::StackArgs A{N,      1 << l1, N / 32, 1 << l1, N / 2, false, sc.first, sc.list, sc.ph,
                    image, (int64_t)N * N, (float)(1.0 / ((double)N * N))};
   const int64_t units = (int64_t)A.tiles * A.nj;
-  rc = l2 == 5 ? f32::launch_stack<5, 32>(map, A, units, 1, st)
-               : f32::launch_stack<6, 32>(map, A, units, 1, st);
+  rc = l2 == 5 ? f32::launch_stack<5, 32>(map, A, units, 1, status, st)
+               : f32::launch_stack<6, 32>(map, A, units, 1, status, st);
   const cudaError_t fe = cudaFreeAsync(sc.list, st);
   if (rc) return rc;
   CG_CUDA(fe);
@@ -1354,9 +1361,9 @@ int fft32_towers_sum(float2 *stack, int layers, int S, double theta, const doubl
   f32::StackArgs A{S,   1,   S / C, 1, S / 2, true, chunk_first, sc.list, sc.ph,
                    out, (int64_t)S * S, 1.0f / (float)((int64_t)S * S)};
   const int64_t units = (int64_t)nchunks * A.tiles;
-  rc = ls == 6   ? f32::launch_stack<6, 32>(map, A, units, 1, st)
-       : ls == 7 ? f32::launch_stack<7, 32>(map, A, units, 1, st)
-                 : f32::launch_stack<8, 16>(map, A, units, 1, st);
+  rc = ls == 6   ? f32::launch_stack<6, 32>(map, A, units, 1, status, st)
+       : ls == 7 ? f32::launch_stack<7, 32>(map, A, units, 1, status, st)
+                 : f32::launch_stack<8, 16>(map, A, units, 1, status, st);
   const cudaError_t fe = cudaFreeAsync(sc.list, st);
   if (rc) return rc;
   CG_CUDA(fe);

@@ -151,7 +151,8 @@ int cg_get_tuning(cg_tuning *out);
  * returns.  The FP32 FFT's column passes wait for their tensor copies under
  * the same limit; a wait that runs out there is counted in a device-wide
  * counter that cg_fft_timeouts reads (after synchronising the device; reset
- * nonzero: set it back to 0), and the transform's output is undefined.  No
+ * nonzero: set it back to 0), in cg_wstack_image and cg_towers_image as
+ * CG_ERR_TIMEOUT in the status block too, and the output is undefined.  No
  * counterpart in the reference: a test hook that makes a wait run out on
  * purpose (a limit of 0 fails every copy not yet landed when it is first
  * polled).  Process-wide. */
