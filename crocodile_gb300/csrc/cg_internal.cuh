@@ -274,6 +274,7 @@ struct cg_plan {
   int subshift; // sub-tile edge = 1 << subshift cells (4, or more for huge grid stacks)
   int64_t max_items;
   int chunk;    // visibilities per work item
+  int chunk_crowded;  // the same for tiles that many such items would make (ItemSize)
   int outer;    // window edge of the separable gridder (grid_outer.cu), 0: another gridder
   int lane_odd; // odd supports on the lane layout's tiles, gridded by the lane kernel
   int lean;     // plan_geometry: the choices that need the least workspace

@@ -293,6 +293,18 @@ __global__ void k_plan_items(int ntiles, int sublog, const int32_t *__restrict__
 // 4096 where two can do it (16384 tiles: 27 us against 10).
 static constexpr int PLAN_SMALL_BUCKETS = 16384, PLAN_SMALL_TILES = 4096;
 
+// Visibilities per item, by the tile's count.  An item's window reaches the grid by
+// one addition per cell, so a crowded tile cut short (32 or 64, where n is small)
+// adds up thousands of windows in 32 bits: 204,800 equal visibilities in one cell, off
+// by 2.4e-5 in items of 64, by 5.3e-6 in items of 512.  Beyond 64 items a tile gets
+// the long ones (its list, which one thread writes, is as much shorter).
+struct ItemSize {
+  int usual, crowded;
+  __device__ __forceinline__ int of(int count) const {
+    return count > 64 * usual ? crowded : usual;
+  }
+};
+
 __device__ __forceinline__ void write_items(int tile, int off, int count, int chunk, int base,
                                             WorkItem *items) {
   for (int j = 0; j * chunk < count; ++j) {
@@ -306,7 +318,7 @@ __device__ __forceinline__ void write_items(int tile, int off, int count, int ch
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_plan_small(
-    int nbuckets, int ntiles, int sublog, const int32_t *__restrict__ counts, int chunk,
+    int nbuckets, int ntiles, int sublog, const int32_t *__restrict__ counts, ItemSize size,
     int32_t *__restrict__ offsets, WorkItem *__restrict__ items, int32_t *__restrict__ nitems) {
   __shared__ int s_warp[33];
   int carry = 0;
@@ -337,7 +349,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_plan_small(
       off = offsets[t << (2 * sublog)];
       c = (next < nbuckets ? offsets[next] : n) - off;
     }
-    const int m = (c + chunk - 1) / chunk;
+    const int chunk = size.of(c), m = (c + chunk - 1) / chunk;
     const int at = carry + block_exclusive_scan(m, s_warp, total);
     write_items(t, off, c, chunk, at, items);
     carry += total;
@@ -379,7 +391,7 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned lo
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
-    int nbuckets, const int32_t *__restrict__ counts, int chunk, int32_t *__restrict__ offsets,
+    int nbuckets, const int32_t *__restrict__ counts, ItemSize size, int32_t *__restrict__ offsets,
     int32_t *__restrict__ ioff, unsigned long long *sums, int32_t *done,
     int32_t *__restrict__ nitems) {
   __shared__ unsigned long long s_warp[33];
@@ -389,6 +401,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
 #pragma unroll
   for (int k = 0; k < SCAN_PER_THREAD; ++k) {
     const int c = base + k < nbuckets ? counts[base + k] : 0;
+    const int chunk = size.of(c);
     v[k] = (unsigned long long)c | (unsigned long long)((c + chunk - 1) / chunk) << 32;
     sum += v[k];
   }
@@ -420,7 +433,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
   if (threadIdx.x == 0) *nitems = (int32_t)(carry >> 32);
 }
 
-__global__ void k_plan_finish(int nbuckets, const int32_t *__restrict__ counts, int chunk,
+__global__ void k_plan_finish(int nbuckets, const int32_t *__restrict__ counts, ItemSize size,
                               int32_t *__restrict__ offsets, const int32_t *__restrict__ ioff,
                               const unsigned long long *__restrict__ sums,
                               WorkItem *__restrict__ items) {
@@ -429,7 +442,7 @@ __global__ void k_plan_finish(int nbuckets, const int32_t *__restrict__ counts, 
   const unsigned long long s = sums[t / SCAN_TILE];
   const int off = offsets[t] + (int32_t)s;
   offsets[t] = off;
-  write_items(t, off, counts[t], chunk, ioff[t] + (int32_t)(s >> 32), items);
+  write_items(t, off, counts[t], size.of(counts[t]), ioff[t] + (int32_t)(s >> 32), items);
 }
 
 __global__ void k_frac_coords(const double *uvw, int64_t stride, double lam,
@@ -847,12 +860,13 @@ static void plan_geometry(cg_plan &p) {
     auto clamp = [](int64_t v, int64_t lo, int64_t hi) {
       return (int)(std::min(hi, std::max(lo, v)) & ~(int64_t)31);
     };
+    const int per_cta = (int)std::min<int64_t>(
+        2048, std::max<int64_t>(256, p.n / (int64_t)(num_sms() * 16) + 1));
     p.chunk = t.chunk > 0 ? t.chunk
               : p.outer   ? clamp(per_warp, 32, 256)
-              : lane
-                  ? (p.lean ? 512 : clamp(per_warp, 64, 512))
-                  : (int)std::min<int64_t>(
-                        2048, std::max<int64_t>(256, p.n / (int64_t)(num_sms() * 16) + 1));
+              : lane      ? (p.lean ? 512 : clamp(per_warp, 64, 512))
+                          : per_cta;
+    p.chunk_crowded = t.chunk > 0 ? t.chunk : lane ? 512 : per_cta;
     p.max_items = (p.n + p.chunk - 1) / p.chunk + p.ntiles;
     // The lane gridder streams each visibility's S x S slice with one bulk copy,
     // which needs a multiple of 16 bytes: for odd S * S it reads a copy of the
@@ -873,7 +887,7 @@ static void plan_geometry(cg_plan &p) {
     p.tpl = 1;
     p.nbuckets = p.gper * p.layers;
     p.win = p.pitch = 0;
-    p.chunk = 0;
+    p.chunk = p.chunk_crowded = 0;
     p.max_items = 0;
     p.slice_stride = p.kd.sep ? p.kd.S : p.kd.S * p.kd.S;
     p.kpad_slices = 0;
@@ -1013,18 +1027,19 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   // 1000 visibilities on 256^2 took eight launches, one on 1531^2 eleven; now four
   // and five (conv_imaging + conv_predict there: 286 -> 266 us, 370 -> 340 us).
   const bool tiled = mode == CG_PLAN_TILED;
+  const ItemSize size = {p->chunk, p->chunk_crowded};
   const int scan_blocks = (p->nbuckets + SCAN_TILE - 1) / SCAN_TILE;
   if (tiled && p->nbuckets <= (p->sublog ? PLAN_SMALL_BUCKETS : PLAN_SMALL_TILES)) {
-    k_plan_small<<<1, SCAN_THREADS, 0, s>>>(p->nbuckets, p->ntiles, p->sublog, p->counts, p->chunk,
+    k_plan_small<<<1, SCAN_THREADS, 0, s>>>(p->nbuckets, p->ntiles, p->sublog, p->counts, size,
                                             p->offsets, p->items, p->nitems);
     CG_LAUNCH("plan offsets and items");
   } else if (tiled && p->sublog == 0) {
     unsigned long long *sums = (unsigned long long *)(ws + L.scan);
     int32_t *tioff = (int32_t *)(ws + L.tioff);
-    k_plan_scan<<<scan_blocks, SCAN_THREADS, 0, s>>>(p->nbuckets, p->counts, p->chunk, p->offsets,
+    k_plan_scan<<<scan_blocks, SCAN_THREADS, 0, s>>>(p->nbuckets, p->counts, size, p->offsets,
                                                      tioff, sums, ctr + 3, p->nitems);
     CG_LAUNCH("plan scan");
-    k_plan_finish<<<(p->nbuckets + 255) / 256, 256, 0, s>>>(p->nbuckets, p->counts, p->chunk,
+    k_plan_finish<<<(p->nbuckets + 255) / 256, 256, 0, s>>>(p->nbuckets, p->counts, size,
                                                             p->offsets, tioff, sums, p->items);
     CG_LAUNCH("plan items");
   } else {
