@@ -859,25 +859,15 @@ __global__ void k_w_phase(int N, double theta, float2 *__restrict__ ph, int32_t 
 }
 
 // exp(2 pi i w ph).  The turns are a double-float product, reduced to a fraction of
-// a turn and then to an eighth on either side of a quarter turn, g.  There sin(2
-// pi g) / g and cos(2 pi g) are their best polynomials in g^2 (Remez exchange; off
-// by 3e-9 and 1e-10 before rounding), and the quarter's number, in the low bits of
-// the rounding sum, swaps them and sets the signs.  All errors together stay
-// below 1.2e-7 (8.6e-8 over 2M arguments of one turn; sincospif, made for any
-// argument, took 3 % more of a whole w-stacking or w-towers call).
+// a turn before the FP32 sincospi, as in the passes that form the sums by
+// themselves (k_wstack_combine, k_towers_combine), bit for bit.  (Short polynomials on
+// an eighth of a turn took 3 % less of a w-stacking or w-towers call, but are off by
+// up to 8.5e-8, 2.7e-8 rms, where sincospi is by 2.1e-8 rms.)
 __device__ __forceinline__ void w_factor(float wh, float wl, float2 ph, float &cs, float &sn) {
   const float hi = wh * ph.x;
-  const float lo = fmaf(wl, ph.x, fmaf(wh, ph.y, fmaf(wh, ph.x, -hi)));
+  const float lo = fmaf(wh, ph.x, -hi) + fmaf(wh, ph.y, wl * ph.x);
   const float f = (hi - rintf(hi)) + lo;
-  const float t = fmaf(4.f, f, 12582912.f);  // 1.5 x 2^23: rounds to whole quarters
-  const float g = fmaf(-0.25f, t - 12582912.f, f), z = g * g;
-  const float s = g * fmaf(fmaf(fmaf(-75.4020680f, z, 81.5925536f), z, -41.3416626f), z, 6.28318529f);
-  const float c =
-      fmaf(fmaf(fmaf(fmaf(59.2867640f, z, -85.4450344f), z, 64.9393391f), z, -19.7392087f), z, 1.f);
-  const unsigned q = __float_as_uint(t);
-  const bool odd = q & 1;
-  sn = __uint_as_float(__float_as_uint(odd ? c : s) ^ ((q << 30) & 0x80000000u));
-  cs = __uint_as_float(__float_as_uint(odd ? s : c) ^ (((q + 1) << 30) & 0x80000000u));
+  sincospif(2.0f * f, &sn, &cs);
 }
 
 // The quadrant's row or column of index i of a centred (or, rolled, of an
