@@ -296,12 +296,14 @@ static constexpr int PLAN_SMALL_BUCKETS = 16384, PLAN_SMALL_TILES = 4096;
 // Visibilities per item, by the tile's count.  An item's window reaches the grid by
 // one addition per cell, so a crowded tile cut short (32 or 64, where n is small)
 // adds up thousands of windows in 32 bits: 204,800 equal visibilities in one cell, off
-// by 2.4e-5 in items of 64, by 5.3e-6 in items of 512.  Beyond 64 items a tile gets
-// the long ones (its list, which one thread writes, is as much shorter).
+// by 2.4e-5 in items of 64, by 5.3e-6 in items of 512.  So a tile makes at most 128
+// items until they are that long (and its list, which one thread writes, is as much
+// shorter).  (The longest for all of a crowded tile: S 16, 200k on 512^2, density 1 / r,
+// 7,800 in the central tile: 146 us, 71 so, 69 in items of 64.)
 struct ItemSize {
   int usual, crowded;
   __device__ __forceinline__ int of(int count) const {
-    return count > 64 * usual ? crowded : usual;
+    return max(usual, min(crowded, (count / 128 + 31) & ~31));
   }
 };
 
