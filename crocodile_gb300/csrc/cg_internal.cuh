@@ -278,6 +278,7 @@ struct cg_plan {
   int outer;    // window edge of the separable gridder (grid_outer.cu), 0: another gridder
   int lane_odd; // odd supports on the lane layout's tiles, gridded by the lane kernel
   int lean;     // plan_geometry: the choices that need the least workspace
+  int direct;   // few visibilities: the direct gridder unless a cell is crowded
   int slice_stride;  // lane layout: elements between S x S slices of the table it reads
   int64_t kpad_slices;  // lane layout, slices padded to a 16-byte multiple: slices to copy
   // device arrays inside the caller's workspace
@@ -289,6 +290,7 @@ struct cg_plan {
   float2 *kpad;       // lane layout, odd S * S: the table with padded slices (workspace)
   int32_t *nitems;    // device counter
   int32_t *ticket;    // device counter for the persistent kernels (2 words)
+  int32_t *split;     // device: number of items for the direct gridder, for the others
   int32_t *status;    // caller's status block
   // group mode: host copies of group ranges
   int32_t *h_offsets;
@@ -311,13 +313,20 @@ inline SortedEnd sorted_end(const cg_plan *p) {
 
 // Few enough visibilities to add their taps one by one to the grid in memory
 // (k_grid_direct): the sum in a cell rounds with each, so its error grows with the
-// root of the number of its taps, where the other gridders sum a tile's share
-// first.  Baselines are dense at the centre, where a density of 1 / r puts 1.3 n S /
-// H taps into a cell.  Against FP64, direct / others: 1.2e-7 / 1.2e-7 of the norm at n
-// S / H 200, 1.6e-7 .. 3.3e-7 / 1e-7 at 730, 9e-7 / 1.5e-7 at 7100.
+// number of its taps (with its root where they differ), where the other gridders sum
+// a tile's share first.  Baselines are dense at the centre, where a density of 1 / r
+// puts 1.3 n S / H taps into a cell.  Against FP64, direct / others: 1.2e-7 / 1.2e-7
+// of the norm at n S / H 200, 1.6e-7 .. 3.3e-7 / 1e-7 at 730, 9e-7 / 1.5e-7 at 7100.
 inline bool direct_fits(const cg_plan &p) {
   return p.kd.S <= 16 && (double)p.n * p.kd.S <= 200.0 * (double)(p.H < p.W ? p.H : p.W);
 }
+
+// That is the host's guess; the plan's counts decide on the device (plan.cu, crowded):
+// where a cell could get more than this many taps, another gridder takes the call.
+// Equal terms are the worst case (a PSF on equal coordinates): 512 in sequence, the
+// most that the lane gridder sums in a window, are off by 3.7e-6, 25,600 by 1.9e-4 and
+// 204,800 by 1.6e-3.
+constexpr int DIRECT_CELL_TAPS = 512;
 int launch_scan(const int32_t *in, int32_t *out, int n, int32_t *scratch,
                 cudaStream_t s);
 size_t scan_scratch_words(int n);

@@ -612,13 +612,14 @@ template <class F>
 __device__ __forceinline__ void direct_batches(const DirectArgs &D, F f) {
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int nitems = *D.A.nitems;
+  if (nitems == 0) return;  // no visibility, or the call is another gridder's
   if (!D.layered) {
     const int64_t n = D.end();
     for (int64_t b = gw * 32; b < n; b += nw * 32)
       f((int)b, (int)min((int64_t)32, n - b), (size_t)0);
     return;
   }
-  const int nitems = *D.A.nitems;
   for (int64_t it = gw; it < nitems; it += nw) {
     const WorkItem w = D.A.items[it];
     const size_t off = (size_t)(w.tile / D.A.tpl) * D.A.H * D.A.W;
@@ -796,12 +797,24 @@ static int direct_grid_launch(const cg_plan *p, const float2 *ktab, const float2
   return direct_launch(p, fn, args, s);
 }
 
-// Whether a call takes the direct gridder by itself.  A wait limit of 0 keeps to the
-// lane kernel (lane_launch) where that would run.
+// Whether a call takes the direct gridder by itself, unless a cell is crowded
+// (DIRECT_CELL_TAPS).  A wait limit of 0 keeps to the lane kernel (lane_launch) where that
+// would run.
 static bool direct_wanted(const cg_plan *p, bool lane) {
   const cg_tuning t = tuning();
-  return t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0 && direct_fits(*p) &&
+  return p->direct && t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0 &&
          !(lane && wait_cycles() == 0);
+}
+
+// The plan as seen by the direct gridder (crowded = false) and by the windowed one
+// launched beside it: one of them finds the work list empty (4 us, 6 with the lane
+// kernel; 100k visibilities on 4096^2, S 8, separable: 33 -> 35 us at a density of 1 /
+// r, and 164 -> 49 all in one cell, whose atomics queue).  With no more visibilities
+// than a cell may have taps the direct one runs alone.
+static cg_plan split_plan(const cg_plan *p, bool crowded) {
+  cg_plan q = *p;
+  q.nitems = p->split + (crowded ? 1 : 0);
+  return q;
 }
 
 static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
@@ -824,14 +837,21 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   void *args[12];
   int gsize = 0, ngroups = 0;
   bool shared = false;
-  if (p->outer) return outer_launch(p, kt, vv, nullptr, weight, mode, gg, s);
   const bool lane = layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0);
   // Taps straight into the grid while visibilities are few (direct_fits: accuracy
   // sets the line, and below it this is the fastest too, direct / lane / warp
   // gridder, us: S 8, 30k on 512^2: 11 / 24 / 23; S 16: 22 / 32 / 53; 60k on 4096^2, S 8:
   // 13 / 56 / 53).
-  if (direct_wanted(p, lane))
-    return direct_grid_launch(p, kt, vv, nullptr, weight, mode, gg, s);
+  cg_plan q;
+  if (direct_wanted(p, lane)) {
+    q = split_plan(p, false);
+    const int rc = direct_grid_launch(&q, kt, vv, nullptr, weight, mode, gg, s);
+    if (rc || p->n <= DIRECT_CELL_TAPS) return rc;
+    q = split_plan(p, true);
+    p = &q;
+    A.nitems = q.nitems;
+  }
+  if (p->outer) return outer_launch(p, kt, vv, nullptr, weight, mode, gg, s);
   if (lane) return lane_launch(p, kt, vv, weight, mode, gg, nullptr, nullptr, 0, false, s);
   if (layout_for(p->kd) != CG_LAYOUT_OWNER) {
     const int need = (S * S + 31) / 32;
@@ -878,6 +898,45 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   CG_REQUIRE(per_sm > 0, "gridder does not fit on an SM (smem %zu)", smem);
   int64_t blocks = std::min<int64_t>((int64_t)per_sm * num_sms(), p->max_items);
   CG_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int32_t), s));
+  CG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, smem, s));
+  return CG_OK;
+}
+
+// vis_out = degrid(grid_in), grid_out += grid(vis_in, or vis_in - vis_out when
+// residual), in one traversal.
+static int fused_launch(const cg_plan *p, const void *ktab, const void *grid_in, const void *vis_in,
+                        int residual, void *vis_out, void *grid_out, bool lane, cudaStream_t s) {
+  const int S = p->kd.S;
+  const cg_tuning t = tuning();
+  if (lane)
+    return lane_launch(p, (const float2 *)ktab, (const float2 *)vis_in, nullptr, 0,
+                       (float2 *)grid_out, (const float2 *)grid_in, (float2 *)vis_out, residual,
+                       true, s);
+  TiledArgs A = tiled_args(p);
+  const int need = (S * S + 31) / 32;
+  int maxt = 1;
+  while (maxt < need) maxt *= 2;
+  void *fn = nullptr;
+#define PICK(M)                                                                      \
+  if (maxt == M) fn = p->kd.sep ? (void *)k_degrid_grid_warp<true, M>                 \
+                                : (void *)k_degrid_grid_warp<false, M>;
+  PICK(1) PICK(2) PICK(4) PICK(8) PICK(16) PICK(32)
+#undef PICK
+  CG_REQUIRE(fn, "no fused kernel for support %d", S);
+  const int threads = 32 * (t.groups > 0 ? std::min(t.groups, 8) : 8);
+  const size_t smem = 2 * (size_t)p->pitch * p->win * sizeof(float2) +
+                      (size_t)GRID_STAGE * (4 + 4 + 8 + 8 + 8);
+  CG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+  CG_REQUIRE(per_sm > 0, "fused kernel does not fit on an SM (smem %zu)", smem);
+  int64_t blocks = std::min<int64_t>((int64_t)per_sm * num_sms(), p->max_items);
+  CG_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int32_t), s));
+  int mode = residual ? 1 : 0;
+  const float2 *kt = (const float2 *)ktab, *gi = (const float2 *)grid_in,
+               *vi = (const float2 *)vis_in;
+  float2 *vo = (float2 *)vis_out, *go = (float2 *)grid_out;
+  void *args[] = {&A, &mode, &kt, &gi, &vi, &vo, &go};
   CG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, smem, s));
   return CG_OK;
 }
@@ -995,9 +1054,8 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
   CG_REQUIRE(vis_in || !residual, "the residual mode needs input visibilities");
   CG_REQUIRE(grid_in != grid_out, "input and output grids must differ");
   cudaStream_t s = (cudaStream_t)stream;
-  const int S = p->kd.S;
-  const cg_tuning t = tuning();
-  const bool lane = layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && t.layout == 0);
+  const bool lane =
+      layout_for(p->kd) == CG_LAYOUT_LANE || (p->lane_odd && tuning().layout == 0);
   // Degrid, then grid, by the kernels that do each best: few visibilities (a tile's
   // windows of both grids cost more than they hold; 60k on 4096^2, S 8, separable:
   // 173 us in one traversal, 22 so), and separable tables on the register-window
@@ -1008,46 +1066,28 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
   const size_t vbytes = (size_t)p->n * sizeof(float2);
   const bool apart = !vis_in || !vis_out || vi0 + vbytes <= vo0 || vo0 + vbytes <= vi0;
   if ((p->outer || direct) && apart && (vis_out || !residual)) {
+    const float2 *kt = (const float2 *)ktab, *vi = (const float2 *)vis_in;
+    const int mode = residual ? 3 : 0;
+    float2 *go = (float2 *)grid_out, *vo = (float2 *)vis_out;
+    const bool beside = direct && vis_in && p->n > DIRECT_CELL_TAPS;
+    cg_plan q = split_plan(p, true);  // a crowded cell: one traversal where no better
+    if (beside && !p->outer) {
+      const int rc = fused_launch(&q, ktab, grid_in, vis_in, residual, vis_out, grid_out, lane, s);
+      if (rc) return rc;
+    }
     if (vis_out) {
       const int rc = cg_degrid(p, ktab, grid_in, vis_out, stream);
       if (rc) return rc;
     }
     if (!vis_in) return CG_OK;
-    const auto launch = p->outer ? outer_launch : direct_grid_launch;
-    return launch(p, (const float2 *)ktab, (const float2 *)vis_in, (const float2 *)vis_out,
-                  nullptr, residual ? 3 : 0, (float2 *)grid_out, s);
+    if (p->outer && (beside || !direct)) {
+      const int rc = outer_launch(direct ? &q : p, kt, vi, vo, nullptr, mode, go, s);
+      if (rc || !direct) return rc;
+    }
+    q = split_plan(p, false);
+    return direct_grid_launch(&q, kt, vi, vo, nullptr, mode, go, s);
   }
-  if (lane)
-    return lane_launch(p, (const float2 *)ktab, (const float2 *)vis_in, nullptr, 0,
-                       (float2 *)grid_out, (const float2 *)grid_in, (float2 *)vis_out, residual,
-                       true, s);
-  TiledArgs A = tiled_args(p);
-  const int need = (S * S + 31) / 32;
-  int maxt = 1;
-  while (maxt < need) maxt *= 2;
-  void *fn = nullptr;
-#define PICK(M)                                                                      \
-  if (maxt == M) fn = p->kd.sep ? (void *)k_degrid_grid_warp<true, M>                 \
-                                : (void *)k_degrid_grid_warp<false, M>;
-  PICK(1) PICK(2) PICK(4) PICK(8) PICK(16) PICK(32)
-#undef PICK
-  CG_REQUIRE(fn, "no fused kernel for support %d", S);
-  const int threads = 32 * (t.groups > 0 ? std::min(t.groups, 8) : 8);
-  const size_t smem = 2 * (size_t)p->pitch * p->win * sizeof(float2) +
-                      (size_t)GRID_STAGE * (4 + 4 + 8 + 8 + 8);
-  CG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
-  CG_REQUIRE(per_sm > 0, "fused kernel does not fit on an SM (smem %zu)", smem);
-  int64_t blocks = std::min<int64_t>((int64_t)per_sm * num_sms(), p->max_items);
-  CG_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int32_t), s));
-  int mode = residual ? 1 : 0;
-  const float2 *kt = (const float2 *)ktab, *gi = (const float2 *)grid_in,
-               *vi = (const float2 *)vis_in;
-  float2 *vo = (float2 *)vis_out, *go = (float2 *)grid_out;
-  void *args[] = {&A, &mode, &kt, &gi, &vi, &vo, &go};
-  CG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, smem, s));
-  return CG_OK;
+  return fused_launch(p, ktab, grid_in, vis_in, residual, vis_out, grid_out, lane, s);
 }
 
 }  // extern "C"

@@ -319,11 +319,64 @@ __device__ __forceinline__ void write_items(int tile, int off, int count, int ch
   }
 }
 
+// Whether a cell could get more than DIRECT_CELL_TAPS taps.  Taps reach it from the
+// visibilities of `reach` tiles to an axis, so no cell does unless the tiles of
+// some reach x reach block hold that many, and then one of them holds `few`
+// (INT32_MAX: a plan that is not for the direct gridder).
+struct Crowd {
+  int few, reach, tblog, nbx, ntx, nty, tpl;
+  template <int R>
+  __device__ __forceinline__ bool blocks(const int32_t *c, int tx, int ty) const {
+    constexpr int M = 2 * R - 1;
+    int v[M][M];
+#pragma unroll
+    for (int y = 0; y < M; ++y)
+#pragma unroll
+      for (int x = 0; x < M; ++x) {  // loads in flight together
+        const int px = tx - R + 1 + x, py = ty - R + 1 + y;
+        v[y][x] = (unsigned)px < (unsigned)ntx && (unsigned)py < (unsigned)nty
+                      ? __ldg(&c[tile_index(px, py, tblog, nbx)])
+                      : 0;
+      }
+    bool over = false;
+#pragma unroll
+    for (int y = 0; y < R; ++y)
+#pragma unroll
+      for (int x = 0; x < R; ++x) {
+        int sum = 0;
+#pragma unroll
+        for (int k = 0; k < R * R; ++k) sum += v[y + k / R][x + k % R];
+        over = over || sum > DIRECT_CELL_TAPS;
+      }
+    return over;
+  }
+  // a tile of `few` or more
+  __device__ bool around(const int32_t *counts, int tile) const {
+    const int lyr = tile / tpl;
+    int tx, ty;
+    tile_xy(tile - lyr * tpl, tblog, nbx, tx, ty);
+    const int32_t *c = counts + (int64_t)lyr * tpl;
+    return reach == 1   ? blocks<1>(c, tx, ty)
+           : reach == 2 ? blocks<2>(c, tx, ty)
+           : reach == 3 ? blocks<3>(c, tx, ty)
+                        : true;  // (requested tiles of 4 and 8 cells)
+  }
+};
+
+// Where the direct gridder could run, the work list goes to it or, when a cell is
+// crowded, to the windowed one that is launched beside it; the other finds none.
+__device__ __forceinline__ void split_items(int nitems, bool crowded, int32_t *split) {
+  split[0] = crowded ? 0 : nitems;
+  split[1] = crowded ? nitems : 0;
+}
+
 __global__ void __launch_bounds__(SCAN_THREADS) k_plan_small(
     int nbuckets, int ntiles, int sublog, const int32_t *__restrict__ counts, ItemSize size,
-    int32_t *__restrict__ offsets, WorkItem *__restrict__ items, int32_t *__restrict__ nitems) {
+    Crowd crowd, int32_t *__restrict__ offsets, WorkItem *__restrict__ items,
+    int32_t *__restrict__ nitems, int32_t *__restrict__ split) {
   __shared__ int s_warp[33];
   int carry = 0;
+  bool over = false;
   for (int b0 = 0; b0 < nbuckets; b0 += SCAN_TILE) {
     const int base = b0 + threadIdx.x * SCAN_PER_THREAD;
     int v[SCAN_PER_THREAD], sum = 0, total;
@@ -351,12 +404,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_plan_small(
       off = offsets[t << (2 * sublog)];
       c = (next < nbuckets ? offsets[next] : n) - off;
     }
+    if (c >= crowd.few) over = over || crowd.around(counts, t);
     const int chunk = size.of(c), m = (c + chunk - 1) / chunk;
     const int at = carry + block_exclusive_scan(m, s_warp, total);
     write_items(t, off, c, chunk, at, items);
     carry += total;
   }
-  if (threadIdx.x == 0) *nitems = carry;
+  const bool crowded = __syncthreads_or(over);
+  if (threadIdx.x == 0) {
+    *nitems = carry;
+    split_items(carry, crowded, split);
+  }
 }
 
 // Larger grids whose buckets are tiles: both scans as one (counts in the lower
@@ -393,16 +451,18 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned lo
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
-    int nbuckets, const int32_t *__restrict__ counts, ItemSize size, int32_t *__restrict__ offsets,
-    int32_t *__restrict__ ioff, unsigned long long *sums, int32_t *done,
-    int32_t *__restrict__ nitems) {
+    int nbuckets, const int32_t *__restrict__ counts, ItemSize size, Crowd crowd,
+    int32_t *__restrict__ offsets, int32_t *__restrict__ ioff, unsigned long long *sums,
+    int32_t *done, int32_t *crowded, int32_t *__restrict__ nitems, int32_t *__restrict__ split) {
   __shared__ unsigned long long s_warp[33];
   __shared__ bool s_last;
   const int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
   unsigned long long v[SCAN_PER_THREAD], sum = 0, total;
+  bool over = false;
 #pragma unroll
   for (int k = 0; k < SCAN_PER_THREAD; ++k) {
     const int c = base + k < nbuckets ? counts[base + k] : 0;
+    if (c >= crowd.few) over = over || crowd.around(counts, base + k);
     const int chunk = size.of(c);
     v[k] = (unsigned long long)c | (unsigned long long)((c + chunk - 1) / chunk) << 32;
     sum += v[k];
@@ -416,8 +476,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
     }
     run += v[k];
   }
+  over = __syncthreads_or(over);
   if (threadIdx.x == 0) {
     sums[blockIdx.x] = total;
+    if (over) atomicOr(crowded, 1);
     __threadfence();
     s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
   }
@@ -432,7 +494,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_plan_scan(
     if (b < (int)gridDim.x) sums[b] = e;
     carry += total;
   }
-  if (threadIdx.x == 0) *nitems = (int32_t)(carry >> 32);
+  if (threadIdx.x == 0) {
+    *nitems = (int32_t)(carry >> 32);
+    split_items((int32_t)(carry >> 32), __ldcg(crowded) != 0, split);
+  }
 }
 
 __global__ void k_plan_finish(int nbuckets, const int32_t *__restrict__ counts, ItemSize size,
@@ -775,8 +840,7 @@ static int tile_edge(const cg_kernel_desc &kd, int req) {
 
 // Window edge of the register-window gridder for separable tables
 // (grid_outer.cu) and its tile edge T (window >= T + S - 1), or 0 where another
-// gridder runs: the direct one for few visibilities (direct_fits), the one with
-// shared-memory tiles for the narrowest supports unless visibilities are dense
+// gridder runs: the one with shared-memory tiles for the narrowest supports unless visibilities are dense
 // (its time goes with S, the window's flush does not; plan and grid, warp gridder
 // / this one, us: S 3, 1M on 2048^2: 153 / 181, S 5: 174 / 179, on 4096^2: 200 / 183,
 // S 6: 210 / 172, S 8: 239 / 170, on 4096^2: 259 / 218).  Stacks of grids, requested
@@ -788,11 +852,13 @@ static int outer_edge(const cg_plan &p, int &T) {
       t.layout > 0 || (int64_t)p.kd.G * p.kd.Q * S >= INT32_MAX)
     return 0;
   const double rho = (double)p.n / ((double)p.H * (double)p.W);
-  if (direct_fits(p) || (S <= 4 && rho < 1.5)) return 0;
+  const bool few = direct_fits(p);
+  if (!few && S <= 4 && rho < 1.5) return 0;
+  // few visibilities: small tiles, whose counts bound a cell's taps more closely;
   // larger tiles where they fit the window and are not full: fewer flushes, but
   // more visibilities to a counter of the plan (S 5, 1M on 1024^2: plan 117 us with
   // tiles of 12, 74 with 8, gridder 99 with either)
-  T = rho < 0.25 && (S <= 5 || (S >= 10 && S <= 13)) ? 12 : 8;
+  T = rho < 0.25 && ((S <= 5 && !few) || (S >= 10 && S <= 13)) ? 12 : 8;
   return S <= 9 ? 16 : 24;
 }
 
@@ -807,8 +873,9 @@ static bool lane_odd(const cg_plan &p) {
   const int S = p.kd.S;
   const int64_t tiles = (int64_t)((p.W + 15) / 16) * ((p.H + 15) / 16) * p.layers;
   const double cells = (double)p.H * (double)p.W * (double)p.layers;
-  return !p.lean && !p.kd.sep && S >= 9 && S <= 16 && S % 2 == 1 && p.tile_req == 0 &&
-         t.tile == 0 && t.layout == 0 && tiles <= (1 << 24) && (double)p.n >= 0.04 * cells &&
+  const bool few = p.layers == 1 && direct_fits(p);  // beside the direct gridder: any
+  return !p.lean && !p.kd.sep && S <= 16 && S % 2 == 1 && p.tile_req == 0 && t.tile == 0 &&
+         t.layout == 0 && tiles <= (1 << 24) && (few || (S >= 9 && (double)p.n >= 0.04 * cells)) &&
          (int64_t)p.kd.G * p.kd.Q * p.kd.Q < INT32_MAX;
 }
 
@@ -819,10 +886,16 @@ static void plan_geometry(cg_plan &p) {
     p.lane_odd = lane_odd(p);
     const bool lane = p.lane_odd || layout_for(p.kd) == CG_LAYOUT_LANE;
     const cg_tuning t = tuning();
+    // few visibilities: one grid's small tiles are the register-window gridder's or
+    // the lane kernel's, which take the call where a cell is crowded
+    p.direct = !p.lean && t.layout == 0 && t.tile == 0 && direct_fits(p) &&
+               (p.layers > 1 || p.tile_req > 0 || p.outer || lane);
     // no order inside a tile (for few visibilities it is not worth its buckets)
-    const bool flat =
-        p.outer || lane || (!p.lean && t.layout == 0 && t.tile == 0 && direct_fits(p));
+    const bool flat = p.outer || lane || p.direct;
     p.T = p.outer ? outer_T : p.lane_odd ? 16 : tile_edge(p.kd, p.tile_req);
+    // few visibilities, 4-D: tiles as small as lets a cell see two to an axis
+    if (p.direct && !p.outer && p.layers == 1 && p.tile_req == 0)
+      p.T = p.kd.S <= 9 ? 8 : p.kd.S <= 13 ? 12 : 16;
     p.ntx = (p.W + p.T - 1) / p.T;
     p.nty = (p.H + p.T - 1) / p.T;
     // Morton blocks of up to 32 x 32 tiles (no larger than the grid needs)
@@ -905,7 +978,7 @@ static Layout layout_of(const cg_plan &p) {
   L.rank = o;    o = align256(o + n * 4);
   L.recs = o;    o = align256(o + n * sizeof(VisRec));
   L.perm = o;    o = align256(o + n * 4);
-  L.ctr = o;     o = align256(o + 4 * 4);  // before the counts: zeroed with them
+  L.ctr = o;     o = align256(o + 8 * 4);  // before the counts: zeroed with them
   L.counts = o;  o = align256(o + (size_t)p.nbuckets * 4);
   L.offsets = o; o = align256(o + (size_t)p.nbuckets * 4);
   L.scan = o;    o = align256(o + scan_scratch_words(p.nbuckets) * 4);
@@ -982,6 +1055,7 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   int32_t *ctr = (int32_t *)(ws + L.ctr);
   p->nitems = ctr;
   p->ticket = ctr + 1;
+  p->split = ctr + 4;
   p->status = d_status;
   // everything later kernels accumulate into starts at zero on every call
   CG_CUDA(cudaMemsetAsync(ctr, 0, (char *)(p->counts + p->nbuckets) - (char *)ctr, s));
@@ -1030,16 +1104,20 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   // and five (conv_imaging + conv_predict there: 286 -> 266 us, 370 -> 340 us).
   const bool tiled = mode == CG_PLAN_TILED;
   const ItemSize size = {p->chunk, p->chunk_crowded};
+  const int reach = kd->S > 1 && p->T > 0 ? (kd->S - 2) / p->T + 2 : 1;
+  const Crowd crowd = {p->direct ? std::max(1, DIRECT_CELL_TAPS / (reach * reach)) : INT32_MAX,
+                       reach, p->tblog, p->nbx, p->ntx, p->nty, p->tpl};
   const int scan_blocks = (p->nbuckets + SCAN_TILE - 1) / SCAN_TILE;
   if (tiled && p->nbuckets <= (p->sublog ? PLAN_SMALL_BUCKETS : PLAN_SMALL_TILES)) {
     k_plan_small<<<1, SCAN_THREADS, 0, s>>>(p->nbuckets, p->ntiles, p->sublog, p->counts, size,
-                                            p->offsets, p->items, p->nitems);
+                                            crowd, p->offsets, p->items, p->nitems, p->split);
     CG_LAUNCH("plan offsets and items");
   } else if (tiled && p->sublog == 0) {
     unsigned long long *sums = (unsigned long long *)(ws + L.scan);
     int32_t *tioff = (int32_t *)(ws + L.tioff);
-    k_plan_scan<<<scan_blocks, SCAN_THREADS, 0, s>>>(p->nbuckets, p->counts, size, p->offsets,
-                                                     tioff, sums, ctr + 3, p->nitems);
+    k_plan_scan<<<scan_blocks, SCAN_THREADS, 0, s>>>(p->nbuckets, p->counts, size, crowd,
+                                                     p->offsets, tioff, sums, ctr + 3, ctr + 6,
+                                                     p->nitems, p->split);
     CG_LAUNCH("plan scan");
     k_plan_finish<<<(p->nbuckets + 255) / 256, 256, 0, s>>>(p->nbuckets, p->counts, size,
                                                             p->offsets, tioff, sums, p->items);

@@ -76,3 +76,18 @@ def test_windowed(env, N, n, S, sep, where):
     """Calls of the windowed gridders (n S > 200 N): plans of one block and of two
     launches, their items short where n is small."""
     _check(env, N, n, S, sep, where)
+
+
+@pytest.mark.parametrize("where", ["cell", "patch", "tile"])
+@pytest.mark.parametrize("S,sep", [(3, True), (8, True), (16, True), (1, False), (7, False), (8, False),
+                                   (9, False), (16, False)])
+@pytest.mark.parametrize("N,per", [(1024, 200), (1024, 30), (300, 200)])
+def test_few_visibilities(env, N, per, S, sep, where):
+    """n S = per N: calls whose number of visibilities alone would send their taps
+    one by one to the grid."""
+    _check(env, N, per * N // S, S, sep, where)
+
+
+@pytest.mark.parametrize("S,sep", [(8, True), (8, False)])
+def test_few_on_a_large_grid(env, S, sep):
+    _check(env, 8192, 204800, S, sep, "cell")
