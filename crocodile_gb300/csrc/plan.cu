@@ -838,6 +838,12 @@ static int tile_edge(const cg_kernel_desc &kd, int req) {
   return 64;
 }
 
+// Most buckets of a plan, which are zeroed and scanned on each call
+static constexpr int64_t MAX_BUCKETS = 1 << 24;
+static int64_t tiles_of(const cg_plan &p, int T) {
+  return (int64_t)((p.W + T - 1) / T) * ((p.H + T - 1) / T) * p.layers;
+}
+
 // Window edge of the register-window gridder for separable tables
 // (grid_outer.cu) and its tile edge T (window >= T + S - 1), or 0 where another
 // gridder runs: the one with shared-memory tiles for the narrowest supports unless visibilities are dense
@@ -859,6 +865,11 @@ static int outer_edge(const cg_plan &p, int &T) {
   // more visibilities to a counter of the plan (S 5, 1M on 1024^2: plan 117 us with
   // tiles of 12, 74 with 8, gridder 99 with either)
   T = rho < 0.25 && ((S <= 5 && !few) || (S >= 10 && S <= 13)) ? 12 : 8;
+  // as many tiles as plans may have buckets: beyond (a side of 32768 with tiles of 8)
+  // the lists would be gigabytes.  Within, this gridder leads however sparse (plan and
+  // grid, us, warp / this one: S 8 on 32768^2, 0.9M 2494 / 774, 9M 6157 / 4329; S 16,
+  // 0.45M, one visibility to ten tiles, 2813 / 768)
+  if (tiles_of(p, T) > MAX_BUCKETS) return 0;
   return S <= 9 ? 16 : 24;
 }
 
@@ -871,11 +882,10 @@ static int outer_edge(const cg_plan &p, int &T) {
 static bool lane_odd(const cg_plan &p) {
   const cg_tuning t = tuning();
   const int S = p.kd.S;
-  const int64_t tiles = (int64_t)((p.W + 15) / 16) * ((p.H + 15) / 16) * p.layers;
   const double cells = (double)p.H * (double)p.W * (double)p.layers;
   const bool few = p.layers == 1 && direct_fits(p);  // beside the direct gridder: any
   return !p.lean && !p.kd.sep && S <= 16 && S % 2 == 1 && p.tile_req == 0 && t.tile == 0 &&
-         t.layout == 0 && tiles <= (1 << 24) && (few || (S >= 9 && (double)p.n >= 0.04 * cells)) &&
+         t.layout == 0 && tiles_of(p, 16) <= MAX_BUCKETS && (few || (S >= 9 && (double)p.n >= 0.04 * cells)) &&
          (int64_t)p.kd.G * p.kd.Q * p.kd.Q < INT32_MAX;
 }
 
@@ -894,8 +904,10 @@ static void plan_geometry(cg_plan &p) {
     const bool flat = p.outer || lane || p.direct;
     p.T = p.outer ? outer_T : p.lane_odd ? 16 : tile_edge(p.kd, p.tile_req);
     // few visibilities, 4-D: tiles as small as lets a cell see two to an axis
-    if (p.direct && !p.outer && p.layers == 1 && p.tile_req == 0)
-      p.T = p.kd.S <= 9 ? 8 : p.kd.S <= 13 ? 12 : 16;
+    if (p.direct && !p.outer && p.layers == 1 && p.tile_req == 0) {
+      const int T = p.kd.S <= 9 ? 8 : p.kd.S <= 13 ? 12 : 16;
+      if (tiles_of(p, T) <= MAX_BUCKETS) p.T = T;
+    }
     p.ntx = (p.W + p.T - 1) / p.T;
     p.nty = (p.H + p.T - 1) / p.T;
     // Morton blocks of up to 32 x 32 tiles (no larger than the grid needs)
@@ -914,7 +926,7 @@ static void plan_geometry(cg_plan &p) {
     p.subshift = 2 + full - p.sublog;
     // keep the histogram (4 B per bucket) within 2^24 buckets: coarser sub-tiles
     // for very large grid stacks
-    while (p.sublog > 0 && ((int64_t)p.ntiles << (2 * p.sublog)) > (1 << 24)) {
+    while (p.sublog > 0 && ((int64_t)p.ntiles << (2 * p.sublog)) > MAX_BUCKETS) {
       --p.sublog;
       ++p.subshift;
     }
