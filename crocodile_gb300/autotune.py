@@ -3,9 +3,10 @@
 Sweeps the grid tile edge, visibilities per work item, row residues per
 gridder thread and thread groups per gridder CTA (``cg_tuning``) on the
 caller's own visibilities, timing plan + grid + degrid with CUDA events, and
-keeps the fastest.  Results are cached in a JSON file keyed by GPU name and a
-workload signature (grid size, support, oversampling, kernel layout and the
-visibility count rounded to a power of two), so later runs start tuned.
+keeps the fastest.  Results are cached in a JSON file keyed by GPU name, the
+tuning's version and a workload signature (grid size, support, oversampling,
+kernel layout and the visibility count rounded to a power of two), so later runs
+start tuned.
 """
 
 import ctypes
@@ -22,6 +23,10 @@ from . import engine as E
 CACHE = os.environ.get("CROCODILE_GB300_TUNING",
                        os.path.join(os.path.expanduser("~"), ".cache", "crocodile_gb300",
                                     "tuning.json"))
+# Part of the cache's keys: raised when a setting's meaning or the automatic choices
+# change, so that entries found best among other kernels are not taken (1: dvis 0 was
+# the tiled degridder, and there was no automatic candidate).
+TUNING_VERSION = 2
 _lock = threading.Lock()
 
 
@@ -58,7 +63,7 @@ def signature(shape, ktab, n):
 
 
 def _key(sig):
-    return "%s|%s" % (torch.cuda.get_device_name(), sig)
+    return "%s|v%d|%s" % (torch.cuda.get_device_name(), TUNING_VERSION, sig)
 
 
 def load_cached(sig):
@@ -85,15 +90,16 @@ def _store(sig, entry):
 
 
 def candidates(S, quick=False):
-    """Launch shapes to try: the automatic choices; the warp layout over tile edge, work-item size and
-    warps per CTA; the owner layout over tile edge, rows per thread and groups;
-    the lane layout (S <= 16) over tile edge, work-item size and degridder."""
+    """Launch shapes to try: the automatic choices; the warp layout over tile edge,
+    work-item size and warps per CTA; the owner layout over tile edge, rows per thread
+    and groups; the lane layout (S <= 16) over tile edge, work-item size and
+    degridder."""
     tiles = [t for t in ((32, 48) if quick else (16, 24, 32, 48, 64)) if t >= min(S, 16)]
     chunks = (0, 1024) if quick else (0, 512, 2048)
     out = [{"tile": 0, "chunk": 0, "rows": 0, "groups": 0, "layout": 0}]  # automatic
     if S <= 16:
-        # the lane layout, each with the tiled degridder (dvis 0) and the ring
-        # degridder (dvis 3)
+        # the lane layout, each with the automatic degridder (dvis 0) and the ring
+        # degridder (dvis 3; the same one for tables beyond 4 GiB)
         for tile, chunk, dvis in itertools.product((16, 32) if quick else (16, 24, 32),
                                                    (512, 1024) if quick else (0, 512, 1024),
                                                    (0, 3)):
