@@ -1126,7 +1126,7 @@ int stack_scratch(int layers, int N, double theta, const double *w, const int32_
 
 template <int LOGL, int C>
 int launch_stack(const CUtensorMap &map, const StackArgs &A, int64_t units, int sign,
-                 int32_t *status, cudaStream_t st) {
+                 long long wait, int32_t *status, cudaStream_t st) {
   using TS = StackShape<LOGL, C>;
   const float2 *tw;
   int rc = twiddles(LOGL, sign, &tw);
@@ -1139,7 +1139,7 @@ int launch_stack(const CUtensorMap &map, const StackArgs &A, int64_t units, int 
   CG_REQUIRE(per_sm > 0, "FP32 FFT stack columns do not fit on an SM (smem %zu)", TS::smem());
   const unsigned grid = (unsigned)std::min<int64_t>(units, (int64_t)num_sms() * per_sm);
   k_fft32_stack<LOGL, C><<<grid, TS::THREADS, TS::smem(), st>>>(map, A, units, tw, sign,
-                                                                wait_cycles(), status);
+                                                                wait, status);
   CG_LAUNCH("FP32 FFT stack columns");
   return CG_OK;
 }
@@ -1322,8 +1322,9 @@ int fft32_wstack(float2 *planes, int layers, int N, double theta, const double *
   f32::StackArgs A{N,      1 << l1, N / 32, 1 << l1, N / 2, false, sc.first, sc.list, sc.ph,
                    image, (int64_t)N * N, (float)(1.0 / ((double)N * N))};
   const int64_t units = (int64_t)A.tiles * A.nj;
-  rc = l2 == 5 ? f32::launch_stack<5, 32>(map, A, units, 1, status, st)
-               : f32::launch_stack<6, 32>(map, A, units, 1, status, st);
+  const long long wait = wait_cycles();
+  rc = l2 == 5 ? f32::launch_stack<5, 32>(map, A, units, 1, wait, status, st)
+               : f32::launch_stack<6, 32>(map, A, units, 1, wait, status, st);
   const cudaError_t fe = cudaFreeAsync(sc.list, st);
   if (rc) return rc;
   CG_CUDA(fe);
@@ -1331,13 +1332,14 @@ int fft32_wstack(float2 *planes, int layers, int N, double theta, const double *
 }
 
 // The raw inverse transforms of a stack of S x S layers and their sums by chunk,
-// as cg_towers_combine forms them.  Sides 64 to 256 (a tile's rows fit a copy box);
-// a wait limit of 0 keeps to the passes that wait for nothing.
+// as cg_towers_combine forms them.  Sides 64 to 256 (a tile's rows fit a copy box).
+// The transforms of these sides by themselves wait for nothing, so a short wait limit
+// does not fail this one either: its waits have at least the default.
 int fft32_towers_sum(float2 *stack, int layers, int S, double theta, const double *layer_w,
                      const int32_t *chunk_first, int nchunks, float2 *out, int32_t *status,
                      cudaStream_t st, bool *used) {
   *used = false;
-  if (!fft32_supported(S, S) || S > 256 || wait_cycles() == 0) return CG_OK;
+  if (!fft32_supported(S, S) || S > 256) return CG_OK;
   const int C = S == 256 ? 16 : 32;
   CUtensorMap map;
   if (!f32::stack_map(&map, stack, S, 1, S, layers, C)) return CG_OK;
@@ -1351,9 +1353,10 @@ int fft32_towers_sum(float2 *stack, int layers, int S, double theta, const doubl
   f32::StackArgs A{S,   1,   S / C, 1, S / 2, true, chunk_first, sc.list, sc.ph,
                    out, (int64_t)S * S, 1.0f / (float)((int64_t)S * S)};
   const int64_t units = (int64_t)nchunks * A.tiles;
-  rc = ls == 6   ? f32::launch_stack<6, 32>(map, A, units, 1, status, st)
-       : ls == 7 ? f32::launch_stack<7, 32>(map, A, units, 1, status, st)
-                 : f32::launch_stack<8, 16>(map, A, units, 1, status, st);
+  const long long wait = std::max(wait_cycles(), f32::FFT_WAIT_CYCLES);
+  rc = ls == 6   ? f32::launch_stack<6, 32>(map, A, units, 1, wait, status, st)
+       : ls == 7 ? f32::launch_stack<7, 32>(map, A, units, 1, wait, status, st)
+                 : f32::launch_stack<8, 16>(map, A, units, 1, wait, status, st);
   const cudaError_t fe = cudaFreeAsync(sc.list, st);
   if (rc) return rc;
   CG_CUDA(fe);

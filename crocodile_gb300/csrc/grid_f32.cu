@@ -798,12 +798,10 @@ static int direct_grid_launch(const cg_plan *p, const float2 *ktab, const float2
 }
 
 // Whether a call takes the direct gridder by itself, unless a cell is crowded
-// (DIRECT_CELL_TAPS).  A wait limit of 0 keeps to the lane kernel (lane_launch) where that
-// would run.
-static bool direct_wanted(const cg_plan *p, bool lane) {
+// (DIRECT_CELL_TAPS).
+static bool direct_wanted(const cg_plan *p) {
   const cg_tuning t = tuning();
-  return p->direct && t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0 &&
-         !(lane && wait_cycles() == 0);
+  return p->direct && t.layout == 0 && t.tile == 0 && t.groups == 0 && t.rows == 0;
 }
 
 // The plan as seen by the direct gridder (crowded = false) and by the windowed one
@@ -843,7 +841,7 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   // gridder, us: S 8, 30k on 512^2: 11 / 24 / 23; S 16: 22 / 32 / 53; 60k on 4096^2, S 8:
   // 13 / 56 / 53).
   cg_plan q;
-  if (direct_wanted(p, lane)) {
+  if (direct_wanted(p)) {
     q = split_plan(p, false);
     const int rc = direct_grid_launch(&q, kt, vv, nullptr, weight, mode, gg, s);
     if (rc || p->n <= DIRECT_CELL_TAPS) return rc;
@@ -1061,7 +1059,7 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
   // 173 us in one traversal, 22 so), and separable tables on the register-window
   // gridder's small tiles, whose table is small, so reading it twice costs nothing.
   // Not in place: the second pass reads what the first would have overwritten.
-  const bool direct = direct_wanted(p, lane);
+  const bool direct = direct_wanted(p);
   const char *vi0 = (const char *)vis_in, *vo0 = (const char *)vis_out;
   const size_t vbytes = (size_t)p->n * sizeof(float2);
   const bool apart = !vis_in || !vis_out || vi0 + vbytes <= vo0 || vo0 + vbytes <= vi0;

@@ -423,8 +423,9 @@ int lane_launch(const cg_plan *p, const float2 *ktab, const float2 *vis, const f
   // fused pass always.  Streamed / loaded, us, S 16: w-projection 2M, 4096^2, 604 /
   // 485, fused 926 / 741; AW 1.75M, 8192^2, 1.8 GB, 694 / 646; dense tiles and a
   // table of gigabytes: AW 2M, 4096^2, 1.6 GB, 598 / 615 (fused 934 / 812), 16.1M, 12 GB,
-  // 4116 / 4273 (fused 6381 / 5712).  A lane layout asked for by the tuning streams,
-  // and so does a wait limit of 0, whose time-outs only the streams have.
+  // 4116 / 4273 (fused 6381 / 5712).  A lane layout asked for by the tuning streams.  So
+  // does a wait limit of 0, under which the gridders of this layout have always given
+  // up at the first poll: programs that make a wait run out that way still can.
   const int64_t table = (int64_t)p->kd.G * p->kd.Q * p->kd.Q * SS * (int64_t)sizeof(float2);
   const int64_t per_tile = p->n / std::max(p->ntx * p->nty * p->layers, 1);
   const bool stream = t.layout == CG_LAYOUT_LANE || wait_cycles() == 0 ||

@@ -152,10 +152,12 @@ int cg_get_tuning(cg_tuning *out);
  * the same limit; a wait that runs out there is counted in a device-wide
  * counter that cg_fft_timeouts reads (after synchronising the device; reset
  * nonzero: set it back to 0), in cg_wstack_image and cg_towers_image as
- * CG_ERR_TIMEOUT in the status block too, and the output is undefined.  No
+ * CG_ERR_TIMEOUT in the status block too, and the output is undefined
+ * (cg_towers_image waits for the default limit at least).  No
  * counterpart in the reference: a test hook that makes a wait run out on
  * purpose (a limit of 0 fails every copy not yet landed when it is first
- * polled).  Process-wide. */
+ * polled, and has the lane gridder bring its slices by copies on calls where it
+ * would load them).  Process-wide. */
 int cg_set_wait_limit(long long cycles);
 long long cg_get_wait_limit(void);
 int cg_fft_timeouts(int32_t *count, int reset);

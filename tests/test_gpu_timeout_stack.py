@@ -40,3 +40,41 @@ def test_wstack_wait_runs_out_and_next_call_is_right():
     st.check()
     assert E.fft_timeouts() == 0
     assert torch.linalg.norm(got - want) <= 1e-6 * torch.linalg.norm(want)
+
+
+def test_limit_of_zero_leaves_other_calls_as_they_are():
+    """Calls whose kernels wait for nothing, or for the default limit at least, give the
+    same results under a wait limit of 0: the direct gridder on a table of the lane
+    layout (one visibility to a cell: sums in any order are the same), and w-towers'
+    sums in the transforms' own pass."""
+    import numpy
+    import torch
+    from crocodile_gb300 import _lib as L, engine as E
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    lib = L.lib()
+    rng = numpy.random.default_rng(5)
+    N, S, n = 256, 16, 25
+    uv = (numpy.stack(numpy.meshgrid(numpy.arange(5), numpy.arange(5)), -1).reshape(-1, 2) - 2) * 32
+    uvw = numpy.column_stack([uv / N, numpy.zeros(n)])
+    kt = E.KernelTable.from_gcf(rng.normal(size=(2, 2, S, S)) + 0j, 0, E.CF)
+    v = E.cuda_tensor(rng.normal(size=n) + 0j, E.CF)
+    stack = E.cuda_tensor(rng.normal(size=(5, 128, 128)) + 0j, E.CF)
+    w, first = numpy.linspace(-100, 100, 5), numpy.array([0, 2, 5], numpy.int32)
+
+    def calls():
+        st = E.Status()
+        plan = E.Plan(uvw, 1.0, (N, N), kt, status=st)
+        grid = plan.grid(kt, v, torch.zeros((N, N), dtype=E.CF, device="cuda"))
+        image = E.towers_image(stack.clone(), 0.2, w, first, st)
+        st.check()
+        return torch.view_as_real(grid), torch.view_as_real(image)
+
+    want = calls()
+    default = lib.cg_get_wait_limit()
+    try:
+        assert lib.cg_set_wait_limit(0) == L.CG_OK
+        got = calls()
+    finally:
+        lib.cg_set_wait_limit(default)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
