@@ -511,8 +511,8 @@ static void *grid_kernel_for(int R) {
   }
 }
 
-// Sparse gridder: for stacks of grids holding few visibilities per tile (the
-// sub-grids of w-towers), where staging and flushing a window per work item
+// Sparse gridder, supports above 16 (k_grid_direct takes the others): for stacks of
+// grids holding few visibilities per tile (the sub-grids of w-towers), where staging and flushing a window per work item
 // costs more than the visibilities' own taps.  No shared memory: each warp
 // takes work items in turn, loads 32 records at a time (one per lane) and, for
 // each visibility, lane l adds taps l + 32 i straight into the grid with
@@ -968,7 +968,7 @@ int cg_grid_sparse(const cg_plan *p, const void *ktab, const void *vis, void *gr
   void (*fn)(TiledArgs, const float2 *, const float2 *, float2 *) = nullptr;
 #define PICK(M)                                                                \
   if (!fn && need <= M) fn = p->kd.sep ? k_grid_sparse<true, M> : k_grid_sparse<false, M>;
-  PICK(1) PICK(2) PICK(4) PICK(8) PICK(16) PICK(32)
+  PICK(16) PICK(32)
 #undef PICK
   CG_REQUIRE(fn, "support too large for the sparse gridder");
   int per_sm = 0;
