@@ -279,6 +279,7 @@ struct cg_plan {
   int lane_odd; // odd supports on the lane layout's tiles, gridded by the lane kernel
   int lean;     // plan_geometry: the choices that need the least workspace
   int direct;   // few visibilities: the direct gridder unless a cell is crowded
+  int beside;   // direct, and n lets a cell be crowded: the others beside it
   int slice_stride;  // lane layout: elements between S x S slices of the table it reads
   int64_t kpad_slices;  // lane layout, slices padded to a 16-byte multiple: slices to copy
   // device arrays inside the caller's workspace

@@ -844,7 +844,7 @@ static int grid_launch(const cg_plan *p, const void *ktab, const void *vis,
   if (direct_wanted(p)) {
     q = split_plan(p, false);
     const int rc = direct_grid_launch(&q, kt, vv, nullptr, weight, mode, gg, s);
-    if (rc || p->n <= DIRECT_CELL_TAPS) return rc;
+    if (rc || !p->beside) return rc;
     q = split_plan(p, true);
     p = &q;
     A.nitems = q.nitems;
@@ -1067,7 +1067,7 @@ int cg_degrid_grid(const cg_plan *p, const void *ktab, const void *grid_in, cons
     const float2 *kt = (const float2 *)ktab, *vi = (const float2 *)vis_in;
     const int mode = residual ? 3 : 0;
     float2 *go = (float2 *)grid_out, *vo = (float2 *)vis_out;
-    const bool beside = direct && vis_in && p->n > DIRECT_CELL_TAPS;
+    const bool beside = direct && vis_in && p->beside;
     cg_plan q = split_plan(p, true);  // a crowded cell: one traversal where no better
     if (beside && !p->outer) {
       const int rc = fused_launch(&q, ktab, grid_in, vis_in, residual, vis_out, grid_out, lane, s);

@@ -322,7 +322,7 @@ __device__ __forceinline__ void write_items(int tile, int off, int count, int ch
 // Whether a cell could get more than DIRECT_CELL_TAPS taps.  Taps reach it from the
 // visibilities of `reach` tiles to an axis, so no cell does unless the tiles of
 // some reach x reach block hold that many, and then one of them holds `few`
-// (INT32_MAX: a plan that is not for the direct gridder).
+// (INT32_MAX: a plan that is not for the direct gridder, or for that alone).
 struct Crowd {
   int few, reach, tblog, nbx, ntx, nty, tpl;
   template <int R>
@@ -900,6 +900,7 @@ static void plan_geometry(cg_plan &p) {
     // the lane kernel's, which take the call where a cell is crowded
     p.direct = !p.lean && t.layout == 0 && t.tile == 0 && direct_fits(p) &&
                (p.layers > 1 || p.tile_req > 0 || p.outer || lane);
+    p.beside = p.direct && p.n > DIRECT_CELL_TAPS;
     // no order inside a tile (for few visibilities it is not worth its buckets)
     const bool flat = p.outer || lane || p.direct;
     p.T = p.outer ? outer_T : p.lane_odd ? 16 : tile_edge(p.kd, p.tile_req);
@@ -1117,7 +1118,7 @@ int plan_build_into(cg_plan *p, int mode, const cg_kernel_desc *kd, int H, int W
   const bool tiled = mode == CG_PLAN_TILED;
   const ItemSize size = {p->chunk, p->chunk_crowded};
   const int reach = kd->S > 1 && p->T > 0 ? (kd->S - 2) / p->T + 2 : 1;
-  const Crowd crowd = {p->direct ? std::max(1, DIRECT_CELL_TAPS / (reach * reach)) : INT32_MAX,
+  const Crowd crowd = {p->beside ? std::max(1, DIRECT_CELL_TAPS / (reach * reach)) : INT32_MAX,
                        reach, p->tblog, p->nbx, p->ntx, p->nty, p->tpl};
   const int scan_blocks = (p->nbuckets + SCAN_TILE - 1) / SCAN_TILE;
   if (tiled && p->nbuckets <= (p->sublog ? PLAN_SMALL_BUCKETS : PLAN_SMALL_TILES)) {

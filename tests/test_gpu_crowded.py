@@ -44,14 +44,14 @@ def _exact(N, S, gcf, uvw, sep, value):
     return out
 
 
-def _check(env, N, n, S, sep, where):
+def _check(env, N, n, S, sep, where, tile=0):
     torch, L, E, O = env
     Q = 4
     rng = numpy.random.default_rng(N + S)
     uvw = _places(N, n, S, where, rng)
     gcf = rng.uniform(0.2, 1, (Q, S) if sep else (Q, Q, S, S)).astype(numpy.float32).astype(complex)
     kt = E.KernelTable.from_gcf(gcf, 0, E.CF)
-    plan = E.Plan(uvw, 1.0, (N, N), kt)
+    plan = E.Plan(uvw, 1.0, (N, N), kt, tile=tile)
     value = numpy.float32(0.7391)
     v = torch.full((n,), float(value), dtype=E.CF, device="cuda")
     w = torch.full((n,), float(value), dtype=torch.float32, device="cuda")
@@ -91,3 +91,13 @@ def test_few_visibilities(env, N, per, S, sep, where):
 @pytest.mark.parametrize("S,sep", [(8, True), (8, False)])
 def test_few_on_a_large_grid(env, S, sep):
     _check(env, 8192, 204800, S, sep, "cell")
+
+
+@pytest.mark.parametrize("where", ["cell", "tile"])
+@pytest.mark.parametrize("S,sep", [(1, True), (8, True), (13, True), (9, False), (16, False)])
+@pytest.mark.parametrize("tile", [4, 8, 16, 32])
+@pytest.mark.parametrize("n", [1, 57, 512, 513, 3000])
+def test_requested_tiles(env, n, tile, S, sep, where):
+    """Tiles as requested, so small that a cell's taps come from many; and calls too
+    small for any cell to be crowded."""
+    _check(env, 512, n, S, sep, where, tile)
