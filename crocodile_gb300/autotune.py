@@ -43,10 +43,11 @@ def get_tuning():
 
 
 def effective_layout(ktab):
-    """The gridder layout the library uses for this kernel table under the
-    current tuning (the rule of layout_for in csrc/api.cu): the tuned layout
-    (the lane layout only for S <= 16), or automatically the lane layout for
-    non-separable tables with even S <= 16 and the warp layout otherwise."""
+    """The gridder layout of this kernel table under the current tuning (the rule of
+    layout_for in csrc/api.cu): the tuned layout (the lane layout only for S <= 16),
+    or automatically the lane layout for non-separable tables with even S <= 16 and
+    the warp layout otherwise.  Without a tuned layout a plan may take another
+    gridder by the number of visibilities (include/crocodile_gb300.h, layout 0)."""
     lay = get_tuning()["layout"]
     if lay == L.CG_LAYOUT_LANE:
         return lay if ktab.S <= 16 else L.CG_LAYOUT_WARP

@@ -322,7 +322,7 @@ inline bool direct_fits(const cg_plan &p) {
   return p.kd.S <= 16 && (double)p.n * p.kd.S <= 200.0 * (double)(p.H < p.W ? p.H : p.W);
 }
 
-// That is the host's guess; the plan's counts decide on the device (plan.cu, crowded):
+// That is the host's guess; the plan's counts decide on the device (Crowd, plan.cu):
 // where a cell could get more than this many taps, another gridder takes the call.
 // Equal terms are the worst case (a PSF on equal coordinates): 512 in sequence, the
 // most that the lane gridder sums in a window, are off by 3.7e-6, 25,600 by 1.9e-4 and

@@ -912,9 +912,9 @@ struct StackShape {
 // tile of C columns) takes its planes in turn, each plane's tile one tensor copy,
 // double-buffered, and keeps the sum and the phases of its elements in
 // registers.  Bound by issue (the factors beside the transform) at about the rate
-// HBM reads the stack.  8 planes of 4096^2, transform and sum: 1.42 ms apart, 1.26
-// so; w_stack_imaging of 32 planes 7.38 -> 6.44 ms; 1200 layers of 256^2 in 200
-// sums: 0.66 and 0.52 ms.  Waits are bounded as in k_fft32_step_tma.
+// HBM reads the stack.  8 planes of 4096^2, transform and sum: 1.43 ms apart, 1.30
+// so; w_stack_imaging of 32 planes 7.38 -> 6.67 ms; 1200 layers of 256^2 in 200
+// sums: 0.62 and 0.54 ms.  Waits are bounded as in k_fft32_step_tma.
 template <int LOGL, int C>
 __global__ void __launch_bounds__(StackShape<LOGL, C>::THREADS, StackShape<LOGL, C>::MINB)
     k_fft32_stack(const __grid_constant__ CUtensorMap tmap, StackArgs A, int64_t units,
@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(StackShape<LOGL, C>::THREADS, StackShape<LOGL,
 // The reverse: rows of every layer's image, the chunk's image (unshifted) over
 // exp(2 pi i w ph), transformed on their way out, so that the layers are written
 // once.  A unit is a group of rows of one chunk, whose image and phases stay in
-// registers over the chunk's layers.  1200 layers of 256^2: 0.67 ms apart, 0.52 so.
+// registers over the chunk's layers.  1200 layers of 256^2: 0.63 ms apart, 0.51 so.
 template <int LOGN>
 __global__ void __launch_bounds__(256, 2)
     k_fft32_rows_stack(const float2 *__restrict__ images, StackArgs A, int64_t units,

@@ -877,8 +877,9 @@ static int outer_edge(const cg_plan &p, int &T) {
 // lane layout's 16-cell tiles under no tuning and no requested tile, for the lane
 // kernel with taps by loads: not for the narrowest, nor where tiles are nearly
 // empty (plan and grid, warp gridder / lane kernel, us: S 9, 123k on 1531^2: 94 / 81,
-// 2M on 4096^2: 541 / 467, 400k: 172 / 168; S 7, 2M: 422 / 419, 545 / 578 fused).  Not for
-// stacks of so many tiles that their numbers would run out.
+// 2M on 4096^2: 541 / 467, 400k: 172 / 168; S 7, 2M: 422 / 419, 545 / 578 fused).  On one
+// grid's few visibilities any, beside the direct gridder.  Not for stacks of so many
+// tiles that their numbers would run out.
 static bool lane_odd(const cg_plan &p) {
   const cg_tuning t = tuning();
   const int S = p.kd.S;

@@ -107,13 +107,14 @@ class KernelTable:
         kernels zero-padded to S + 1 (a zero first row and column, so that tap j + 1
         of the padded kernel sits where tap j of the original did: footprints start
         at x - (S + 1) / 2 instead of x - S // 2).  Gridding and degridding with it
-        give the same results (the extra taps add zeros), and the lane-layout
-        gridder, which streams even-support slices by bulk copies, takes it: the
-        w-projection step at 4096^2, 2M visibilities, S 15 runs in 1.24-1.27 ms
-        against 1.40 ms with the S 15 table.  Returns self when the table does not
-        qualify or a footprint could leave the grid (the padded one reaches one
-        cell lower): uvw [n, 3] device coordinates in wavelengths, lam the scale
-        (grid cells = N u / lam), shape the grid (H, W)."""
+        give the same results (the extra taps add zeros), and even supports' slices
+        are what the lane gridder can stream by bulk copies (tables beyond 1 GiB under
+        dense visibilities; otherwise it loads them): the w-projection step at 4096^2,
+        2M visibilities, S 15 took 1.24-1.27 ms against 1.40 ms with the S 15 table on
+        the warp gridder.  Returns self when the table does not qualify or a
+        footprint could leave the grid (the padded one reaches one cell lower): uvw
+        [n, 3] device coordinates in wavelengths, lam the scale (grid cells = N u /
+        lam), shape the grid (H, W)."""
         if self.sep or self.dtype != CF or self.S not in (13, 15) or uvw.shape[0] == 0:
             return self
         N = min(int(shape[-2]), int(shape[-1]))

@@ -127,9 +127,10 @@ typedef struct {
  * layout 0 lets each plan and call choose: non-separable tables, S <= 16, get
  * 16-cell tiles and the lane kernel (its slices by loads, or by bulk copies
  * where the table is large and the tiles dense), or taps added straight to the
- * grid where visibilities are few; separable tables, S <= 16, the gridder with
- * its window in registers or again the direct one; wider supports
- * CG_LAYOUT_WARP.  Process-wide. */
+ * grid where visibilities are few and no cell is crowded (tiles of 8 or 12
+ * cells there); separable tables, S <= 16, the gridder with its window in
+ * registers or again the direct one; wider supports, and grids of too many
+ * such tiles, CG_LAYOUT_WARP.  Process-wide. */
 #define CG_LAYOUT_WARP 1
 #define CG_LAYOUT_OWNER 2
 #define CG_LAYOUT_LANE 3
@@ -174,9 +175,10 @@ typedef struct cg_plan cg_plan;
 
 size_t cg_plan_workspace_bytes(int mode, int64_t n, int H, int W,
                                const cg_kernel_desc *kd);
-/* Builds the plan on `stream`.  CG_PLAN_GROUPS synchronises once to learn
- * the group sizes.  A data error leaves the plan marked failed (see
- * cg_status_check); grid/degrid then do nothing. */
+/* Builds the plan on `stream`.  CG_PLAN_GROUPS on a stack of grids
+ * synchronises once to learn the group sizes.  A data error leaves the plan
+ * marked failed (see cg_status_check); grid/degrid then do nothing, or, once
+ * the status block is reset, take the visibilities that were not refused. */
 int cg_plan_create(cg_plan **plan, int mode, const cg_kernel_desc *kd, int H,
                    int W, const double *uvw, int64_t stride, double lam,
                    const int32_t *kidx, int64_t n, void *workspace,
@@ -477,6 +479,11 @@ int cg_towers_add(const void *sub_c64, int nchunks, int S, const int32_t *origin
  * w_kernel_function(l, m, layer_w[L]), rolled and sign-modulated so that an
  * unshifted forward cg_fft_raw of the stack gives the centred sub-grids, which a
  * layered plan's cg_degrid then degrids with the residual-w kernels. */
+int cg_towers_cut(const void *grid_c64, int N, const int32_t *origin, int nchunks, int S,
+                  void *out_c64, cg_stream_t stream);
+int cg_towers_expand(const void *images_c64, int S, double theta, const double *layer_w,
+                     const int32_t *chunk_first, int nchunks, void *out_c64, int32_t *d_status,
+                     cg_stream_t stream);
 /* cg_towers_image: the unshifted inverse cg_fft_raw of the gridded layers and
  * cg_towers_combine in one (the stack is left undefined); cg_towers_layers:
  * cg_towers_expand and the forward cg_fft_raw of its layers in one.  For sides 64
@@ -487,11 +494,6 @@ int cg_towers_image(void *stack_c64, int layers, int S, double theta, const doub
 int cg_towers_layers(const void *images_c64, int layers, int S, double theta,
                      const double *layer_w, const int32_t *chunk_first, int nchunks,
                      void *stack_c64, int32_t *d_status, cg_stream_t stream);
-int cg_towers_cut(const void *grid_c64, int N, const int32_t *origin, int nchunks, int S,
-                  void *out_c64, cg_stream_t stream);
-int cg_towers_expand(const void *images_c64, int S, double theta, const double *layer_w,
-                     const int32_t *chunk_first, int nchunks, void *out_c64, int32_t *d_status,
-                     cg_stream_t stream);
 
 /* ------------------------------------------------------------------ */
 /* Kernel generation (FP64 arithmetic; outputs c64 or c128). */

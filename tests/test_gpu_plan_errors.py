@@ -68,3 +68,22 @@ def test_refused_rows_are_left_out(env, n, nbad, layers, sep):
         plan.check()
         for a, b in got:
             assert numpy.linalg.norm(a.cpu().numpy() - b) <= tol * numpy.linalg.norm(b)
+
+
+def test_aw_kernels_bad_index(env):
+    """An antenna index beyond the A-kernels is an IndexError of its call; the next call
+    gives the kernels that it gave before, bit for bit."""
+    torch, L, E, O = env
+    rng = numpy.random.default_rng(2)
+    A = rng.normal(size=(5, 16, 16)) + 1j * rng.normal(size=(5, 16, 16))
+    W = rng.normal(size=(2, 2, 2, 16, 16)) + 1j * rng.normal(size=(2, 2, 2, 16, 16))
+    a1, a2 = rng.integers(0, 5, (2, 6)).astype(numpy.int32)
+    wi = rng.integers(0, 2, 6).astype(numpy.int32)
+    want = E.aw_kernels(A, W, a1, a2, wi, dtype=E.CF)
+    for i, bad in ((5, 5), (0, -1), (2, 100)):
+        b = a1.copy()
+        b[i] = bad
+        with pytest.raises(IndexError):
+            E.aw_kernels(A, W, b, a2, wi, dtype=E.CF)
+    got = E.aw_kernels(A, W, a1, a2, wi, dtype=E.CF)
+    assert torch.equal(torch.view_as_real(got), torch.view_as_real(want))
