@@ -170,6 +170,15 @@ def kernel_groups(lead_shape, src, n):
 # --------------------------------------------------------------------------
 # plans and gridding
 
+def _holds(what, t, count, itemsize):
+    """t, or a ValueError where it holds less than count items: the kernels take the
+    lengths from the plan."""
+    if t is not None and t.numel() * t.element_size() < count * itemsize:
+        raise ValueError("%s of %d bytes where %d items of %d are needed"
+                         % (what, t.numel() * t.element_size(), count, itemsize))
+    return t
+
+
 class Plan:
     """Sorted, bit-exact cell assignment of a visibility set (cg_plan_create).
 
@@ -191,15 +200,18 @@ class Plan:
         if self.uvw.dim() != 2 or self.uvw.shape[1] < 2:
             raise ValueError("uvw must be [n, >=2]")
         self.n = self.uvw.shape[0]
-        self.kidx = None if kidx is None else cuda_tensor(kidx, torch.int32)
+        self.kidx = None if kidx is None else _holds("kidx", cuda_tensor(kidx, torch.int32),
+                                                     self.n, 4)
         self.shape = (int(shape[0]), int(shape[1]))
         self.mode = mode
         self.sep, self.Q, self.S, self.G = ktab.sep, ktab.Q, ktab.S, ktab.G
         kd = ktab.desc()
         self._kd = kd
         self.layers = 1 if layers is None else int(layers[0])
-        self.layer = None if layers is None else cuda_tensor(layers[1], torch.int32)
-        self.group = None if groups is None else cuda_tensor(groups[1], torch.int32)
+        self.layer = None if layers is None else _holds(
+            "layers", cuda_tensor(layers[1], torch.int32), self.n, 4)
+        self.group = None if groups is None else _holds(
+            "groups", cuda_tensor(groups[1], torch.int32), self.n, 4)
         opts = L.PlanOpts(self.layers, None if self.layer is None else self.layer.data_ptr(),
                           0.0 if wbins is None else float(wbins[0]),
                           0 if wbins is None else int(wbins[1]),
@@ -250,6 +262,12 @@ class Plan:
             raise ValueError("kernel table does not match the plan's kernel layout")
         return ktab.to(dtype).table
 
+    def _vis(self, what, t, itemsize=8):
+        return _p(_holds(what, t, self.n, itemsize))
+
+    def _cells(self, t, itemsize=8):
+        return _p(_holds("grid", t, self.layers * self.shape[0] * self.shape[1], itemsize))
+
     def layer_mean_w(self):
         """(mean w [layers] float64, visibility count [layers] int32) per grid layer."""
         mean = torch.empty(self.layers, dtype=torch.float64, device="cuda")
@@ -261,27 +279,29 @@ class Plan:
     def grid(self, ktab, vis, grid):
         """grid (c64 [H, W], or [layers, H, W]) += convgrid of vis (c64 [n])."""
         t = self._table(ktab, CF)
-        L.call("cg_grid", self.handle, _p(t), _p(vis), _p(grid), stream())
+        L.call("cg_grid", self.handle, _p(t), self._vis("vis", vis), self._cells(grid), stream())
         return grid
 
     def grid_sparse(self, ktab, vis, grid):
         """grid += convgrid(vis) with per-tap atomics (cg_grid_sparse): for plans with
         few visibilities per tile."""
         t = self._table(ktab, CF)
-        L.call("cg_grid_sparse", self.handle, _p(t), _p(vis), _p(grid), stream())
+        L.call("cg_grid_sparse", self.handle, _p(t), self._vis("vis", vis), self._cells(grid),
+               stream())
         return grid
 
     def grid_weighted(self, ktab, vis, weight, grid):
         """grid += convgrid of vis * weight (vis None: weight alone, the PSF pass)."""
         t = self._table(ktab, CF)
-        L.call("cg_grid_weighted", self.handle, _p(t), _p(vis), _p(weight), _p(grid), stream())
+        L.call("cg_grid_weighted", self.handle, _p(t), self._vis("vis", vis),
+               self._vis("weight", weight, 4), self._cells(grid), stream())
         return grid
 
     def degrid(self, ktab, grid, out=None):
         t = self._table(ktab, CF)
         if out is None:
             out = torch.empty(self.n, dtype=CF, device="cuda")
-        L.call("cg_degrid", self.handle, _p(t), _p(grid), _p(out), stream())
+        L.call("cg_degrid", self.handle, _p(t), self._cells(grid), self._vis("out", out), stream())
         return out
 
     def degrid_grid(self, ktab, grid_in, vis_in, grid_out, residual=False, vis_out=None):
@@ -290,20 +310,23 @@ class Plan:
         t = self._table(ktab, CF)
         if vis_out is None:
             vis_out = torch.empty(self.n, dtype=CF, device="cuda")
-        L.call("cg_degrid_grid", self.handle, _p(t), _p(grid_in), _p(vis_in), int(bool(residual)),
-               _p(vis_out), _p(grid_out), stream())
+        L.call("cg_degrid_grid", self.handle, _p(t), self._cells(grid_in),
+               self._vis("vis_in", vis_in), int(bool(residual)), self._vis("vis_out", vis_out),
+               self._cells(grid_out), stream())
         return vis_out
 
     def grid_fp64(self, ktab, vis, grid):
         t = self._table(ktab, CD)
-        L.call("cg_grid_fp64", self.handle, _p(t), _p(vis), _p(grid), stream())
+        L.call("cg_grid_fp64", self.handle, _p(t), self._vis("vis", vis, 16),
+               self._cells(grid, 16), stream())
         return grid
 
     def degrid_fp64(self, ktab, grid, out=None):
         t = self._table(ktab, CD)
         if out is None:
             out = torch.empty(self.n, dtype=CD, device="cuda")
-        L.call("cg_degrid_fp64", self.handle, _p(t), _p(grid), _p(out), stream())
+        L.call("cg_degrid_fp64", self.handle, _p(t), self._cells(grid, 16),
+               self._vis("out", out, 16), stream())
         return out
 
 

@@ -87,3 +87,40 @@ def test_aw_kernels_bad_index(env):
             E.aw_kernels(A, W, b, a2, wi, dtype=E.CF)
     got = E.aw_kernels(A, W, a1, a2, wi, dtype=E.CF)
     assert torch.equal(torch.view_as_real(got), torch.view_as_real(want))
+
+
+def test_arrays_that_are_too_short(env):
+    """Fewer visibilities, weights, indices, results or cells than the plan has are
+    refused before anything runs; more than it has are taken as before."""
+    torch, L, E, O = env
+    n, N, S, G = 40, 64, 8, 3
+    rng = numpy.random.default_rng(4)
+    uvw = numpy.column_stack([rng.uniform(-0.3, 0.3, (n, 2)), numpy.zeros(n)])
+    gcf = rng.normal(size=(G, 4, S)) + 0j
+    idx = rng.integers(0, 2, n).astype(numpy.int32)
+    short, more = idx[:-1], numpy.append(idx, 0).astype(numpy.int32)
+    kt, kd = E.KernelTable.from_gcf(gcf, 1, E.CF), E.KernelTable.from_gcf(gcf, 1, E.CD)
+    groups = L.CG_PLAN_GROUPS
+    for kw in (dict(kidx=short), dict(kidx=idx, layers=(2, short)),
+               dict(kidx=idx, mode=groups, groups=(2, short))):
+        with pytest.raises(ValueError):
+            E.Plan(uvw, 1.0, (N, N), kt, **kw)
+    E.Plan(uvw, 1.0, (N, N), kt, more, layers=(2, more)).check()
+    plan = E.Plan(uvw, 1.0, (N, N), kt, idx, layers=(2, idx))
+    plain = E.Plan(uvw, 1.0, (N, N), kd, idx, mode=groups)
+    v, v1 = (torch.zeros(k, dtype=E.CF, device="cuda") for k in (n, n - 1))
+    g, g1 = (torch.zeros((k, N, N), dtype=E.CF, device="cuda") for k in (2, 1))
+    w1 = torch.zeros(n - 1, dtype=torch.float32, device="cuda")
+    for call in (lambda: plan.grid(kt, v1, g), lambda: plan.grid(kt, v, g1),
+                 lambda: plan.grid_sparse(kt, v1, g), lambda: plan.grid_sparse(kt, v, g1),
+                 lambda: plan.grid_weighted(kt, None, w1, g), lambda: plan.degrid(kt, g1),
+                 lambda: plan.degrid(kt, g, v1), lambda: plan.degrid_grid(kt, g1, v, g.clone()),
+                 lambda: plan.degrid_grid(kt, g, v1, g.clone()),
+                 lambda: plan.degrid_grid(kt, g, v, g1),
+                 lambda: plan.degrid_grid(kt, g, v, g.clone(), vis_out=v1),
+                 lambda: plain.grid_fp64(kd, v, g.to(E.CD)),  # complex64: half the bytes
+                 lambda: plain.degrid_fp64(kd, g1)):
+        with pytest.raises(ValueError):
+            call()
+    plan.check()
+    plain.check()
