@@ -212,6 +212,7 @@ class Plan:
             "layers", cuda_tensor(layers[1], torch.int32), self.n, 4)
         self.group = None if groups is None else _holds(
             "groups", cuda_tensor(groups[1], torch.int32), self.n, 4)
+        self.tile = int(tile)
         opts = L.PlanOpts(self.layers, None if self.layer is None else self.layer.data_ptr(),
                           0.0 if wbins is None else float(wbins[0]),
                           0 if wbins is None else int(wbins[1]),
@@ -234,6 +235,25 @@ class Plan:
         out = (ctypes.c_int64 * 4)()
         L.call("cg_plan_info", self.handle, out)
         return {"tile": out[0], "max_items": out[1], "chunk": out[2], "buckets": out[3]}
+
+    def few_per_tile(self):
+        """Whether a stack's tiles average fewer than 16 visibilities, which adding tap by
+        tap to the grids (grid_sparse) suits best.  Tiles as requested or tuned, else the
+        edges of the gridders with windows in shared memory: plans cut smaller tiles for
+        other gridders, which take fewer visibilities to a tile.  Never for one grid, whose
+        automatic gridder adds tap by tap itself where that is accurate."""
+        if self.layers == 1:
+            return False
+        t = L.Tuning()
+        L.call("cg_get_tuning", ctypes.byref(t))
+        if self.tile or t.tile or t.layout:
+            edge = self.info()["tile"]
+        elif not self.sep and self.S <= 16 and self.S % 2 == 0:
+            edge = 16
+        else:
+            edge = 32 if self.S <= 8 else 48 if self.S <= 16 else 64
+        tiles = self.layers * -(-self.shape[0] // edge) * -(-self.shape[1] // edge)
+        return self.n < 16 * tiles
 
     def export(self):
         """(recs [n, 4] int32 {x0, y0, k0, k1} in sorted order, perm [n] sorted

@@ -905,8 +905,8 @@ def w_stack_imaging(theta, lam, uvw, src, vis, kv, plane, precision=None, per_pl
     index.  All planes grid in one launch into a stack of grids and transform in one
     batched FFT; ``per_plane=True`` grids and transforms one plane per launch instead
     (the comparator).  ``gridder``: "tiled" (cg_grid), "sparse" (cg_grid_sparse, per-tap
-    atomics) or "auto", sparse when the stack's tiles average fewer than 16 visibilities
-    (4M visibilities over 32 planes of 4096^2: 1.4 ms sparse against 2.4 ms tiled).
+    atomics) or "auto", sparse when the tiles of more than one plane average fewer than 16
+    visibilities (4M visibilities over 32 planes of 4096^2: 1.4 ms sparse against 2.4 ms tiled).
     FP32 only."""
     if _prec(precision) != "fp32":
         raise ValueError("w_stack_imaging runs the FP32 tiled path only")
@@ -926,8 +926,7 @@ def w_stack_imaging(theta, lam, uvw, src, vis, kv, plane, precision=None, per_pl
     if not per_plane:
         plan = E.Plan(uvw_t, lam, (N, N), ktab, kidx, status=st,
                       layers=(layers, ptab if _is_dev(ptab) else ptab.astype(numpy.int32)))
-        tiles = layers * (-(-N // plan.info()["tile"])) ** 2
-        if gridder == "sparse" or (gridder == "auto" and n < 16 * tiles):
+        if gridder == "sparse" or (gridder == "auto" and plan.few_per_tile()):
             plan.grid_sparse(ktab, vis_t, planes)
         elif gridder in ("auto", "tiled"):
             plan.grid(ktab, vis_t, planes)
@@ -1010,8 +1009,7 @@ def w_towers_imaging(theta, lam, uvw, src, vis, subgrid_size, margin, wincrement
     stack = torch.zeros((len(used), s, s), dtype=E.CF, device="cuda")
     plan = E.Plan(rel, s / theta, (s, s), ktab, kidx, status=st, layers=(len(used), row),
                   tile=tile)
-    tiles = len(used) * (-(-s // plan.info()["tile"])) ** 2
-    if gridder == "sparse" or (gridder == "auto" and n < 16 * tiles):
+    if gridder == "sparse" or (gridder == "auto" and plan.few_per_tile()):
         plan.grid_sparse(ktab, vis_t, stack)
     elif gridder in ("auto", "tiled"):
         plan.grid(ktab, vis_t, stack)
@@ -1110,8 +1108,7 @@ def aw_towers_imaging(theta, lam, uvw, src, vis, subgrid_size, margin, wstep, ai
         st.check()
         return _host(grid, like=uvw)
     stack = torch.zeros((len(used), 2 * s, 2 * s), dtype=E.CF, device="cuda")
-    tiles = len(used) * (-(-2 * s // plan.info()["tile"])) ** 2
-    if gridder == "sparse" or (gridder == "auto" and n < 16 * tiles):
+    if gridder == "sparse" or (gridder == "auto" and plan.few_per_tile()):
         plan.grid_sparse(ktab, vis_t, stack)
     elif gridder in ("auto", "tiled"):
         plan.grid(ktab, vis_t, stack)

@@ -101,3 +101,21 @@ def test_requested_tiles(env, n, tile, S, sep, where):
     """Tiles as requested, so small that a cell's taps come from many; and calls too
     small for any cell to be crowded."""
     _check(env, 512, n, S, sep, where, tile)
+
+
+@pytest.mark.parametrize("layers,N,n,S,sep", [(1, 1024, 100000, 8, True), (1, 1024, 100000, 8, False),
+                                              (1, 2048, 60000, 3, True), (2, 256, 6500, 9, False)])
+def test_wstack_planes(env, layers, N, n, S, sep):
+    """w-stacking of crowded planes that are not sparse by the edge of the windowed
+    gridders' tiles, whatever tiles the plan has: the image (w 0: the sum of the planes'
+    inverse transforms) against 64 bits."""
+    torch, L, E, O = env
+    from crocodile_gb300 import synthesis
+    rng = numpy.random.default_rng(N + S)
+    uvw = _places(N, n, S, "cell", rng)
+    gcf = rng.uniform(0.2, 1, (4, S) if sep else (4, 4, S, S)).astype(numpy.float32).astype(complex)
+    value = numpy.float32(0.7391)
+    image = synthesis.w_stack_imaging(1.0, N, N * uvw, None, numpy.full(n, value + 0j), gcf,
+                                      numpy.arange(n) % layers)
+    want = O.ifft(_exact(N, S, gcf, uvw, sep, float(value)))
+    assert numpy.linalg.norm(image - want) <= TOL * numpy.linalg.norm(want)
