@@ -949,11 +949,15 @@ static void plan_geometry(cg_plan &p) {
     auto clamp = [](int64_t v, int64_t lo, int64_t hi) {
       return (int)(std::min(hi, std::max(lo, v)) & ~(int64_t)31);
     };
+    // (a lane item with taps for less than half its window's cells adds them to the grid
+    // one by one, which full items of narrow supports on wide tiles must not)
+    const int64_t lane_least =
+        std::max<int64_t>(64, (int64_t)p.win * p.win / (2 * p.kd.S * p.kd.S) + 32);
     const int per_cta = (int)std::min<int64_t>(
         2048, std::max<int64_t>(256, p.n / (int64_t)(num_sms() * 16) + 1));
     p.chunk = t.chunk > 0 ? t.chunk
               : p.outer   ? clamp(per_warp, 32, 256)
-              : lane      ? (p.lean ? 512 : clamp(per_warp, 64, 512))
+              : lane      ? (p.lean ? 512 : clamp(per_warp, lane_least, 512))
                           : per_cta;
     p.chunk_crowded = t.chunk > 0 ? t.chunk : lane ? 512 : per_cta;
     p.max_items = (p.n + p.chunk - 1) / p.chunk + p.ntiles;

@@ -119,3 +119,11 @@ def test_wstack_planes(env, layers, N, n, S, sep):
                                       numpy.arange(n) % layers)
     want = O.ifft(_exact(N, S, gcf, uvw, sep, float(value)))
     assert numpy.linalg.norm(image - want) <= TOL * numpy.linalg.norm(want)
+
+
+@pytest.mark.parametrize("N,n,S,tile", [(777, 13593, 2, 32), (777, 13593, 4, 64), (256, 60000, 2, 32),
+                                        (256, 60000, 4, 64), (256, 60000, 1, 16)])
+def test_narrow_supports_on_wide_tiles(env, N, n, S, tile):
+    """Lane items of few taps beside their window's cells: those of full length are
+    summed in the window all the same."""
+    _check(env, N, n, S, False, "cell", tile)
