@@ -603,11 +603,12 @@ static void *grid_warp_kernel_for(int maxt) {
 struct DirectArgs {
   TiledArgs A;
   SortedEnd end;
+  int batch;     // one grid: visibilities to a warp at a time
   int layered;  // grids of a stack: by work item, which knows its layer
 };
 
 // Calls f(start, nb, grid offset) for batches of at most 32 sorted
-// visibilities of one grid, warp by warp.
+// visibilities of one grid, warp by warp (D.batch: direct_launch).
 template <class F>
 __device__ __forceinline__ void direct_batches(const DirectArgs &D, F f) {
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -615,9 +616,8 @@ __device__ __forceinline__ void direct_batches(const DirectArgs &D, F f) {
   const int nitems = *D.A.nitems;
   if (nitems == 0) return;  // no visibility, or the call is another gridder's
   if (!D.layered) {
-    const int64_t n = D.end();
-    for (int64_t b = gw * 32; b < n; b += nw * 32)
-      f((int)b, (int)min((int64_t)32, n - b), (size_t)0);
+    const int64_t n = D.end(), m = D.batch;
+    for (int64_t b = gw * m; b < n; b += nw * m) f((int)b, (int)min(m, n - b), (size_t)0);
     return;
   }
   for (int64_t it = gw; it < nitems; it += nw) {
@@ -770,12 +770,20 @@ static void *grid_direct_for(int support) {
   return nullptr;
 }
 
-static int direct_launch(const cg_plan *p, void *fn, void **args, cudaStream_t s) {
+// Batches of 32 while they fill the GPU; fewer visibilities are spread over more warps,
+// down to as many as a warp works on at once, since a warp takes the visibilities of
+// its batch in turn (2,000 visibilities on 2048^2, S 16, 4-D, degrid: 33 us in batches
+// its batch in turn (2,000 visibilities on 2048^2, S 16, 4-D, degrid: 33 us in batches
+// of 32, 8 so; 21 by the tiled degridder).
+static int direct_launch(const cg_plan *p, void *fn, DirectArgs &D, void **args, cudaStream_t s) {
   int per_sm = 0;
   CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-  const int64_t warps = p->layers > 1 ? p->max_items : (p->n + 31) / 32;
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>((int64_t)std::max(per_sm, 1) * num_sms(), (warps + 7) / 8));
+  const int64_t most = (int64_t)std::max(per_sm, 1) * num_sms();  // blocks of 8 warps
+  const int least = 32 / direct_lanes(p->kd.S);
+  D.batch = 32;
+  while (D.batch > least && p->n < most * 8 * D.batch) D.batch /= 2;
+  const int64_t warps = p->layers > 1 ? p->max_items : (p->n + D.batch - 1) / D.batch;
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(most, (warps + 7) / 8));
   CG_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(256), args, 0, s));
   return CG_OK;
 }
@@ -794,7 +802,7 @@ static int direct_grid_launch(const cg_plan *p, const float2 *ktab, const float2
   void *fn = p->kd.sep ? grid_direct_for<true>(p->kd.S) : grid_direct_for<false>(p->kd.S);
   DirectArgs D = direct_args(p);
   void *args[] = {&D, &mode, &ktab, &vis, &sub, &weight, &grid};
-  return direct_launch(p, fn, args, s);
+  return direct_launch(p, fn, D, args, s);
 }
 
 // Whether a call takes the direct gridder by itself, unless a cell is crowded
@@ -1016,7 +1024,7 @@ int cg_degrid(const cg_plan *p, const void *ktab, const void *grid, void *out,
     void *fn = p->kd.sep ? degrid_direct_for<true>(p->kd.S) : degrid_direct_for<false>(p->kd.S);
     DirectArgs D = direct_args(p);
     void *args[] = {&D, &ktab, &grid, &out};
-    return direct_launch(p, fn, args, s);
+    return direct_launch(p, fn, D, args, s);
   }
   TiledArgs A = tiled_args(p);
   const int SS = p->kd.S * p->kd.S;
