@@ -959,7 +959,7 @@ static void plan_geometry(cg_plan &p) {
               : p.outer   ? clamp(per_warp, 32, 256)
               : lane      ? (p.lean ? 512 : clamp(per_warp, lane_least, 512))
                           : per_cta;
-    p.chunk_crowded = t.chunk > 0 ? t.chunk : lane ? 512 : per_cta;
+    p.chunk_crowded = t.chunk > 0 ? t.chunk : lane && !p.lane_odd ? 512 : per_cta;
     p.max_items = (p.n + p.chunk - 1) / p.chunk + p.ntiles;
     // The lane gridder streams each visibility's S x S slice with one bulk copy,
     // which needs a multiple of 16 bytes: for odd S * S it reads a copy of the
