@@ -846,11 +846,14 @@ static int64_t tiles_of(const cg_plan &p, int T) {
 
 // Window edge of the register-window gridder for separable tables
 // (grid_outer.cu) and its tile edge T (window >= T + S - 1), or 0 where another
-// gridder runs: the one with shared-memory tiles for the narrowest supports unless visibilities are dense
-// (its time goes with S, the window's flush does not; plan and grid, warp gridder
-// / this one, us: S 3, 1M on 2048^2: 153 / 181, S 5: 174 / 179, on 4096^2: 200 / 183,
-// S 6: 210 / 172, S 8: 239 / 170, on 4096^2: 259 / 218).  Stacks of grids, requested
-// or tuned tiles and tuned layouts keep the other gridders.
+// gridder runs: the one with shared-memory tiles for supports to 4 (its time goes with
+// S, the window's flush does not; plan and grid, warp gridder / this one, us: S 3, 1M on
+// 2048^2: 153 / 181, S 5: 174 / 179, on 4096^2: 200 / 183, S 6: 210 / 172, S 8: 239 / 170, on
+// 4096^2: 259 / 218; 8 visibilities a cell of 512^2, S 1: 284 / 389, S 4: 311 / 384, S 5: 372 /
+// 384, S 6: 433 / 387), but for dense visibilities of small calls, where its launches
+// are the shorter (8 a cell of 48^2, 18,432, S 1: 39 / 33, S 4: 41 / 33; 98,304 on 256^2,
+// S 1: 46 / 49, S 4: 48 / 50).  Stacks of grids, requested or tuned tiles and tuned
+// layouts keep the other gridders.
 static int outer_edge(const cg_plan &p, int &T) {
   const cg_tuning t = tuning();
   const int S = p.kd.S;
@@ -859,7 +862,7 @@ static int outer_edge(const cg_plan &p, int &T) {
     return 0;
   const double rho = (double)p.n / ((double)p.H * (double)p.W);
   const bool few = direct_fits(p);
-  if (!few && S <= 4 && rho < 1.5) return 0;
+  if (!few && S <= 4 && (rho < 1.5 || p.n >= 65536)) return 0;
   // few visibilities: small tiles, whose counts bound a cell's taps more closely;
   // larger tiles where they fit the window and are not full: fewer flushes, but
   // more visibilities to a counter of the plan (S 5, 1M on 1024^2: plan 117 us with

@@ -127,3 +127,11 @@ def test_narrow_supports_on_wide_tiles(env, N, n, S, tile):
     """Lane items of few taps beside their window's cells: those of full length are
     summed in the window all the same."""
     _check(env, N, n, S, False, "cell", tile)
+
+
+@pytest.mark.parametrize("S", [1, 2, 4, 5])
+@pytest.mark.parametrize("n", [65535, 65536])
+def test_narrow_supports_dense(env, n, S):
+    """Narrow separable supports on either side of the line between the gridders, on
+    dense visibilities of one tile."""
+    _check(env, 96, n, S, True, "tile")
